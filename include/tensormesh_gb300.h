@@ -151,6 +151,63 @@ typedef struct tm_assemble_args {
 int tm_assemble(const tm_patch_plan* plan, const tm_assemble_args* args, void* stream);
 
 /*
+ * Element-once assembly: every element is integrated once into `work`, then
+ * every CSR entry sums its elements' values (no patch plan; faster wherever
+ * the scratch fits).  Same arguments and results as tm_assemble; FP64 in
+ * double-float (TM_PREC_EMULATED).  The plan's arrays are device arrays:
+ *   elements[E*B]          connectivity
+ *   indptr[N+1]            node-level CSR row pointer
+ *   nptr[N+1], nrec[E*B]   incidences of every node (tm_node_lists)
+ *   groups of rows_per_cta rows that are neighbours in space, with the
+ *   elements they touch (tm_group_fill; P1 triangles and tetrahedra):
+ *   order[N]               the rows in group order
+ *   base[3*(G+1)]          first gelem, gent and grec of each group
+ *   gelem[], gent[], grec[]
+ * max_entries, max_elems: most CSR entries and elements of one group.  Calls that run at the same time need a work array each.
+ */
+typedef struct tm_gather_plan {
+  int32_t n_elements;
+  int32_t n_points;
+  int32_t rows_per_cta;
+  int32_t max_entries;
+  int32_t max_elems;
+  int32_t pad0;
+  const int32_t* elements;
+  const int64_t* indptr;
+  const int64_t* nptr;
+  const uint32_t* nrec;
+  const int32_t* order;
+  const int64_t* base;
+  const int32_t* gelem;
+  const uint32_t* gent;
+  const uint16_t* grec;
+} tm_gather_plan;
+
+/* bytes of `work`, or minus a status (TM_ERR_UNSUPPORTED: use tm_assemble) */
+int64_t tm_gather_workspace_bytes(int32_t element, int32_t form, int32_t dtype, int32_t n_comp, int64_t n_elements);
+
+int tm_assemble_gather(const tm_gather_plan* plan, const tm_assemble_args* args, void* work, int64_t work_bytes,
+                       void* stream);
+
+/*
+ * The plan's lists.  slots[E*B*B] is tm_pattern_fill's slot map.
+ * tm_node_lists counts with nptr == NULL, then fills with the scanned nptr.
+ * tm_group_count writes [distinct elements, entries, records] of every group
+ * and sets *bad when a group exceeds the record format (use fewer rows); base
+ * is the exclusive scan of the sizes, cnt[nnz] is scratch that tm_group_fill
+ * consumes.  quads = 1: the records of scalar forms, 0: of elasticity blocks.
+ * rows_per_group <= 64.
+ */
+int tm_group_count(int32_t n_basis, int64_t n_points, int32_t rows_per_group, int32_t quads, const int32_t* order,
+                   const int64_t* nptr, const uint32_t* nrec, const int64_t* indptr, const int64_t* slots,
+                   int32_t* cnt, int32_t* sizes, int32_t* bad, void* stream);
+int tm_group_fill(int32_t n_basis, int64_t n_points, int32_t rows_per_group, int32_t quads, const int32_t* order,
+                  const int64_t* nptr, const uint32_t* nrec, const int64_t* indptr, const int64_t* slots,
+                  int32_t* cnt, const int64_t* base, int32_t* gelem, uint32_t* gent, uint16_t* grec, void* stream);
+int tm_node_lists(const int32_t* elements, int64_t n_elements, int32_t n_basis, int64_t n_points, const int64_t* nptr,
+                  int32_t* cnt, uint32_t* nrec, void* stream);
+
+/*
  * Backward (adjoint) assembly.  Given dL/d(values) of a tm_assemble call
  * with the same plan and args, writes per-(patch, element) partial gradients:
  *   pair_dX[n_pairs][B][D]          dL/dX of the element's nodes;

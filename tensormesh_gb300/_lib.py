@@ -43,6 +43,8 @@ EXPORTS = [
     "tm_sell_plan", "tm_pcg_sell_workspace_bytes", "tm_pcg_jacobi_sell",
     "tm_fcg_workspace_doubles", "tm_fcg_twolevel_iterations", "tm_kp_count", "tm_kp_fill",
     "tm_sell_fill", "tm_spmv_sell",
+    "tm_gather_workspace_bytes", "tm_assemble_gather", "tm_node_lists",
+    "tm_group_count", "tm_group_fill",
 ]
 
 P = ctypes.c_void_p
@@ -84,6 +86,16 @@ class AssembleArgs(ctypes.Structure):
     ]
 
 
+class GatherPlan(ctypes.Structure):
+    _fields_ = [
+        ("n_elements", ctypes.c_int32), ("n_points", ctypes.c_int32),
+        ("rows_per_cta", ctypes.c_int32), ("max_entries", ctypes.c_int32),
+        ("max_elems", ctypes.c_int32), ("pad0", ctypes.c_int32),
+        ("elements", P), ("indptr", P), ("nptr", P), ("nrec", P), ("order", P), ("base", P),
+        ("gelem", P), ("gent", P), ("grec", P),
+    ]
+
+
 class BackwardArgs(ctypes.Structure):
     _fields_ = [("grad_out", P), ("pair_dX", P), ("pair_dcoef", P)]
 
@@ -117,6 +129,10 @@ def _declare(lib):
     i32, i64 = ctypes.c_int32, ctypes.c_int64
     sig = {
         "tm_assemble": [ctypes.POINTER(PatchPlan), ctypes.POINTER(AssembleArgs), P],
+        "tm_assemble_gather": [ctypes.POINTER(GatherPlan), ctypes.POINTER(AssembleArgs), P, i64, P],
+        "tm_group_count": [i32, i64, i32, i32, P, P, P, P, P, P, P, P, P],
+        "tm_group_fill": [i32, i64, i32, i32, P, P, P, P, P, P, P, P, P, P, P],
+        "tm_node_lists": [P, i64, i32, i64, P, P, P, P],
         "tm_quadrature_points": [i32, i32, i32, P, P, P, i64, P, P],
         "tm_spmv_csr": [i32, i64, i64, P, P, P, P, P, P],
         "tm_pcg_jacobi": [i32, i64, P, P, P, P, P, ctypes.c_double, ctypes.c_double, i32, P, i64, P],
@@ -156,6 +172,8 @@ def _declare(lib):
         "tm_pcg_jacobi_sell": [i32, i64, P, P, P, P, i64, P, P, ctypes.c_double, ctypes.c_double, i32, i32, P, i64,
                                P],
     }
+    lib.tm_gather_workspace_bytes.argtypes = [i32, i32, i32, i32, i64]
+    lib.tm_gather_workspace_bytes.restype = i64
     lib.tm_sell_plan.argtypes = [i64, P, P, P, ctypes.POINTER(i32), P]
     lib.tm_fcg_workspace_doubles.argtypes = []
     lib.tm_fcg_workspace_doubles.restype = i64

@@ -1,0 +1,105 @@
+// Element-once assembly of P1 triangles and tetrahedra (Laplace, elasticity).
+#include "gather_p1.cuh"
+#include "gather_sum.cuh"
+
+namespace tmg {
+namespace ga {
+
+template <int D, bool kElast> int64_t p1_bytes(int dtype, int64_t n_el) {
+  return n_el * p1_values<D, kElast>() * (dtype == TM_F64 ? 8 : 4);
+}
+
+int64_t p1_scratch_bytes(int element, int form, int dtype, int64_t n_el) {
+  const bool el = form == TM_FORM_ELASTICITY;
+  const int64_t v = element == TM_TRI3 ? (el ? p1_bytes<2, true>(dtype, n_el) : p1_bytes<2, false>(dtype, n_el))
+                                       : (el ? p1_bytes<3, true>(dtype, n_el) : p1_bytes<3, false>(dtype, n_el));
+  return 256 + up256((n_el + 31) / 32 * 4) + up256(v);
+}
+
+// Clears the flag, sums the weights and sets the common exponent to that of
+// element 0.
+template <class T, int D>
+__global__ void p1_head_kernel(const int32_t* __restrict__ el, tm_assemble_args args, Head* head) {
+  constexpr int NB = D + 1;
+  double wsum = 0.0;
+  for (int q = 0; q < args.n_quad; ++q) wsum += args.tables[q];
+  int S = 0;
+  if constexpr (sizeof(T) == 8) {
+    int v[NB];
+    load_conn<NB>(el, 0, v);
+    Edges<T, D, NB> ed;
+    ed.load(static_cast<const T*>(args.points), v);
+    const int ec = dexp(p1_coef<NB>(args, 0, v, wsum));
+    S = elem_exp(ed.ok() ? ed.emax : 1023, ec > 0 && ec < 2047 ? ec : 1023, D - 2);
+  }
+  head->S = S;
+  head->any = 0u;
+  head->w = sizeof(T) == 8 ? pair_of(wsum) : make_float2((float)wsum, 0.f);
+  head->wsum = wsum;
+}
+
+template <class T, int D, bool kElast>
+int launch_p1(const tm_gather_plan& plan, const tm_assemble_args& args, void* work, cudaStream_t s) {
+  using S = typename Sto<T>::S;
+  const int64_t n = plan.n_elements;
+  const Scratch sc = scratch_of(work, n, n * p1_values<D, kElast>() * (int64_t)sizeof(S));
+  S* vals = reinterpret_cast<S*>(sc.vals);
+  p1_head_kernel<T, D><<<1, 1, 0, s>>>(plan.elements, args, sc.head);
+  p1_element_kernel<T, D, kElast><<<(unsigned)((n + kElThreads - 1) / kElThreads), kElThreads, 0, s>>>(
+      n, plan.elements, args, sc.head, sc.wide, vals);
+  const S* cv = vals;
+  const Head* ch = sc.head;
+  const uint32_t* cw = sc.wide;
+  T* out = static_cast<T*>(args.out);
+  if constexpr (kElast)
+    return launch_group(group_blocks_kernel<T, D>, plan, kBlkGrpThreads, group_blocks_smem<T, D>(plan), s, cv, ch, cw, args.lam,
+                        args.mu, out);
+  else
+    return launch_group(group_rows_kernel<T, D + 1, false>, plan, kGrpThreads, group_rows_smem<T, D + 1>(plan), s, cv, cv, ch, cw,
+                        out);
+}
+
+int assemble_p1(const tm_gather_plan& plan, const tm_assemble_args& a, void* work, cudaStream_t s) {
+  const bool el = a.form == TM_FORM_ELASTICITY;
+  if (a.element == TM_TRI3) {
+    if (a.dtype == TM_F64)
+      return el ? launch_p1<double, 2, true>(plan, a, work, s) : launch_p1<double, 2, false>(plan, a, work, s);
+    return el ? launch_p1<float, 2, true>(plan, a, work, s) : launch_p1<float, 2, false>(plan, a, work, s);
+  }
+  if (a.dtype == TM_F64)
+    return el ? launch_p1<double, 3, true>(plan, a, work, s) : launch_p1<double, 3, false>(plan, a, work, s);
+  return el ? launch_p1<float, 3, true>(plan, a, work, s) : launch_p1<float, 3, false>(plan, a, work, s);
+}
+
+}  // namespace ga
+}  // namespace tmg
+
+extern "C" int64_t tm_gather_workspace_bytes(int32_t element, int32_t form, int32_t dtype, int32_t n_comp,
+                                             int64_t n_elements) {
+  (void)n_comp;
+  if (n_elements < 0 || (dtype != TM_F32 && dtype != TM_F64)) return -TM_ERR_INVALID;
+  if (element != TM_TRI3 && element != TM_TET4) return -TM_ERR_UNSUPPORTED;
+  if (form != TM_FORM_LAPLACE && form != TM_FORM_ELASTICITY) return -TM_ERR_UNSUPPORTED;
+  return tmg::ga::p1_scratch_bytes(element, form, dtype, n_elements);
+}
+
+extern "C" int tm_assemble_gather(const tm_gather_plan* plan, const tm_assemble_args* args, void* work,
+                                  int64_t work_bytes, void* stream) {
+  if (!plan || !args) return TM_ERR_INVALID;
+  if (plan->n_elements < 0 || plan->n_points < 0) return TM_ERR_INVALID;
+  if (args->dtype != TM_F32 && args->dtype != TM_F64) return TM_ERR_INVALID;
+  if (args->n_quad < 1 || args->n_quad > 11) return TM_ERR_INVALID;
+  if (args->coef_kind < TM_COEF_SCALAR || args->coef_kind > TM_COEF_QUAD) return TM_ERR_INVALID;
+  if (args->dtype == TM_F64 && args->precision != TM_PREC_EMULATED) return TM_ERR_UNSUPPORTED;
+  const int64_t need = tm_gather_workspace_bytes(args->element, args->form, args->dtype, args->n_comp,
+                                                 plan->n_elements);
+  if (need < 0) return (int)-need;
+  if (plan->n_elements == 0) return TM_OK;
+  if (!args->tables || !args->points || !args->out || !work) return TM_ERR_INVALID;
+  if (!plan->elements || !plan->indptr || !plan->order || !plan->base || !plan->gelem || !plan->gent || !plan->grec)
+    return TM_ERR_INVALID;
+  if (args->coef_kind != TM_COEF_SCALAR && !args->coef) return TM_ERR_INVALID;
+  if (plan->n_points < 1 || plan->rows_per_cta < 1 || plan->max_entries < 1 || plan->max_elems < 1) return TM_ERR_INVALID;
+  if (work_bytes < need) return TM_ERR_INDEX;
+  return tmg::ga::assemble_p1(*plan, *args, work, static_cast<cudaStream_t>(stream));
+}

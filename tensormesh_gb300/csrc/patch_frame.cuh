@@ -221,14 +221,16 @@ TM_D FrameInfo patch_frame(const T* __restrict__ pts, const int32_t* __restrict_
 
 // v * 2^k.  An exponent add when v and the result are normal; the rare
 // remaining cases (zero, inf / nan, subnormal input or result) go through
-// scalbn.
+// scalbn, kept out of line: inlined it is turned into selects, and its FP64
+// multiplications run for every value on a pipe 1/64 as wide as FP32's.
+static __device__ __noinline__ double tm_scale_pow2_rare(double v, int k) { return scalbn(v, k); }
 TM_D double tm_scale_pow2(double v, int k) {
   const unsigned long long b = (unsigned long long)__double_as_longlong(v);
   const int e = (int)((b >> 52) & 0x7ff);
   const int ne = e + k;
   if (e != 0 && e != 2047 && ne > 0 && ne < 2047) return __longlong_as_double((long long)b + (long long)k * (1ll << 52));
-  if (v == 0.0 || e == 2047) return v;
-  return scalbn(v, k);
+  if ((b << 1) == 0ull || e == 2047) return v;   // an integer test: the FP64 pipe is slow
+  return tm_scale_pow2_rare(v, k);
 }
 TM_D float tm_scale_pow2(float v, int k) {
   const unsigned b = __float_as_uint(v);

@@ -419,3 +419,99 @@ class PatchPlan:
         return sum(getattr(self, n).numel() * getattr(self, n).element_size()
                    for n in ("vptr", "vtx", "eptr", "elem", "econn", "rptr", "rows", "racc", "iptr",
                              "inc_elem", "inc_a", "inc_pos"))
+
+
+class GatherPlan:
+    """Lists of the element-once assembly (tm_assemble_gather), built on the
+    device by the project's kernels: the incidences of every node and, for P1
+    meshes, groups of rows that are neighbours in space with the elements they
+    touch.  ``ok`` is False where the lists do not apply (an element that
+    repeats a node, or sizes past their index types); the patch kernels run
+    then."""
+
+    # rows per group: 32 scalar rows (a tetrahedral group touches about 440
+    # elements, 21 KB of staged values, so eight 128-thread CTAs share an SM:
+    # 124 us at 80^3 against 136 us for 64 rows and 256 threads); as many rows
+    # of blocks as have at most 512 entries, one for each thread of the CTA
+    ROWS = {1: (32, 16, 8, 4, 2, 1), 2: (64, 56, 48, 40, 32, 24, 16, 8, 4, 2, 1),
+            3: (34, 32, 30, 28, 26, 24, 22, 20, 16, 12, 8, 4, 2, 1)}
+    BLOCK_ENTRIES = 512
+    SMEM_BYTES = 200 * 1024
+
+    def __init__(self, elements: torch.Tensor, points: torch.Tensor, pattern: NodePattern):
+        E, B = elements.shape
+        dev = elements.device
+        self.pattern, self.elements = pattern, elements
+        self._structs = {}
+        self.ok = dev.type == "cuda" and E > 0 and B <= 4 and E * B < 2**31 - 1 and \
+            pattern.nnz < 2**31 - 1 and not self._repeats(elements)
+        if not self.ok:
+            return
+        s = _lib.stream_handle(dev)
+        N = pattern.n_points
+        ncnt = torch.empty(N, dtype=torch.int32, device=dev)
+        _lib.call("tm_node_lists", elements.data_ptr(), E, B, N, None, ncnt.data_ptr(), None, s)
+        self.nptr = torch.zeros(N + 1, dtype=torch.int64, device=dev)
+        torch.cumsum(ncnt, 0, out=self.nptr[1:])
+        self.nrec = torch.empty(E * B, dtype=torch.int32, device=dev)
+        _lib.call("tm_node_lists", elements.data_ptr(), E, B, N, self.nptr.data_ptr(), ncnt.data_ptr(),
+                  self.nrec.data_ptr(), s)
+        c = points.detach().to(torch.float64).contiguous()
+        key = morton_keys(c, c.min(0).values.contiguous(), c.max(0).values.contiguous(), 63 // c.shape[1])
+        self.order = torch.argsort(key, stable=True).to(torch.int32)
+
+    @staticmethod
+    def _repeats(elements: torch.Tensor) -> bool:
+        B = elements.shape[1]
+        bad = torch.zeros((), dtype=torch.bool, device=elements.device)
+        for a in range(B):
+            for b in range(a + 1, B):
+                bad |= (elements[:, a] == elements[:, b]).any()
+        return bool(bad)
+
+    def struct(self, H: int):
+        """ctypes view with the groups for H x H blocks, or None."""
+        if not self.ok:
+            return None
+        if H not in self._structs:
+            self._structs[H] = self._groups(H)
+        s = self._structs[H]
+        return None if s is None else s[0]
+
+    def _groups(self, H: int):
+        E, B = self.elements.shape
+        N, dev, pat = self.pattern.n_points, self.elements.device, self.pattern
+        quads = int(H == 1)
+        bad = torch.empty(1, dtype=torch.int32, device=dev)
+        cnt = torch.empty(pat.nnz, dtype=torch.int32, device=dev)
+        lists = (self.order.data_ptr(), self.nptr.data_ptr(), self.nrec.data_ptr(), pat.indptr.data_ptr(),
+                 pat.slots.data_ptr(), cnt.data_ptr())
+        stream = _lib.stream_handle(dev)
+        for rows in self.ROWS[H]:
+            G = -(-N // rows)
+            sizes = torch.empty((G, 3), dtype=torch.int32, device=dev)
+            _lib.call("tm_group_count", B, N, rows, quads, *lists, sizes.data_ptr(), bad.data_ptr(), stream)
+            most = torch.cat([sizes.max(0).values, bad]).tolist()
+            if H == 1:
+                words = most[0] * (B * (B - 1) // 2 + 2) + most[1]    # float64 words, head-room included
+            else:
+                words = max(most[0] * 14, most[1] * H * H)
+            if not most[3] and 8 * words <= self.SMEM_BYTES and (H == 1 or most[1] <= self.BLOCK_ENTRIES):
+                break
+        else:
+            return None
+        base = torch.zeros((G + 1, 3), dtype=torch.int64, device=dev)
+        torch.cumsum(sizes, 0, out=base[1:])
+        n_elem, n_ent, n_rec = base[-1].tolist()
+        gelem = torch.empty(n_elem, dtype=torch.int32, device=dev)
+        gent = torch.empty(n_ent, dtype=torch.int32, device=dev)
+        grec = torch.zeros(n_rec + 8, dtype=torch.int16, device=dev)
+        _lib.call("tm_group_fill", B, N, rows, quads, *lists, base.data_ptr(), gelem.data_ptr(), gent.data_ptr(),
+                  grec.data_ptr(), stream)
+        s = _lib.GatherPlan()
+        s.n_elements, s.n_points, s.rows_per_cta, s.max_entries, s.max_elems = E, N, rows, most[1], most[0]
+        keep = dict(elements=self.elements, indptr=pat.indptr, nptr=self.nptr, nrec=self.nrec, order=self.order,
+                    base=base, gelem=gelem, gent=gent, grec=grec)
+        for name, t in keep.items():
+            setattr(s, name, t.data_ptr())
+        return s, keep

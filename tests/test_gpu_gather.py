@@ -1,0 +1,171 @@
+"""Element-once assembly of P1 meshes (tm_assemble_gather): sizes around the
+32-row groups, random numbering, every coefficient kind, high-valence nodes,
+and the group lists themselves.
+
+Bars: float64 values within 1e-12 of max|K| of the oracle (the bar of every
+float64 assembly), float32 within 1e-5, CSR values symmetric and bitwise
+repeatable."""
+import numpy as np
+import pytest
+import torch
+
+import tensormesh_gb300 as tg
+from oracle import fem
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+class KappaLaplace(tg.ElementAssembler):
+    def forward(self, gradu, gradv, kappa):
+        return kappa * (gradu @ gradv)
+
+
+class EElasticity(tg.ElementAssembler):
+    def forward(self, gradu, gradv, kappa):
+        lam, mu = tg.forms.reference_lame(1.0, 0.3)
+        return kappa * tg.forms.elasticity_block(gradu, gradv, lam, mu)
+
+
+@pytest.fixture(autouse=True)
+def every_size(monkeypatch):
+    """The element-once path at any size (its dispatch keeps small meshes on
+    the one-launch patch kernels)."""
+    monkeypatch.setattr("tensormesh_gb300.assemble._GATHER_MIN_ELEMENTS", 0)
+
+
+FORMS = {"laplace": KappaLaplace, "elasticity": EElasticity}
+
+
+def ragged(etype, n, seed):
+    base = tg.Mesh.gen_unit_square(n) if etype == "triangle" else tg.Mesh.gen_unit_cube(n)
+    rng = np.random.default_rng(seed)
+    pts = base.points.numpy() + rng.uniform(-0.2, 0.2, size=tuple(base.points.shape)) / n
+    new = rng.permutation(pts.shape[0])
+    moved = np.empty_like(pts)
+    moved[new] = pts
+    el = new[base.cells[etype].numpy()]
+    return moved, el[rng.permutation(el.shape[0])]
+
+
+def check(pts, el, etype, form, coef, dtype=torch.float64, q=2, data="element_data"):
+    mesh = tg.Mesh(points=torch.tensor(pts, device=DEV, dtype=dtype), cells={etype: torch.tensor(el, device=DEV)})
+    asm = FORMS[form].from_mesh(mesh, quadrature_order=q)
+    c = torch.tensor(coef, device=DEV, dtype=dtype)
+    call = lambda: asm(mesh.points, **{data: {"kappa": c}})  # noqa: E731
+    K = call()
+    assert asm.topology.gather.struct(1) is not None
+    p64, c64 = mesh.points.double().cpu().numpy(), c.double().cpu().numpy()
+    oc = {"coef": c64} if data == "element_data" else {"coef": element_mean(c64, el)}
+    ip, ix, dv = fem.assemble_csr(p64, el, etype, form, q, **oc)
+    assert np.array_equal(K.indptr.cpu().numpy(), ip) and np.array_equal(K.indices.cpu().numpy(), ix)
+    err = np.max(np.abs(K.values.double().cpu().numpy() - dv)) / np.max(np.abs(dv))
+    assert err <= (1e-12 if dtype == torch.float64 else 1e-5), err
+    assert torch.equal(call().values, K.values)
+
+
+def element_mean(c, el):
+    # an order-2 rule integrates a linear coefficient against constant gradients exactly
+    return c[el].mean(1)
+
+
+@pytest.mark.parametrize("etype,n", [("triangle", 1), ("triangle", 5), ("triangle", 11), ("tetra", 1), ("tetra", 3),
+                                     ("tetra", 6)])
+@pytest.mark.parametrize("form", ["laplace", "elasticity"])
+@pytest.mark.parametrize("dtype", [torch.float64, torch.float32])
+def test_ragged_groups_match_oracle(etype, n, form, dtype):
+    pts, el = ragged(etype, n, 3 * n)
+    check(pts, el, etype, form, np.exp(np.random.default_rng(n).normal(size=el.shape[0])), dtype)
+
+
+@pytest.mark.parametrize("form", ["laplace", "elasticity"])
+def test_point_coefficients(form):
+    pts, el = ragged("tetra", 4, 9)
+    check(pts, el, "tetra", form, np.exp(np.random.default_rng(1).normal(size=pts.shape[0])), data="point_data")
+
+
+@pytest.mark.parametrize("ring", [90, 200])
+@pytest.mark.parametrize("form", ["laplace", "elasticity"])
+def test_high_valence_nodes(ring, form):
+    """Two apexes with `ring` + 1 neighbours each: lists and rows far longer
+    than a regular mesh's."""
+    t = np.arange(ring) * 2 * np.pi / ring
+    pts = np.concatenate([[[0.0, 0.0, -0.3], [0.0, 0.0, 0.3]], np.stack([np.cos(t), np.sin(t), 0 * t], 1)])
+    el = np.array([[0, 2 + k, 2 + (k + 1) % ring, 1] for k in range(ring)], dtype=np.int64)
+    check(pts, el, "tetra", form, np.exp(np.random.default_rng(ring).normal(size=ring)))
+
+
+def test_zero_and_far_coefficients():
+    """Zero coefficients, and coefficients far outside the common exponent's
+    window on either side of element 0's, in one call: every entry keeps its
+    own relative accuracy where a single element makes it."""
+    pts, el = ragged("tetra", 3, 5)
+    g = np.exp(np.random.default_rng(6).normal(size=el.shape[0]))
+    for scale in (0.0, 1e-40, 1e40):
+        check(pts, el, "tetra", "laplace", g * np.where(np.arange(el.shape[0]) % 3 == 1, scale, 1.0))
+        check(pts, el, "tetra", "elasticity", g * np.where(np.arange(el.shape[0]) % 3 == 0, scale, 1.0))
+
+
+def test_an_element_that_repeats_a_node_keeps_the_patch_kernels():
+    pts, el = ragged("tetra", 2, 8)
+    bad = np.concatenate([el, el[:1]])
+    bad[-1, 3] = bad[-1, 0]
+    mesh = tg.Mesh(points=torch.tensor(pts, device=DEV), cells={"tetra": torch.tensor(bad, device=DEV)})
+    assert KappaLaplace.from_mesh(mesh).topology.gather.struct(1) is None
+
+
+@pytest.mark.parametrize("etype,n", [("triangle", 7), ("tetra", 4)])
+@pytest.mark.parametrize("H", [1, 0])
+def test_group_lists_cover_every_entry(etype, n, H):
+    """The lists decoded on the host name, for every CSR position off the
+    diagonal, the elements that hold its node pair, ascending."""
+    pts, el = ragged(etype, n, 2)
+    mesh = tg.Mesh(points=torch.tensor(pts, device=DEV), cells={etype: torch.tensor(el, device=DEV)})
+    topo = KappaLaplace.from_mesh(mesh).topology
+    H = H or topo.dim
+    topo.gather.struct(H)
+    s, keep = topo.gather._structs[H]
+    B = el.shape[1]
+    P = B * (B - 1) // 2
+    pairs = [(a, b) for a in range(B) for b in range(a + 1, B)]
+    k = {name: t.cpu().numpy() for name, t in keep.items()}
+    ent, rec = k["gent"].view(np.uint32), k["grec"].view(np.uint16)
+    ip, ix = topo.pattern.indptr.cpu().numpy(), topo.pattern.indices.cpu().numpy()
+    holds = {}
+    for e, nodes in enumerate(el):
+        for i in nodes:
+            for j in nodes:
+                if i != j:
+                    holds.setdefault((i, j), []).append(e)
+    assert sorted(k["order"].tolist()) == list(range(pts.shape[0]))
+    for g in range(k["base"].shape[0] - 1):
+        e0, t, r0 = k["base"][g]
+        elems = k["gelem"][e0:k["base"][g + 1][0]]
+        assert np.all(np.diff(elems) > 0)
+        for lr, r in enumerate(k["order"][g * s.rows_per_cta:(g + 1) * s.rows_per_cta]):
+            for c in ix[ip[r]:ip[r + 1]]:
+                w = int(ent[t])
+                t += 1
+                if c == r:
+                    assert w == 0xffffffff
+                    continue
+                assert (w >> 16) & 63 == lr
+                at, got = r0 + (w & 0xffff) * (4 if H == 1 else 1), []
+                while True:
+                    v = int(rec[at])
+                    if H == 1:
+                        if (v & 0x7fff) // P < len(elems):
+                            e = int(elems[(v & 0x7fff) // P])
+                            assert set(el[e][list(pairs[(v & 0x7fff) % P])]) == {r, c}
+                            got.append(e)
+                        at += 1
+                        if (at - r0) % 4 == 0 and v & 0x8000:
+                            break
+                    else:
+                        e = int(elems[(v & 0x7fff) >> 4])
+                        assert (el[e][(v >> 2) & 3], el[e][v & 3]) == (r, c)
+                        got.append(e)
+                        at += 1
+                        if v & 0x8000:
+                            break
+                assert got == holds[(r, c)]
