@@ -208,6 +208,15 @@ int tm_node_lists(const int32_t* elements, int64_t n_elements, int32_t n_basis, 
                   int32_t* cnt, uint32_t* nrec, void* stream);
 
 /*
+ * flags[0] (flags[1]) is set to 1 when array a (b) holds a nan or an inf, and
+ * left alone otherwise.  flags: memory the device can write (pinned host
+ * memory or device memory); the caller clears it and waits for the stream.
+ * Either array may be empty.
+ */
+int tm_check_finite(int32_t dtype_a, int64_t n_a, const void* a, int32_t dtype_b, int64_t n_b, const void* b,
+                    int32_t* flags, void* stream);
+
+/*
  * Backward (adjoint) assembly.  Given dL/d(values) of a tm_assemble call
  * with the same plan and args, writes per-(patch, element) partial gradients:
  *   pair_dX[n_pairs][B][D]          dL/dX of the element's nodes;

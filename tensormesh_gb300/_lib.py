@@ -44,7 +44,7 @@ EXPORTS = [
     "tm_fcg_workspace_doubles", "tm_fcg_twolevel_iterations", "tm_kp_count", "tm_kp_fill",
     "tm_sell_fill", "tm_spmv_sell",
     "tm_gather_workspace_bytes", "tm_assemble_gather", "tm_node_lists",
-    "tm_group_count", "tm_group_fill",
+    "tm_group_count", "tm_group_fill", "tm_check_finite",
 ]
 
 P = ctypes.c_void_p
@@ -133,6 +133,7 @@ def _declare(lib):
         "tm_group_count": [i32, i64, i32, i32, P, P, P, P, P, P, P, P, P],
         "tm_group_fill": [i32, i64, i32, i32, P, P, P, P, P, P, P, P, P, P, P],
         "tm_node_lists": [P, i64, i32, i64, P, P, P, P],
+        "tm_check_finite": [i32, i64, P, i32, i64, P, P, P],
         "tm_quadrature_points": [i32, i32, i32, P, P, P, i64, P, P],
         "tm_spmv_csr": [i32, i64, i64, P, P, P, P, P, P],
         "tm_pcg_jacobi": [i32, i64, P, P, P, P, P, ctypes.c_double, ctypes.c_double, i32, P, i64, P],

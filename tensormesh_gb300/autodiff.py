@@ -7,7 +7,7 @@ import torch
 from . import _lib
 from . import element as E_
 from .sparse import SparseMatrix
-from .validate import check_finite
+from .validate import finite_check
 
 _FORM_CODE = {"laplace": _lib.TM_FORM_LAPLACE, "mass": _lib.TM_FORM_MASS, "elasticity": _lib.TM_FORM_ELASTICITY}
 
@@ -33,19 +33,17 @@ def assemble_matrix(asm, form, points, element_data, point_data, scalar_data) ->
     H = topo.dim if form.kind == "elasticity" else 1
     dptr, dind = topo.dof_pattern(H)
     kind, coef, scal = _coefficient(form, points, element_data, point_data, scalar_data)
-    check_finite((("points", points), ("the coefficient", coef)))
-    pts = points.detach().contiguous()
-    out = torch.empty(dind.shape[0], dtype=points.dtype, device=points.device)
     from .adjoint import needs_grad, AssembleMatrixFn
-    if needs_grad(points, coef):
-        values = AssembleMatrixFn.apply(points, coef, asm, form, kind, scal)
-    else:
-        _tables = E_.kernel_tables  # noqa: F841  (keeps symbol referenced)
-        from .assemble import launch_assemble
-        launch_assemble(topo, _FORM_CODE[form.kind], pts, out, quadrature_order=asm.quadrature_order,
-                        coef_kind=kind, coef=None if coef is None else coef.detach(), scal=(scal, 0.0, 0.0),
-                        lame=(form.lam, form.mu), precision=asm.precision, slot_budget=asm.slot_budget)
-        values = out
+    with finite_check(("points", points), ("the coefficient", coef)):
+        if needs_grad(points, coef):
+            values = AssembleMatrixFn.apply(points, coef, asm, form, kind, scal)
+        else:
+            from .assemble import launch_assemble
+            values = torch.empty(dind.shape[0], dtype=points.dtype, device=points.device)
+            launch_assemble(topo, _FORM_CODE[form.kind], points.detach().contiguous(), values,
+                            quadrature_order=asm.quadrature_order, coef_kind=kind,
+                            coef=None if coef is None else coef.detach(), scal=(scal, 0.0, 0.0),
+                            lame=(form.lam, form.mu), precision=asm.precision, slot_budget=asm.slot_budget)
     n = topo.n_points * H
     return SparseMatrix(values, shape=(n, n), indptr=dptr, indices=dind)
 
@@ -102,15 +100,15 @@ def _dtype(t):
 def assemble_load(asm, form, points, point_data, scalar_data) -> torch.Tensor:
     topo = asm.topology
     kind, coef, scal, H = _load_coefficient(asm, form, points, point_data, scalar_data)
-    check_finite((("points", points), ("the load coefficient", coef)))
     from .adjoint import needs_grad, AssembleLoadFn
-    if needs_grad(points, coef):
-        out = AssembleLoadFn.apply(points, coef, asm, kind, tuple(scal), H)
-    else:
-        from .assemble import launch_assemble
-        out = torch.empty(topo.n_points * H, dtype=points.dtype, device=points.device)
-        launch_assemble(topo, _lib.TM_FORM_LOAD, points.detach().contiguous(), out,
-                        quadrature_order=asm.quadrature_order, coef_kind=kind,
-                        coef=None if coef is None else coef.detach(), scal=tuple(scal), n_comp=H,
-                        precision=asm.precision)
+    with finite_check(("points", points), ("the load coefficient", coef)):
+        if needs_grad(points, coef):
+            out = AssembleLoadFn.apply(points, coef, asm, kind, tuple(scal), H)
+        else:
+            from .assemble import launch_assemble
+            out = torch.empty(topo.n_points * H, dtype=points.dtype, device=points.device)
+            launch_assemble(topo, _lib.TM_FORM_LOAD, points.detach().contiguous(), out,
+                            quadrature_order=asm.quadrature_order, coef_kind=kind,
+                            coef=None if coef is None else coef.detach(), scal=tuple(scal), n_comp=H,
+                            precision=asm.precision)
     return out

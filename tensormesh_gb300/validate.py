@@ -9,12 +9,14 @@ matrices.  Here both are rejected before any kernel launch:
   pattern is built (``IndexError``);
 * floating inputs of a call (points, per-element / per-point / per-quadrature
   coefficients): all finite (``ValueError`` naming the input).  This check
-  reads the inputs on the device and waits for the answer (one host
-  synchronisation per call); ``set_input_checks(False)`` turns it off for
-  callers that pipeline many calls and validate their data elsewhere.
+  reads the inputs on the device (one launch, tm_check_finite) and waits for
+  the answer (one host synchronisation per call, after the call's own kernels
+  are queued); ``set_input_checks(False)`` turns it off for callers that
+  pipeline many calls and validate their data elsewhere.
 """
 from __future__ import annotations
 
+import threading
 from typing import Iterable, Optional, Tuple
 
 import torch
@@ -41,6 +43,64 @@ def check_connectivity(elements: torch.Tensor, n_points: int) -> None:
         row = int(torch.nonzero((elements < 0) | (elements >= n_points), as_tuple=True)[0][0])
         raise IndexError(f"element {row} refers to node {bad}, outside [0, {n_points}) "
                          f"(the mesh has {n_points} points)")
+
+
+_KERNEL_DTYPES = {torch.float32: 0, torch.float64: 1}   # TM_F32, TM_F64
+_LOCAL = threading.local()
+
+
+def _flag_buffer(device):
+    """This thread's pinned flags and event for ``device``."""
+    table = _LOCAL.__dict__.setdefault("flags", {})
+    key = str(device)
+    if key not in table:
+        flags = torch.zeros(2, dtype=torch.int32, pin_memory=True)
+        table[key] = (flags, flags.numpy(), torch.cuda.Event())
+    return table[key]
+
+
+class finite_check:
+    """Context that checks named inputs while the body queues its kernels: the
+    check is launched on entry, the answer is waited for on exit (ValueError
+    naming the first input that holds a nan or inf).
+
+        with finite_check(("points", points), ("the coefficient", coef)):
+            launch(...)
+    """
+
+    def __init__(self, *items: Tuple[str, Optional[torch.Tensor]]):
+        self.items, self.pending = items, None
+
+    def __enter__(self):
+        if not _CHECK_FINITE:
+            return self
+        named = [(n, t.detach()) for n, t in self.items
+                 if t is not None and torch.is_tensor(t) and t.is_floating_point() and t.numel()]
+        if not named:
+            return self
+        dev = named[0][1].device
+        if (dev.type != "cuda" or len(named) > 2 or
+                any(t.device != dev or t.dtype not in _KERNEL_DTYPES or not t.is_contiguous() for _, t in named)):
+            check_finite(self.items)
+            return self
+        from . import _lib
+        flags, view, event = _flag_buffer(dev)
+        view[:] = 0
+        (_, a), (_, b) = named[0], (named[1] if len(named) > 1 else (None, None))
+        _lib.call("tm_check_finite", _KERNEL_DTYPES[a.dtype], a.numel(), a.data_ptr(),
+                  _KERNEL_DTYPES[a.dtype if b is None else b.dtype], 0 if b is None else b.numel(),
+                  0 if b is None else b.data_ptr(), flags.data_ptr(), _lib.stream_handle(dev))
+        event.record(torch.cuda.current_stream(dev))
+        self.pending = (named, view, event)
+        return self
+
+    def __exit__(self, kind, *_):
+        if self.pending is None:
+            return
+        named, view, event = self.pending
+        event.synchronize()   # also when the body raised: the flags serve this thread's next check
+        if kind is None and view.any():
+            raise ValueError(f"{named[0 if view[0] else 1][0]} holds a non-finite value (nan or inf)")
 
 
 def check_finite(items: Iterable[Tuple[str, Optional[torch.Tensor]]]) -> None:
