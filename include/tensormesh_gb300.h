@@ -237,6 +237,19 @@ typedef struct tm_backward_args {
 int tm_assemble_backward(const tm_patch_plan* plan, const tm_assemble_args* args, const tm_backward_args* bw,
                          void* stream);
 
+/*
+ * The same per element for P1 Laplace and elasticity matrices (other elements
+ * and forms: TM_ERR_UNSUPPORTED): el_dX[E][B][D]; el_dcoef TM_COEF_ELEMENT
+ * [E], TM_COEF_POINT [E][B], TM_COEF_QUAD [E][Q].  Either may be NULL.  The
+ * plan needs elements and indptr; slots is tm_pattern_fill's slot map.
+ * tm_node_sum adds the incidences of every node (tm_node_lists) in element
+ * order: dst[node][w] = sum src[nrec][w].
+ */
+int tm_backward_gather(const tm_gather_plan* plan, const int64_t* slots, const tm_assemble_args* args,
+                       const void* grad_out, void* el_dX, void* el_dcoef, void* stream);
+int tm_node_sum(int32_t dtype, int64_t n_points, const int64_t* nptr, const uint32_t* nrec, int32_t width,
+                const void* src, void* dst, void* stream);
+
 /* dst[s][w] = sum_{k = ptr[s]}^{ptr[s+1]-1} src[perm[k]][w], in k order
  * (deterministic segmented reduction). */
 int tm_segment_sum(int32_t dtype, int64_t n_segments, const int64_t* ptr, const int64_t* perm, int32_t width,

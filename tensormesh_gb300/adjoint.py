@@ -82,6 +82,11 @@ def _args(topo, form_code, points, quadrature_order, kind, coef, scal, lame, n_c
 def run_backward(topo, form_code, points, quadrature_order, kind, coef, scal, lame, n_comp, grad_out,
                  want_points: bool, want_coef: bool):
     """Returns (grad_points [N, D] or None, grad_coef (coef's shape) or None)."""
+    if topo.n_basis == topo.dim + 1 and form_code in (_lib.TM_FORM_LAPLACE, _lib.TM_FORM_ELASTICITY):
+        lists = topo.gather.struct(0)
+        if lists is not None:
+            return _run_backward_p1(topo, lists, form_code, points, quadrature_order, kind, coef, scal, lame,
+                                    grad_out, want_points, want_coef)
     Hb = topo.dim if form_code == _lib.TM_FORM_ELASTICITY else 1
     maps, plan_struct = backward_maps(topo, Hb)
     P, B, D = maps.n_pairs, topo.n_basis, topo.dim
@@ -113,6 +118,37 @@ def run_backward(topo, form_code, points, quadrature_order, kind, coef, scal, la
         else:
             gc = segment_sum(maps.elem_ptr, maps.elem_perm, pair_dc, Q * comp)
         gc = gc.view(coef.shape)
+    return gp, gc
+
+
+def node_sum(lists, src, width):
+    """src [E * B, width] summed to the nodes, elements ascending."""
+    out = torch.empty(lists.n_points * width, dtype=src.dtype, device=src.device)
+    _lib.call("tm_node_sum", _dt(src), lists.n_points, lists.nptr, lists.nrec, width, src.data_ptr(), out.data_ptr(),
+              _lib.stream_handle(src.device))
+    return out
+
+
+def _run_backward_p1(topo, lists, form_code, points, quadrature_order, kind, coef, scal, lame, grad_out,
+                     want_points: bool, want_coef: bool):
+    """run_backward of P1 Laplace and elasticity matrices: every element once
+    (tm_backward_gather), reduced to the nodes by tm_node_sum."""
+    E, B, D = topo.n_elements, topo.n_basis, topo.dim
+    Q = E_.n_quadrature(topo.element_type, quadrature_order)
+    dev, dtype = points.device, points.dtype
+    pts = points.detach().contiguous()
+    c = None if coef is None else coef.detach().contiguous()
+    a, _tables = _args(topo, form_code, pts, quadrature_order, kind, c, scal, lame, 1)
+    g = grad_out.detach().to(dtype).contiguous()
+    el_dx = torch.empty(E * B * D, dtype=dtype, device=dev) if want_points else None
+    size = {_lib.TM_COEF_ELEMENT: E, _lib.TM_COEF_POINT: E * B, _lib.TM_COEF_QUAD: E * Q}.get(kind)
+    el_dc = torch.empty(size, dtype=dtype, device=dev) if want_coef and size is not None else None
+    _lib.call("tm_backward_gather", lists, topo.pattern.slots.data_ptr(), a, g.data_ptr(), _lib.ptr(el_dx),
+              _lib.ptr(el_dc), _lib.stream_handle(dev))
+    gp = node_sum(lists, el_dx, D).view(topo.n_points, D) if el_dx is not None else None
+    gc = None
+    if el_dc is not None:
+        gc = (node_sum(lists, el_dc, 1) if kind == _lib.TM_COEF_POINT else el_dc).view(coef.shape)
     return gp, gc
 
 

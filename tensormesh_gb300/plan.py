@@ -470,7 +470,8 @@ class GatherPlan:
         return bool(bad)
 
     def struct(self, H: int):
-        """ctypes view with the groups for H x H blocks, or None."""
+        """ctypes view with the groups for H x H blocks (H = 0: the lists
+        without groups), or None."""
         if not self.ok:
             return None
         if H not in self._structs:
@@ -478,7 +479,18 @@ class GatherPlan:
         s = self._structs[H]
         return None if s is None else s[0]
 
+    def _view(self, rows=0, max_entries=0, max_elems=0, **groups):
+        s = _lib.GatherPlan()
+        s.n_elements, s.n_points = self.elements.shape[0], self.pattern.n_points
+        s.rows_per_cta, s.max_entries, s.max_elems = rows, max_entries, max_elems
+        keep = dict(elements=self.elements, indptr=self.pattern.indptr, nptr=self.nptr, nrec=self.nrec, **groups)
+        for name, t in keep.items():
+            setattr(s, name, t.data_ptr())
+        return s, keep
+
     def _groups(self, H: int):
+        if H == 0:
+            return self._view()
         E, B = self.elements.shape
         N, dev, pat = self.pattern.n_points, self.elements.device, self.pattern
         quads = int(H == 1)
@@ -508,10 +520,4 @@ class GatherPlan:
         grec = torch.zeros(n_rec + 8, dtype=torch.int16, device=dev)
         _lib.call("tm_group_fill", B, N, rows, quads, *lists, base.data_ptr(), gelem.data_ptr(), gent.data_ptr(),
                   grec.data_ptr(), stream)
-        s = _lib.GatherPlan()
-        s.n_elements, s.n_points, s.rows_per_cta, s.max_entries, s.max_elems = E, N, rows, most[1], most[0]
-        keep = dict(elements=self.elements, indptr=pat.indptr, nptr=self.nptr, nrec=self.nrec, order=self.order,
-                    base=base, gelem=gelem, gent=gent, grec=grec)
-        for name, t in keep.items():
-            setattr(s, name, t.data_ptr())
-        return s, keep
+        return self._view(rows, most[1], most[0], order=self.order, base=base, gelem=gelem, gent=gent, grec=grec)
