@@ -50,8 +50,14 @@ class _NeoHookeanEnergy(torch.autograd.Function):
                   points.data_ptr(), topo.elements.data_ptr(), n_el, uu.data_ptr(), float(mu), float(lam),
                   e_el.data_ptr(), 0 if g_el is None else g_el.data_ptr(), _lib.stream_handle(dev))
         if want:
-            ptr, perm = _node_maps(topo)
-            ctx.save_for_backward(segment_sum(ptr, perm, g_el, D).view(topo.n_points, D))
+            lists = topo.gather.struct(0)
+            if lists is not None:
+                from .adjoint import node_sum
+                total = node_sum(lists, g_el, D)
+            else:
+                ptr, perm = _node_maps(topo)
+                total = segment_sum(ptr, perm, g_el, D)
+            ctx.save_for_backward(total.view(topo.n_points, D))
         ctx.keep = tables
         return e_el.sum().to(points.dtype)
 
