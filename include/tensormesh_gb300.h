@@ -163,7 +163,11 @@ int tm_assemble(const tm_patch_plan* plan, const tm_assemble_args* args, void* s
  *   order[N]               the rows in group order
  *   base[3*(G+1)]          first gelem, gent and grec of each group
  *   gelem[], gent[], grec[]
- * max_entries, max_elems: most CSR entries and elements of one group.  Calls that run at the same time need a work array each.
+ *   P2: lists of every CSR position (tm_gather_fill); rows_per_cta consecutive
+ *   rows form a CTA:
+ *   ent[nnz], rec[]
+ * max_entries, max_elems: most CSR entries and elements of one group (P2:
+ * entries of one CTA's rows).  Calls that run at the same time need a work array each.
  */
 typedef struct tm_gather_plan {
   int32_t n_elements;
@@ -181,6 +185,8 @@ typedef struct tm_gather_plan {
   const int32_t* gelem;
   const uint32_t* gent;
   const uint16_t* grec;
+  const uint32_t* ent;
+  const uint32_t* rec;
 } tm_gather_plan;
 
 /* bytes of `work`, or minus a status (TM_ERR_UNSUPPORTED: use tm_assemble) */
@@ -192,12 +198,21 @@ int tm_assemble_gather(const tm_gather_plan* plan, const tm_assemble_args* args,
 /*
  * The plan's lists.  slots[E*B*B] is tm_pattern_fill's slot map.
  * tm_node_lists counts with nptr == NULL, then fills with the scanned nptr.
+ * tm_gather_count writes the list length of every CSR position (zero on and
+ * below the diagonal); the caller scans cnt into start[nnz+1] (int64,
+ * exclusive) and allocates rec with start[nnz] + 8 words; tm_gather_fill
+ * consumes cnt.  Limits: E * B * (B - 1) / 2 < 2^30 - 1.  *bad is set when an
+ * element repeats a node (no lists then).
  * tm_group_count writes [distinct elements, entries, records] of every group
  * and sets *bad when a group exceeds the record format (use fewer rows); base
  * is the exclusive scan of the sizes, cnt[nnz] is scratch that tm_group_fill
  * consumes.  quads = 1: the records of scalar forms, 0: of elasticity blocks.
  * rows_per_group <= 64.
  */
+int tm_gather_count(const int32_t* elements, int64_t n_elements, int32_t n_basis, int64_t nnz, const int64_t* slots,
+                    int32_t* cnt, int32_t* bad, void* stream);
+int tm_gather_fill(const int32_t* elements, int64_t n_elements, int32_t n_basis, int64_t nnz, const int64_t* slots,
+                   const int64_t* start, int32_t* cnt, uint32_t* ent, uint32_t* rec, void* stream);
 int tm_group_count(int32_t n_basis, int64_t n_points, int32_t rows_per_group, int32_t quads, const int32_t* order,
                    const int64_t* nptr, const uint32_t* nrec, const int64_t* indptr, const int64_t* slots,
                    int32_t* cnt, int32_t* sizes, int32_t* bad, void* stream);

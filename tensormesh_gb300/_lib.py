@@ -43,7 +43,7 @@ EXPORTS = [
     "tm_sell_plan", "tm_pcg_sell_workspace_bytes", "tm_pcg_jacobi_sell",
     "tm_fcg_workspace_doubles", "tm_fcg_twolevel_iterations", "tm_kp_count", "tm_kp_fill",
     "tm_sell_fill", "tm_spmv_sell",
-    "tm_gather_workspace_bytes", "tm_assemble_gather", "tm_node_lists",
+    "tm_gather_workspace_bytes", "tm_assemble_gather", "tm_gather_count", "tm_gather_fill", "tm_node_lists",
     "tm_group_count", "tm_group_fill", "tm_check_finite",
     "tm_backward_gather", "tm_node_sum",
 ]
@@ -93,7 +93,7 @@ class GatherPlan(ctypes.Structure):
         ("rows_per_cta", ctypes.c_int32), ("max_entries", ctypes.c_int32),
         ("max_elems", ctypes.c_int32), ("pad0", ctypes.c_int32),
         ("elements", P), ("indptr", P), ("nptr", P), ("nrec", P), ("order", P), ("base", P),
-        ("gelem", P), ("gent", P), ("grec", P),
+        ("gelem", P), ("gent", P), ("grec", P), ("ent", P), ("rec", P),
     ]
 
 
@@ -131,6 +131,8 @@ def _declare(lib):
     sig = {
         "tm_assemble": [ctypes.POINTER(PatchPlan), ctypes.POINTER(AssembleArgs), P],
         "tm_assemble_gather": [ctypes.POINTER(GatherPlan), ctypes.POINTER(AssembleArgs), P, i64, P],
+        "tm_gather_count": [P, i64, i32, i64, P, P, P, P],
+        "tm_gather_fill": [P, i64, i32, i64, P, P, P, P, P, P],
         "tm_group_count": [i32, i64, i32, i32, P, P, P, P, P, P, P, P, P],
         "tm_group_fill": [i32, i64, i32, i32, P, P, P, P, P, P, P, P, P, P, P],
         "tm_node_lists": [P, i64, i32, i64, P, P, P, P],

@@ -39,8 +39,9 @@ PRECISION = {"emulated": _lib.TM_PREC_EMULATED, "native": _lib.TM_PREC_NATIVE}
 
 
 class MeshTopology:
-    """Pattern + patch plan of one connectivity, shared by every assembler
-    built on it (the analogue of the reference's ``edges`` + projector)."""
+    """Pattern and assembly plan (element lists, or the patch plan) of one
+    connectivity, shared by every assembler built on it (the analogue of the
+    reference's ``edges`` + projector)."""
 
     def __init__(self, elements: torch.Tensor, points: torch.Tensor, element_type: str):
         self.element_type = element_type
@@ -59,11 +60,14 @@ class MeshTopology:
         self.timings["pattern_s"] = _now(elements.device) - t0
         self._coords = points.detach()
         self._plans = {}
-        self.plan, self._plan_struct = self.plan_for(1)
-        t0 = _now(elements.device)
-        self.gather = GatherPlan(self.elements, self._coords, self.pattern)
-        self.gather.struct(1)
-        self.timings["gather_s"] = _now(elements.device) - t0
+        self._gather = None
+        self.scratch_bytes = {}
+        # what the calls on this mesh run on: lists of the element-once
+        # kernels, or the patch plan (each is built on first use otherwise)
+        if self.element_once:
+            self.gather.struct(1)
+        else:
+            self.plan_for(1)
         self._block = {}
         self._incidence = None
 
@@ -84,6 +88,31 @@ class MeshTopology:
             self.timings[f"plan_{budget}_s"] = _now(self._coords.device) - t0
         return self._plans[budget]
 
+    @property
+    def element_once(self) -> bool:
+        """Whether float64 emulated and float32 assembly runs element-once."""
+        return self.elements.is_cuda and self.n_elements >= _GATHER_MIN_ELEMENTS[self.element_type] and self.gather.ok
+
+    @property
+    def gather(self) -> GatherPlan:
+        if self._gather is None:
+            self._refusals()
+            t0 = _now(self.elements.device)
+            self._gather = GatherPlan(self.elements, self._coords, self.pattern)
+            self.timings["gather_s"] = _now(self.elements.device) - t0
+        return self._gather
+
+    def _refusals(self):
+        """The sizes the patch plan refuses, refused without building it."""
+        if self.n_elements and int((self.pattern.indptr[1:] - self.pattern.indptr[:-1]).max()) > 255:
+            raise NotImplementedError("a CSR row longer than 255 entries is not supported by the patch plan")
+        if self.n_elements * self.n_basis >= 2**31:
+            raise NotImplementedError("mesh too large for 32-bit plan offsets")
+
+    @property
+    def plan(self) -> PatchPlan:
+        return self.plan_for(1)[0]
+
     def dof_pattern(self, H: int):
         if H not in self._block:
             self._block[H] = block_pattern(self.pattern.indptr, self.pattern.indices, H)
@@ -91,7 +120,7 @@ class MeshTopology:
 
     @property
     def plan_struct(self):
-        return self._plan_struct
+        return self.plan_for(1)[1]
 
 
 def _now(device) -> float:
@@ -144,23 +173,28 @@ def _mesh_single_type(mesh):
     return etype, elements
 
 
-_GATHER_MIN_ELEMENTS = 16384
+# Fewest elements for the element-once kernels.  Below, the one-launch patch
+# kernel takes less host time than three launches and a scratch allocation
+# (us a call, patch / element-once): P1, 24576 tetrahedra 92 / 104 with the GPU
+# idle half of it, and element-once ahead from there in GPU time; P2 triangles
+# 2048 elasticity 113 / 104; P2 tetrahedra 48 elements 166 / 109 (Laplace),
+# 3072 elements 581 / 107.
+_GATHER_MIN_ELEMENTS = {"triangle": 16384, "tetra": 16384, "triangle6": 2048, "tetra10": 0}
 
 
 def _gather_scratch(topo: MeshTopology, a: _lib.AssembleArgs, H: int):
     """(plan, scratch) of the element-once assembly, (None, None) where the
-    patch kernels run: native FP64, forms without element-once kernels, meshes
-    whose lists do not apply, scratch that does not fit the device, and small
-    meshes, whose call is bound by its launches (one against three: 245 and
-    269 us at 512 triangles; 260 and 290 us at 3000 tetrahedra)."""
-    if topo.n_elements < _GATHER_MIN_ELEMENTS:
+    patch kernels run: small meshes, native FP64, meshes whose lists do not
+    apply, and scratch that does not fit the device."""
+    if not topo.element_once or (a.dtype == _lib.TM_F64 and a.precision != _lib.TM_PREC_EMULATED):
         return None, None
-    if a.dtype == _lib.TM_F64 and a.precision != _lib.TM_PREC_EMULATED:
-        return None, None
-    n = int(_lib.load().tm_gather_workspace_bytes(a.element, a.form, a.dtype, a.n_comp, topo.n_elements))
+    key = (a.form, a.dtype, a.n_comp)
+    n = topo.scratch_bytes.get(key)
+    if n is None:
+        n = topo.scratch_bytes[key] = int(_lib.load().tm_gather_workspace_bytes(a.element, *key, topo.n_elements))
     if n < 0:
         return None, None
-    plan = topo.gather.struct(H)
+    plan = topo.gather.struct(0 if a.form == _lib.TM_FORM_LOAD else H)
     if plan is None:
         return None, None
     try:
@@ -229,6 +263,8 @@ class ElementAssembler(_AssemblerDevice, nn.Module):
     def __init__(self, topology: MeshTopology, points: torch.Tensor, quadrature_order: int, *args, **kwargs):
         super().__init__()
         self.topology = topology
+        if self.precision == "native":
+            topology.plan_for(1)
         self.quadrature_order = int(quadrature_order)
         self.register_buffer("points", points, persistent=False)
         self.element_types = [topology.element_type]

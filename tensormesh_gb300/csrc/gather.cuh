@@ -22,11 +22,17 @@
 // native FP64 by the same thread or block.
 #pragma once
 #include "p1tet_fast.cuh"
+#include <climits>
 
 namespace tmg {
 namespace ga {
 
 constexpr uint32_t kDiag = 0xffffffffu;   // entry word of a diagonal position
+// lists of P2 meshes
+constexpr uint32_t kLower = 0x80000000u;  // entry word: below the diagonal (the list is the mirror entry's)
+constexpr uint32_t kEnd = 0x80000000u;    // record: last of its list
+constexpr uint32_t kFlip = 0x40000000u;   // record: local pair (a, b), a < b, has node a > node b
+constexpr uint32_t kIdx = 0x3fffffffu;    // record: element * pairs + pair
 constexpr int kWindow = 60;
 
 struct Head {
@@ -64,20 +70,27 @@ inline Scratch scratch_of(void* work, int64_t n_el, int64_t vals_bytes) {
 // Biased exponent field of a double (0 for zero and subnormals).
 TM_D int dexp(double x) { return (int)(((unsigned)__double2hiint(x) >> 20) & 0x7ffu); }
 
-// x 2^(1023 - emax) as a pair, emax >= the biased exponent of x: hi = x
-// truncated to 24 significant bits, lo = the remaining 29 bits rounded to
-// float (2^-48 of x).  Values below 2^-90 of the scale give 0.
+// x 2^(1023 - emax) as a pair, emax >= the biased exponent of x: hi = x rounded
+// to 24 significant bits (half up), lo = the rest rounded to float (2^-49 of
+// x).  Values below 2^-90 of the scale give 0.  Rounding, not truncating, hi
+// matters: products drop lo * lo, and |lo| <= 2^-24 |hi| keeps that below
+// 2^-48 of the product.
 TM_D L2 l2_scaled(double x, int emax) {
   const unsigned hw = (unsigned)__double2hiint(x), lw = (unsigned)__double2loint(x);
   const int de = (int)((hw >> 20) & 0x7ffu) - emax;
   const unsigned sgn = hw & 0x80000000u;
   const unsigned m = __funnelshift_l(lw, hw, 3) & 0x7fffffu;
-  const float h = __uint_as_float(sgn | ((unsigned)(de + 127) << 23) | m);
+  const unsigned up = (lw >> 28) & 1u;
+  const float h = __uint_as_float((sgn | ((unsigned)(de + 127) << 23) | m) + up);
   const float sc = __uint_as_float(sgn | ((unsigned)max(de + 75, 0) << 23));
-  const float l = __fmul_rn(__int2float_rn((int)(lw & 0x1fffffffu)), sc);
+  const float l = __fmul_rn(__int2float_rn((int)(lw & 0x1fffffffu) - (int)(up << 29)), sc);
   const bool tiny = de < -90;
   return L2{tiny ? 0.f : h, tiny ? 0.f : l};
 }
+
+// Renormalised value (|lo| <= 2^-24 |hi|) after sums that may have cancelled.
+template <class A> TM_D A norm(A a) { return a; }
+template <> TM_D L2 norm<L2>(L2 a) { return l2_norm(a); }
 
 // Scaled input in arithmetic A (the native pass scales exactly).
 template <class A> TM_D A scaled(double x, int emax);

@@ -3,6 +3,14 @@
 //
 //   nptr, nrec   e * B + a of every incidence of a node, ascending
 //
+// for P2 meshes, per node-level CSR position
+//
+//   ent[t]   kDiag, or the start of its list of records (a position below the
+//            diagonal names its mirror's list)
+//   rec[]    per position above the diagonal, contiguous: one record per
+//            element that holds the node pair, elements ascending, the last
+//            one marked
+//
 // and, for P1 meshes, the groups of rows described below.  Count, scan (by the
 // caller), fill with integer atomics, then a sort of every short list, so the
 // result does not depend on the order the atomics resolve in.
@@ -10,6 +18,77 @@
 
 namespace tmg {
 namespace ga {
+
+// local pair (a, b), a < b, of pair index k
+TM_D void pair_nodes(int k, int B, int& a, int& b) {
+  a = 0;
+  int left = B - 1;
+  while (k >= left) {
+    k -= left;
+    ++a;
+    --left;
+  }
+  b = a + 1 + k;
+}
+
+__global__ void list_count_kernel(const int32_t* __restrict__ el, int64_t n, int B, int P,
+                                  const int64_t* __restrict__ slots, int32_t* __restrict__ cnt, int32_t* bad) {
+  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;  // element * P + pair
+  if (i >= n) return;
+  const int64_t e = i / P;
+  int a, b;
+  pair_nodes((int)(i - e * P), B, a, b);
+  const int va = el[e * B + a], vb = el[e * B + b];
+  if (va == vb) {
+    atomicExch(bad, 1);  // a repeated node: the caller keeps the patch kernels
+    return;
+  }
+  const int64_t s = va < vb ? slots[(e * B + a) * B + b] : slots[(e * B + b) * B + a];
+  atomicAdd(cnt + s, 1);
+}
+
+__global__ void list_fill_kernel(const int32_t* __restrict__ el, int64_t n, int B, int P,
+                                 const int64_t* __restrict__ slots, const int64_t* __restrict__ start,
+                                 int32_t* __restrict__ cnt, uint32_t* __restrict__ ent, uint32_t* __restrict__ rec) {
+  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const int64_t e = i / P;
+  const int k = (int)(i - e * P);
+  int a, b;
+  pair_nodes(k, B, a, b);
+  const bool flip = el[e * B + a] > el[e * B + b];
+  const int64_t sab = slots[(e * B + a) * B + b], sba = slots[(e * B + b) * B + a];
+  const int64_t up = flip ? sba : sab, low = flip ? sab : sba;
+  const uint32_t s0 = (uint32_t)start[up];
+  // every element of the pair writes the same entry words
+  ent[up] = s0;
+  ent[low] = s0 | kLower;
+  if (b == a + 1) {
+    ent[slots[(e * B + a) * B + a]] = kDiag;
+    if (b == B - 1) ent[slots[(e * B + b) * B + b]] = kDiag;
+  }
+  const int at = atomicSub(cnt + up, 1) - 1;
+  rec[s0 + at] = (uint32_t)i | (flip ? kFlip : 0u);
+}
+
+// Sorts every list and marks its last record.  A list's length is the gap to
+// the next list's start.
+__global__ void list_sort_kernel(int64_t nnz, const int64_t* __restrict__ start, uint32_t* __restrict__ rec) {
+  const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (t >= nnz) return;
+  const int64_t s0 = start[t], s1 = start[t + 1];
+  if (s1 == s0) return;
+  for (int64_t i = s0 + 1; i < s1; ++i) {
+    const uint32_t v = rec[i];
+    int64_t j = i;
+    while (j > s0 && (rec[j - 1] & kIdx) > (v & kIdx)) {
+      rec[j] = rec[j - 1];
+      --j;
+    }
+    rec[j] = v;
+  }
+  rec[s1 - 1] |= kEnd;
+}
 
 __global__ void node_count_kernel(const int32_t* __restrict__ el, int64_t n, int32_t* __restrict__ cnt) {
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -233,6 +312,37 @@ group_fill_kernel(int rows_per_group, int n_points, int B, int quads, const int3
 
 }  // namespace ga
 }  // namespace tmg
+
+extern "C" int tm_gather_count(const int32_t* elements, int64_t n_elements, int32_t n_basis, int64_t nnz,
+                               const int64_t* slots, int32_t* cnt, int32_t* bad, void* stream) {
+  if (n_elements < 0 || n_basis < 2 || nnz < 0 || !cnt || !bad) return TM_ERR_INVALID;
+  if (n_elements > 0 && (!elements || !slots)) return TM_ERR_INVALID;
+  const int P = n_basis * (n_basis - 1) / 2;
+  if (n_elements * P >= (int64_t)tmg::ga::kIdx) return TM_ERR_INDEX;
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  if (cudaMemsetAsync(cnt, 0, sizeof(int32_t) * nnz, s) != cudaSuccess) return TM_ERR_CUDA;
+  if (cudaMemsetAsync(bad, 0, sizeof(int32_t), s) != cudaSuccess) return TM_ERR_CUDA;
+  const int64_t n = n_elements * P;
+  if (n > 0)
+    tmg::ga::list_count_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(elements, n, n_basis, P, slots, cnt, bad);
+  return cudaPeekAtLastError() == cudaSuccess ? TM_OK : TM_ERR_CUDA;
+}
+
+extern "C" int tm_gather_fill(const int32_t* elements, int64_t n_elements, int32_t n_basis, int64_t nnz,
+                              const int64_t* slots, const int64_t* start, int32_t* cnt, uint32_t* ent, uint32_t* rec,
+                              void* stream) {
+  if (n_elements < 0 || n_basis < 2 || nnz < 0) return TM_ERR_INVALID;
+  if (n_elements == 0 || nnz == 0) return TM_OK;
+  if (!elements || !slots || !start || !cnt || !ent || !rec) return TM_ERR_INVALID;
+  const int P = n_basis * (n_basis - 1) / 2;
+  if (n_elements * P >= (int64_t)tmg::ga::kIdx) return TM_ERR_INDEX;
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  const int64_t n = n_elements * P;
+  tmg::ga::list_fill_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(elements, n, n_basis, P, slots, start, cnt,
+                                                                        ent, rec);
+  tmg::ga::list_sort_kernel<<<(unsigned)((nnz + 255) / 256), 256, 0, s>>>(nnz, start, rec);
+  return cudaPeekAtLastError() == cudaSuccess ? TM_OK : TM_ERR_CUDA;
+}
 
 extern "C" int tm_node_lists(const int32_t* elements, int64_t n_elements, int32_t n_basis, int64_t n_points,
                              const int64_t* nptr, int32_t* cnt, uint32_t* nrec, void* stream) {

@@ -9,11 +9,10 @@ template <int D, bool kElast> int64_t p1_bytes(int dtype, int64_t n_el) {
   return n_el * p1_values<D, kElast>() * (dtype == TM_F64 ? 8 : 4);
 }
 
-int64_t p1_scratch_bytes(int element, int form, int dtype, int64_t n_el) {
+int64_t p1_value_bytes(int element, int form, int dtype, int64_t n_el) {
   const bool el = form == TM_FORM_ELASTICITY;
-  const int64_t v = element == TM_TRI3 ? (el ? p1_bytes<2, true>(dtype, n_el) : p1_bytes<2, false>(dtype, n_el))
-                                       : (el ? p1_bytes<3, true>(dtype, n_el) : p1_bytes<3, false>(dtype, n_el));
-  return 256 + up256((n_el + 31) / 32 * 4) + up256(v);
+  return element == TM_TRI3 ? (el ? p1_bytes<2, true>(dtype, n_el) : p1_bytes<2, false>(dtype, n_el))
+                            : (el ? p1_bytes<3, true>(dtype, n_el) : p1_bytes<3, false>(dtype, n_el));
 }
 
 // Clears the flag, sums the weights and sets the common exponent to that of
@@ -73,33 +72,3 @@ int assemble_p1(const tm_gather_plan& plan, const tm_assemble_args& a, void* wor
 
 }  // namespace ga
 }  // namespace tmg
-
-extern "C" int64_t tm_gather_workspace_bytes(int32_t element, int32_t form, int32_t dtype, int32_t n_comp,
-                                             int64_t n_elements) {
-  (void)n_comp;
-  if (n_elements < 0 || (dtype != TM_F32 && dtype != TM_F64)) return -TM_ERR_INVALID;
-  if (element != TM_TRI3 && element != TM_TET4) return -TM_ERR_UNSUPPORTED;
-  if (form != TM_FORM_LAPLACE && form != TM_FORM_ELASTICITY) return -TM_ERR_UNSUPPORTED;
-  return tmg::ga::p1_scratch_bytes(element, form, dtype, n_elements);
-}
-
-extern "C" int tm_assemble_gather(const tm_gather_plan* plan, const tm_assemble_args* args, void* work,
-                                  int64_t work_bytes, void* stream) {
-  if (!plan || !args) return TM_ERR_INVALID;
-  if (plan->n_elements < 0 || plan->n_points < 0) return TM_ERR_INVALID;
-  if (args->dtype != TM_F32 && args->dtype != TM_F64) return TM_ERR_INVALID;
-  if (args->n_quad < 1 || args->n_quad > 11) return TM_ERR_INVALID;
-  if (args->coef_kind < TM_COEF_SCALAR || args->coef_kind > TM_COEF_QUAD) return TM_ERR_INVALID;
-  if (args->dtype == TM_F64 && args->precision != TM_PREC_EMULATED) return TM_ERR_UNSUPPORTED;
-  const int64_t need = tm_gather_workspace_bytes(args->element, args->form, args->dtype, args->n_comp,
-                                                 plan->n_elements);
-  if (need < 0) return (int)-need;
-  if (plan->n_elements == 0) return TM_OK;
-  if (!args->tables || !args->points || !args->out || !work) return TM_ERR_INVALID;
-  if (!plan->elements || !plan->indptr || !plan->order || !plan->base || !plan->gelem || !plan->gent || !plan->grec)
-    return TM_ERR_INVALID;
-  if (args->coef_kind != TM_COEF_SCALAR && !args->coef) return TM_ERR_INVALID;
-  if (plan->n_points < 1 || plan->rows_per_cta < 1 || plan->max_entries < 1 || plan->max_elems < 1) return TM_ERR_INVALID;
-  if (work_bytes < need) return TM_ERR_INDEX;
-  return tmg::ga::assemble_p1(*plan, *args, work, static_cast<cudaStream_t>(stream));
-}

@@ -116,9 +116,9 @@ TM_D bool p1_element(const A (&d)[D][D], A cw, A (&out)[p1_values<D, kElast>()])
     det = P::sub(P::mul(d[0][0], d[1][1]), P::mul(d[0][1], d[1][0]));
   } else {
     auto cross = [](const A* u, const A* v, A* o) {
-      o[0] = P::sub(P::mul(u[1], v[2]), P::mul(u[2], v[1]));
-      o[1] = P::sub(P::mul(u[2], v[0]), P::mul(u[0], v[2]));
-      o[2] = P::sub(P::mul(u[0], v[1]), P::mul(u[1], v[0]));
+      o[0] = norm(P::sub(P::mul(u[1], v[2]), P::mul(u[2], v[1])));
+      o[1] = norm(P::sub(P::mul(u[2], v[0]), P::mul(u[0], v[2])));
+      o[2] = norm(P::sub(P::mul(u[0], v[1]), P::mul(u[1], v[0])));
     };
     cross(d[1], d[2], C[0]);
     cross(d[2], d[0], C[1]);

@@ -423,9 +423,9 @@ class PatchPlan:
 
 class GatherPlan:
     """Lists of the element-once assembly (tm_assemble_gather), built on the
-    device by the project's kernels: the incidences of every node and, for P1
-    meshes, groups of rows that are neighbours in space with the elements they
-    touch.  ``ok`` is False where the lists do not apply (an element that
+    device by the project's kernels: the incidences of every node, for P1
+    meshes groups of rows that are neighbours in space with the elements they
+    touch, for P2 meshes the elements of every CSR position.  ``ok`` is False where the lists do not apply (an element that
     repeats a node, or sizes past their index types); the patch kernels run
     then."""
 
@@ -443,8 +443,9 @@ class GatherPlan:
         dev = elements.device
         self.pattern, self.elements = pattern, elements
         self._structs = {}
-        self.ok = dev.type == "cuda" and E > 0 and B <= 4 and E * B < 2**31 - 1 and \
-            pattern.nnz < 2**31 - 1 and not self._repeats(elements)
+        self.p1 = B <= 4
+        self.ok = dev.type == "cuda" and E > 0 and E * B < 2**31 - 1 and pattern.nnz < 2**31 - 1 and \
+            E * (B * (B - 1) // 2) < (1 << 30) - 1 and not self._repeats(elements)
         if not self.ok:
             return
         s = _lib.stream_handle(dev)
@@ -456,6 +457,8 @@ class GatherPlan:
         self.nrec = torch.empty(E * B, dtype=torch.int32, device=dev)
         _lib.call("tm_node_lists", elements.data_ptr(), E, B, N, self.nptr.data_ptr(), ncnt.data_ptr(),
                   self.nrec.data_ptr(), s)
+        if not self.p1:
+            return
         c = points.detach().to(torch.float64).contiguous()
         key = morton_keys(c, c.min(0).values.contiguous(), c.max(0).values.contiguous(), 63 // c.shape[1])
         self.order = torch.argsort(key, stable=True).to(torch.int32)
@@ -479,6 +482,34 @@ class GatherPlan:
         s = self._structs[H]
         return None if s is None else s[0]
 
+    def _lists(self, H: int):
+        """P2: the record lists of every CSR position (shared by all forms) and
+        the rows a CTA sums: 64, fewer where their blocks fill shared memory."""
+        E, B = self.elements.shape
+        N, pat, dev = self.pattern.n_points, self.pattern, self.elements.device
+        if not hasattr(self, "ent"):
+            cnt = torch.empty(pat.nnz, dtype=torch.int32, device=dev)
+            bad = torch.empty(1, dtype=torch.int32, device=dev)
+            stream = _lib.stream_handle(dev)
+            _lib.call("tm_gather_count", self.elements.data_ptr(), E, B, pat.nnz, pat.slots.data_ptr(),
+                      cnt.data_ptr(), bad.data_ptr(), stream)
+            start = torch.zeros(pat.nnz + 1, dtype=torch.int64, device=dev)
+            torch.cumsum(cnt, 0, out=start[1:])
+            ent = torch.empty(pat.nnz, dtype=torch.int32, device=dev)
+            self.rec = torch.zeros(E * (B * (B - 1) // 2) + 8, dtype=torch.int32, device=dev)
+            _lib.call("tm_gather_fill", self.elements.data_ptr(), E, B, pat.nnz, pat.slots.data_ptr(),
+                      start.data_ptr(), cnt.data_ptr(), ent.data_ptr(), self.rec.data_ptr(), stream)
+            self.ent = ent
+        rows = 64
+        while True:
+            edge = torch.arange(0, N + rows, rows, device=dev).clamp_(max=N)
+            at = pat.indptr[edge]
+            most = int((at[1:] - at[:-1]).max())
+            if rows == 1 or most * H * H * 8 <= 64 * 1024:
+                break
+            rows //= 2
+        return self._view(rows, most, ent=self.ent, rec=self.rec)
+
     def _view(self, rows=0, max_entries=0, max_elems=0, **groups):
         s = _lib.GatherPlan()
         s.n_elements, s.n_points = self.elements.shape[0], self.pattern.n_points
@@ -491,6 +522,8 @@ class GatherPlan:
     def _groups(self, H: int):
         if H == 0:
             return self._view()
+        if not self.p1:
+            return self._lists(H)
         E, B = self.elements.shape
         N, dev, pat = self.pattern.n_points, self.elements.device, self.pattern
         quads = int(H == 1)

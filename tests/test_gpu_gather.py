@@ -31,7 +31,7 @@ class EElasticity(tg.ElementAssembler):
 def every_size(monkeypatch):
     """The element-once path at any size (its dispatch keeps small meshes on
     the one-launch patch kernels)."""
-    monkeypatch.setattr("tensormesh_gb300.assemble._GATHER_MIN_ELEMENTS", 0)
+    monkeypatch.setattr("tensormesh_gb300.assemble._GATHER_MIN_ELEMENTS", dict.fromkeys(tg.element.ELEMENT_TYPES, 0))
 
 
 FORMS = {"laplace": KappaLaplace, "elasticity": EElasticity}
@@ -169,6 +169,99 @@ def test_group_lists_cover_every_entry(etype, n, H):
                         if v & 0x8000:
                             break
                 assert got == holds[(r, c)]
+
+
+# -- quadrature kernels: P2 elements, mass matrices, loads ------------------------------
+class KappaMass(tg.ElementAssembler):
+    def forward(self, u, v, kappa):
+        return kappa * u * v
+
+
+FORMS["mass"] = KappaMass
+
+
+def curved(etype, n, seed):
+    """A P2 mesh with every node moved and renumbered."""
+    base = (tg.Mesh.gen_unit_square(n) if etype == "triangle6" else tg.Mesh.gen_unit_cube(n)).to_p2()
+    rng = np.random.default_rng(seed)
+    pts = base.points.numpy() + rng.uniform(-0.04, 0.04, size=tuple(base.points.shape)) / n
+    new = rng.permutation(pts.shape[0])
+    moved = np.empty_like(pts)
+    moved[new] = pts
+    return moved, new[base.cells[etype].numpy()]
+
+
+MESHES = [("triangle6", 1), ("triangle6", 5), ("tetra10", 1), ("tetra10", 3)]
+
+
+@pytest.mark.parametrize("etype,n", MESHES)
+@pytest.mark.parametrize("form", ["laplace", "mass", "elasticity"])
+@pytest.mark.parametrize("q", [1, 3, 4])
+@pytest.mark.parametrize("dtype", [torch.float64, torch.float32])
+def test_p2_forms_match_oracle(etype, n, form, q, dtype):
+    pts, el = curved(etype, n, n)
+    check(pts, el, etype, form, np.exp(np.random.default_rng(n).normal(size=el.shape[0])), dtype, q=q)
+
+
+@pytest.mark.parametrize("etype,n", [("triangle", 6), ("tetra", 4)])
+@pytest.mark.parametrize("q", [1, 2, 4])
+def test_p1_mass_matches_oracle(etype, n, q):
+    pts, el = ragged(etype, n, n)
+    check(pts, el, etype, "mass", np.exp(np.random.default_rng(n).normal(size=el.shape[0])), q=q)
+
+
+@pytest.mark.parametrize("etype,n", [("triangle", 6), ("tetra", 4)] + MESHES[1::2])
+@pytest.mark.parametrize("scale", [1e-9, 1e9])
+def test_units_and_far_coefficients_with_quadrature(etype, n, scale):
+    """Mass matrices (length^D) in extreme units, with elements whose
+    coefficient is zero or far outside the common exponent's window."""
+    pts, el = ragged(etype, n, 1) if n >= 4 and etype in ("triangle", "tetra") else curved(etype, n, 1)
+    g = np.exp(np.random.default_rng(2).normal(size=el.shape[0]))
+    for far in (0.0, 1e-40, 1e40):
+        check(pts * scale, el, etype, "mass", g * np.where(np.arange(el.shape[0]) % 3 == 1, far, 1.0))
+        if etype in ("triangle6", "tetra10"):
+            check(pts * scale, el, etype, "elasticity", g * np.where(np.arange(el.shape[0]) % 3 == 1, far, 1.0))
+
+
+def test_slivers_with_quadrature():
+    """Needle elements (conditioning 1e7) take the native pass of their CTA."""
+    ring, height = 30, 200.0
+    t = np.arange(ring) * 2 * np.pi / ring
+    pts = np.concatenate([[[0.0, 0.0, -height], [0.0, 0.0, height]], np.stack([np.cos(t), np.sin(t), 0.1 * np.sin(3 * t)], 1)])
+    el = np.array([[0, 2 + k, 2 + (k + 1) % ring, 1] for k in range(ring)], dtype=np.int64)
+    kappa = np.exp(np.random.default_rng(ring).normal(size=ring))
+    check(pts, el, "tetra", "mass", kappa)
+    p2 = tg.Mesh(points=torch.tensor(pts), cells={"tetra": torch.tensor(el)}).to_p2()
+    check(p2.points.numpy(), p2.cells["tetra10"].numpy(), "tetra10", "laplace", kappa)
+
+
+@pytest.mark.parametrize("etype,n", [("triangle", 6), ("tetra", 4)] + MESHES)
+@pytest.mark.parametrize("q", [1, 2, 4])
+@pytest.mark.parametrize("dtype", [torch.float64, torch.float32])
+def test_loads_match_oracle(etype, n, q, dtype):
+    pts, el = (ragged if etype in ("triangle", "tetra") else curved)(etype, n, 4)
+    mesh = tg.Mesh(points=torch.tensor(pts, device=DEV, dtype=dtype), cells={etype: torch.tensor(el, device=DEV)})
+    p64 = mesh.points.double().cpu().numpy()
+
+    class PointLoad(tg.NodeAssembler):
+        def forward(self, v, f):
+            return v * f
+
+    f = torch.tensor(np.random.default_rng(3).normal(size=(pts.shape[0], 3)), device=DEV, dtype=dtype)
+    cases = [
+        (tg.const_node_assembler(torch.tensor([2.0, -1.0], device=DEV, dtype=dtype)).from_mesh(mesh, quadrature_order=q)(mesh.points),
+         fem.assemble_load(p64, el, etype, q, "const", [2.0, -1.0])),
+        # a source that decays by 40 orders of magnitude over the mesh, and one with zeros
+        (tg.func_node_assembler(lambda x: torch.exp(-90.0 * x[..., 0])).from_mesh(mesh, quadrature_order=q)(mesh.points),
+         fem.assemble_load(p64, el, etype, q, "func", lambda x: np.exp(-90.0 * x[..., 0]))),
+        (tg.func_node_assembler(lambda x: torch.relu(x[..., 0] - 0.5)).from_mesh(mesh, quadrature_order=q)(mesh.points),
+         fem.assemble_load(p64, el, etype, q, "func", lambda x: np.maximum(x[..., 0] - 0.5, 0.0))),
+        (PointLoad.from_mesh(mesh, quadrature_order=q)(mesh.points, point_data={"f": f}),
+         fem.assemble_load(p64, el, etype, q, "point", f.double().cpu().numpy())),
+    ]
+    for got, ref in cases:
+        err = np.max(np.abs(got.double().cpu().numpy() - ref)) / np.max(np.abs(ref))
+        assert err <= (1e-12 if dtype == torch.float64 else 1e-5), err
 
 
 # -- backward ----------------------------------------------------------------------
