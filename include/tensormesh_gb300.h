@@ -570,6 +570,17 @@ int tm_morton_keys(int64_t n, int32_t dim, const double* coords, const double* l
  */
 int tm_selftest_barrier_timeout(int32_t n_blocks, int64_t spins, int32_t* out_status, void* work, void* stream);
 
+/*
+ * Self-test of the SELL solver's grid-wide sums: n_blocks CTAs of 512 threads
+ * add vals[n_blocks * 512] (and minus half of them) `rounds` times; CTA c
+ * writes its totals to out[2 c], out[2 c + 1].  With absent != 0 the last CTA
+ * never publishes and the others give up after `spins` polls: *out_status is
+ * TM_ERR_TIMEOUT.  work: 16-byte aligned, 8192 + 64 n_blocks bytes suffice.
+ * Synchronises the stream.
+ */
+int tm_selftest_grid_sum(int32_t n_blocks, int32_t absent, int32_t rounds, int64_t spins, const double* vals,
+                         double* out, int32_t* out_status, void* work, int64_t work_bytes, void* stream);
+
 /* 1/diag(A) with missing diagonals taken as 1 (torch_solve.py:24-59). */
 int tm_csr_diagonal_inverse(int32_t dtype, int64_t n, const int64_t* indptr, const int32_t* indices,
                             const void* values, void* out, void* stream);

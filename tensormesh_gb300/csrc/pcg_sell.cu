@@ -96,8 +96,11 @@ template <> struct SellT<F2> {
 // for matrices whose every |column - row| fits; FEM orderings keep the
 // coupling bandwidth small), the latter saving 2 of the 12 bytes an entry
 // streams per iteration.
-TM_D int col_of(const int32_t* scol, int64_t k, int64_t) { return __ldg(scol + k); }
-TM_D int col_of(const int16_t* scol, int64_t k, int64_t row) { return (int)row + (int)__ldg(scol + k); }
+// kGen: the array may lie in shared memory.
+template <bool kGen> TM_D int col_of(const int32_t* scol, int64_t k, int64_t) { return kGen ? scol[k] : __ldg(scol + k); }
+template <bool kGen> TM_D int col_of(const int16_t* scol, int64_t k, int64_t row) {
+  return (int)row + (int)(kGen ? scol[k] : __ldg(scol + k));
+}
 
 // Largest |column - row| of the matrix (atomic max into *span).
 __global__ void sell_span_kernel(int64_t n, const int64_t* __restrict__ indptr, const int32_t* __restrict__ idx,
@@ -233,9 +236,8 @@ __global__ void sell_fill_kernel(int64_t n, const int64_t* __restrict__ indptr, 
 // acc[u] = sum_j sval[.] * g(scol[.]) over the rows of slices sl + u * kSellWarps
 // (u < kSellRows) of [sl, s_hi), for the calling lane's row.  g gathers the
 // operand's column value (one vector, or a combination of two).
-template <class S, class CT, class G>
-TM_D void sell_rows(const int64_t* __restrict__ sptr, const CT* __restrict__ scol, const S* __restrict__ sval,
-                    const G& g, int64_t sl, int64_t s_hi, typename SellT<S>::A (&acc)[kSellRows]) {
+template <class S, class CT, bool kGen = false, class G>
+TM_D void sell_rows(const int64_t* __restrict__ sptr, const CT* scol, const S* sval, const G& g, int64_t sl, int64_t s_hi, typename SellT<S>::A (&acc)[kSellRows]) {
   using Tr = SellT<S>;
   const int lane = threadIdx.x & 31;
   int64_t off[kSellRows];
@@ -259,7 +261,7 @@ TM_D void sell_rows(const int64_t* __restrict__ sptr, const CT* __restrict__ sco
       for (int j = 0; j < kSellIlp; ++j) {
         const bool ok = j0 + j < len[u];
         const int64_t k = off[u] + (int64_t)(j0 + j) * 32;
-        c[u][j] = ok ? col_of(scol, k, (sl + (int64_t)u * kSellWarps) * 32 + lane) : 0;
+        c[u][j] = ok ? col_of<kGen>(scol, k, (sl + (int64_t)u * kSellWarps) * 32 + lane) : 0;
         v[u][j] = ok ? sval[k] : S{};
       }
 #pragma unroll
@@ -278,43 +280,109 @@ TM_D void sell_rows(const int64_t* __restrict__ sptr, const CT* __restrict__ sco
 //   sweep 2: alpha = rz / (p, q); x += alpha M pt; r -= alpha q; partial
 //            rz = sum M r^2 and rr = sum r^2                        [barrier]
 // The iterates are those of tm_pcg_jacobi's recurrence (z = M r, p = z +
-// beta p), so its rounding behaviour is that of standard PCG.
-template <class S, class CT>
-__global__ void __launch_bounds__(kSellThreads, 2)
+// beta p), so its rounding behaviour is that of standard PCG.  The barriers are
+// the grid sums (grid_sum); the scalars' FP64 divisions and the square root run
+// in one thread of a CTA.
+//
+// kMode kGrid streams the matrix.  kResident: a CTA's share of the matrix, x, q, M and its own rows of r and pt stay
+// in shared memory for the whole solve, and an iteration reads only the
+// gathered r and pt from L2.  kCluster: the same in one cluster, whose barriers
+// take a microsecond instead of three.  Chosen by launch_pcg_sell; a CTA whose
+// share exceeds `cap` entries (uneven rows) reads the matrix from global memory.
+enum { kGrid = 0, kResident = 1, kCluster = 2 };
+template <class S, class CT, int kMode>
+__global__ void __launch_bounds__(kSellThreads, kMode ? 1 : 2)
 pcg_sell_hs_kernel(int64_t n, const int64_t* __restrict__ sptr, const CT* __restrict__ scol,
                    const S* __restrict__ sval, const S* __restrict__ dinv, const typename SellT<S>::V* __restrict__ bv,
                    typename SellT<S>::V* __restrict__ xv, S* x, S* r, S* q, S* pt0, S* pt1, const S* y,
-                   double* partials, PcgState* st, double rtol, double atol, int maxiter) {
+                   ulonglong2* slots, PcgState* st, double rtol, double atol, int maxiter, int cap) {
   using Tr = SellT<S>;
   using A = typename Tr::A;
-  __shared__ double s_red[32];
+  constexpr bool kRes = kMode != kGrid;
+  static_assert(kSellThreads == kSlotThreads, "grid_sum's shared array");
+  __shared__ double s_slot[2 * 16 * 2];
+  __shared__ int s_red[8 * (kSlotThreads / 32)];
+  __shared__ S s_scalar;   // alpha, then beta
+  __shared__ int s_stop;   // -1: go on, else the status to end with
+  extern __shared__ __align__(16) unsigned char smem_raw[];
   const unsigned nb = gridDim.x;
-  unsigned my_gen = 0;  // the host zeroes st->gen before the launch
+  const GridSlots gs{slots, nb};
+  unsigned gen = 0;        // the host zeroes the slots before the launch
   if (*((volatile int*)&st->status) != TM_OK) return;  // slice plan rejected by the fill kernel
   const int64_t n_slices = (n + 31) >> 5;
   const int64_t per = (n_slices + nb - 1) / nb;
   const int64_t s_lo = min(n_slices, (int64_t)blockIdx.x * per), s_hi = min(n_slices, s_lo + per);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  double* pA = partials;
-  double* pB = partials + nb;
-  double* pC = partials + 2 * (int64_t)nb;
   auto row_of = [&](int64_t sl, int u) { return (sl + (int64_t)u * kSellWarps) * 32 + lane; };
   auto valid = [&](int64_t sl, int u) { return sl + (int64_t)u * kSellWarps < s_hi && row_of(sl, u) < n; };
-  auto publish2 = [&](double* da, A va, double* db, A vb) {
-    double a = Tr::to_double(va), b = Tr::to_double(vb);
-    block_sum2(a, b, s_red);
-    if (threadIdx.x == 0) {
-      da[blockIdx.x] = a;
-      db[blockIdx.x] = b;
+
+  // own-row vectors: shared memory indexed by row - 32 s_lo, or the global arrays
+  const int64_t row0 = s_lo * 32;
+  S *ox = x, *orr = r, *oq = q, *op = nullptr;
+  const S* od = dinv;
+  const S* mval = sval;
+  const CT* mcol = scol;
+  if constexpr (kRes) {
+    const int64_t rows = per * 32;
+    S* s = reinterpret_cast<S*>(smem_raw);
+    ox = s - row0;
+    orr = s + rows - row0;
+    oq = s + 2 * rows - row0;
+    op = s + 3 * rows - row0;
+    S* d = s + 4 * rows - row0;
+    for (int64_t i = row0 + threadIdx.x; i < min(n, s_hi * 32); i += kSellThreads) d[i] = dinv[i];
+    od = d;
+    const int64_t k0 = s_lo < s_hi ? sptr[s_lo] : 0, k1 = s_lo < s_hi ? sptr[s_hi] : 0;
+    if (k1 - k0 <= cap) {
+      S* mv = s + 5 * rows;
+      CT* mc = reinterpret_cast<CT*>(mv + cap);
+      for (int64_t k = k0 + threadIdx.x; k < k1; k += kSellThreads) {
+        mv[k - k0] = sval[k];
+        mc[k - k0] = scol[k];
+      }
+      mval = mv - k0;
+      mcol = mc - k0;
     }
+    __syncthreads();
+  }
+  auto product = [&](const auto& g, int64_t sl, A (&acc)[kSellRows]) {
+    sell_rows<S, CT, kRes>(sptr, mcol, mval, g, sl, s_hi, acc);
+  };
+  auto barrier1 = [&](double& a) -> bool {
+    double b = 0.0;
+    if constexpr (kMode == kCluster) {
+      cluster_sum<false>(++gen, nb, a, b, s_red, s_slot);
+      return true;
+    } else {
+      return grid_sum<false>(st, gs, ++gen, a, b, s_red);
+    }
+  };
+  auto barrier2 = [&](double& a, double& b) -> bool {
+    if constexpr (kMode == kCluster) {
+      cluster_sum<true>(++gen, nb, a, b, s_red, s_slot);
+      return true;
+    } else {
+      return grid_sum<true>(st, gs, ++gen, a, b, s_red);
+    }
+  };
+  // Ends a barrier: lane 0 of warp 0 runs f on the sums (it sets s_scalar and s_stop).
+  auto finish = [&](bool ok, const auto& f) -> bool {
+    if (threadIdx.x == 0) {
+      s_stop = -1;
+      if (!ok) s_stop = TM_ERR_TIMEOUT;
+      else f();
+    }
+    __syncthreads();
+    return s_stop != TM_ERR_TIMEOUT;
   };
 
   // ---- r = b - (A M) y, x = x0, pt_old = 0; rz, rr, bb
+  double rz = 0.0, rr = 0.0, tol = 0.0, tol2 = 0.0;   // kept by thread 0 of every CTA
   {
     A rz_l = Tr::zero(), rr_l = Tr::zero(), bb_l = Tr::zero();
     for (int64_t sl = s_lo + warp; sl < s_hi; sl += (int64_t)kSellRows * kSellWarps) {
       A acc[kSellRows];
-      sell_rows<S, CT>(sptr, scol, sval, [&](int c) { return Tr::ld(y, c); }, sl, s_hi, acc);
+      product([&](int c) { return Tr::ld(y, c); }, sl, acc);
 #pragma unroll
       for (int u = 0; u < kSellRows; ++u) {
         if (!valid(sl, u)) continue;
@@ -322,90 +390,106 @@ pcg_sell_hs_kernel(int64_t n, const int64_t* __restrict__ sptr, const CT* __rest
         const A b = Tr::in(bv[row]);
         const A rv = b - acc[u];
         Tr::st(r, row, rv);
-        Tr::st(x, row, Tr::in(xv[row]));
+        if constexpr (kRes) {
+          Tr::st(orr, row, rv);
+          Tr::st(op, row, Tr::zero());
+        }
+        Tr::st(ox, row, Tr::in(xv[row]));
         Tr::st(pt0, row, Tr::zero());
-        rz_l += Tr::ld(dinv, row) * rv * rv;
+        rz_l += Tr::ld(od, row) * rv * rv;
         rr_l += rv * rv;
         bb_l += b * b;
       }
     }
-    publish2(pA, rz_l, pB, rr_l);
-    const double t = block_sum(Tr::to_double(bb_l), s_red);
-    if (threadIdx.x == 0) pC[blockIdx.x] = t;
+    double a = Tr::to_double(bb_l), b;
+    bool ok = barrier1(a);
+    if (!finish(ok, [&] {
+          tol = fmax(rtol * sqrt(a), atol);
+          tol2 = tol * tol * (1.0 + 1e-12);
+          if (blockIdx.x == 0) st->bnorm = sqrt(a);
+        }))
+      return;
+    a = Tr::to_double(rz_l);
+    b = Tr::to_double(rr_l);
+    ok = barrier2(a, b);
+    if (!finish(ok, [&] {
+          rz = a;
+          rr = b;
+          if (sqrt(rr) <= tol) s_stop = TM_OK;
+          else if (maxiter == 0) s_stop = TM_ERR_MAXITER;
+        }))
+      return;
   }
-  if (!grid_sync(st, nb, my_gen)) return;
-  double rz, rr;
-  sum_partials2(pA, pB, nb, s_red, rz, rr);
-  const double bnorm = sqrt(sum_partials(pC, nb, s_red));
-  const double tol = fmax(rtol * bnorm, atol);
-  if (blockIdx.x == 0 && threadIdx.x == 0) st->bnorm = bnorm;
-  if (!grid_sync(st, nb, my_gen)) return;  // the partial buffers are reused below
 
   A beta = Tr::zero();
   S* pold = pt0;
   S* pnew = pt1;
   int it = 0;
-  int status = TM_ERR_MAXITER;
-  for (;; ++it) {
-    if (sqrt(rr) <= tol) {
-      status = TM_OK;
-      break;
-    }
-    if (it == maxiter) break;
+  int status = s_stop;
+  while (status < 0) {
     // sweep 1
     A pq_l = Tr::zero();
     const S* cpold = pold;
     for (int64_t sl = s_lo + warp; sl < s_hi; sl += (int64_t)kSellRows * kSellWarps) {
       A acc[kSellRows];
-      sell_rows<S, CT>(sptr, scol, sval, [&](int c) { return Tr::ld(r, c) + beta * Tr::ld(cpold, c); }, sl,
-                       s_hi, acc);
+      product([&](int c) { return Tr::ld(r, c) + beta * Tr::ld(cpold, c); }, sl, acc);
 #pragma unroll
       for (int u = 0; u < kSellRows; ++u) {
         if (!valid(sl, u)) continue;
         const int64_t row = row_of(sl, u);
-        const A pv = Tr::ld(r, row) + beta * Tr::ld(cpold, row);
+        const A pv = Tr::ld(orr, row) + beta * Tr::ld(kRes ? op : cpold, row);
         Tr::st(pnew, row, pv);
-        Tr::st(q, row, acc[u]);
-        pq_l += Tr::ld(dinv, row) * pv * acc[u];
+        if constexpr (kRes) Tr::st(op, row, pv);
+        Tr::st(oq, row, acc[u]);
+        pq_l += Tr::ld(od, row) * pv * acc[u];
       }
     }
-    {
-      const double t = block_sum(Tr::to_double(pq_l), s_red);
-      if (threadIdx.x == 0) pA[blockIdx.x] = t;
-    }
-    if (!grid_sync(st, nb, my_gen)) return;
-    const double pq = sum_partials(pA, nb, s_red);
-    if (!(pq > 0.0)) {
-      status = TM_ERR_BREAKDOWN;
-      break;
-    }
-    const A alpha = Tr::from_double(rz / pq);
+    double a = Tr::to_double(pq_l), b;
+    bool ok = barrier1(a);
+    if (!finish(ok, [&] {
+          if (!(a > 0.0)) s_stop = TM_ERR_BREAKDOWN;
+          else s_scalar = Tr::pack(Tr::from_double(rz / a));
+        }))
+      return;
+    status = s_stop;
+    if (status >= 0) break;
+    const A alpha = Tr::mk(s_scalar);
     // sweep 2
     A rz_l = Tr::zero(), rr_l = Tr::zero();
     for (int64_t sl = s_lo + warp; sl < s_hi; sl += kSellWarps) {
       const int64_t row = sl * 32 + lane;
       if (row >= n) continue;
-      const A di = Tr::ld(dinv, row), pv = Tr::ld(pnew, row), qv = Tr::ld(q, row);
-      const A xo = Tr::ld(x, row), ro = Tr::ld(r, row);
+      const A di = Tr::ld(od, row), pv = Tr::ld(kRes ? op : pnew, row), qv = Tr::ld(oq, row);
+      const A xo = Tr::ld(ox, row), ro = Tr::ld(orr, row);
       const A rn = ro - alpha * qv;
-      Tr::st(x, row, xo + alpha * (di * pv));
+      Tr::st(ox, row, xo + alpha * (di * pv));
       Tr::st(r, row, rn);
+      if constexpr (kRes) Tr::st(orr, row, rn);
       rz_l += di * rn * rn;
       rr_l += rn * rn;
     }
-    publish2(pB, rz_l, pC, rr_l);
-    if (!grid_sync(st, nb, my_gen)) return;
-    double rzn;
-    sum_partials2(pB, pC, nb, s_red, rzn, rr);
-    beta = Tr::from_double(rzn / rz);
-    rz = rzn;
+    a = Tr::to_double(rz_l);
+    b = Tr::to_double(rr_l);
+    ok = barrier2(a, b);
+    ++it;
+    if (!finish(ok, [&] {
+          s_scalar = Tr::pack(Tr::from_double(a / rz));
+          rz = a;
+          rr = b;
+          // (the slow square root only near the end)
+          if (rr <= tol2 && sqrt(rr) <= tol) s_stop = TM_OK;
+          else if (it == maxiter) s_stop = TM_ERR_MAXITER;
+        }))
+      return;
+    status = s_stop;
+    beta = Tr::mk(s_scalar);
     S* t = pold;
     pold = pnew;
     pnew = t;
   }
   for (int64_t sl = s_lo + warp; sl < s_hi; sl += kSellWarps) {
     const int64_t row = sl * 32 + lane;
-    if (row < n) xv[row] = Tr::out(Tr::ld(x, row));
+    if (row < n) xv[row] = Tr::out(Tr::ld(ox, row));
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     st->iters = it;
@@ -627,11 +711,10 @@ inline int64_t align256(int64_t b) { return (b + 255) & ~int64_t(255); }
 
 constexpr int kSellMaxBlocks = 4096;
 
-// Cooperative grid: two CTAs per SM when each gets at least kSlicesPerCta
-// slices, else one.  Small systems are bound by the two grid barriers and
-// the partial-sum reads per iteration, which cost more with more CTAs
-// (us per iteration, 304 / 152 CTAs: 2D 65k rows 23.2 / 16.3, 3D 64^3 31.2 /
-// 27.3, 96^3 64.4 / 80.1, 128^3 127 / 172).
+// Streaming grid: two CTAs per SM when each gets at least kSlicesPerCta
+// slices, else one (fewer CTAs make the grid sums cheaper; measured with the
+// earlier barriers, us per iteration at 304 / 152 CTAs: 96^3 64.4 / 80.1,
+// 128^3 127 / 172, 64^3 31.2 / 27.3).
 constexpr int kSlicesPerCta = 48;
 
 template <class K>
@@ -642,7 +725,75 @@ int sell_blocks(K kern, int64_t n_slices) {
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kSellThreads, 0);
   int nb = sms * min(per_sm, 2);
   if (n_slices < (int64_t)kSlicesPerCta * nb) nb = min(nb, sms);
-  return min(kSellMaxBlocks, nb);
+  return min(kSellMaxBlocks, nb);   // at most two CTAs per SM: grid_sum's words fit the partial sums' array
+}
+
+// How a standard solve is launched.
+struct SellLaunch {
+  int mode = kGrid, nb = 0, cap = 0;
+  size_t bytes = 0;
+};
+
+// Shared memory of a resident CTA when nb of them share the system: five
+// own-row vectors and the matrix entries, a quarter more than the average
+// share where that fits (uneven rows).  0 when the average share does not fit.
+template <class S, class CT>
+size_t resident_bytes(int64_t n_slices, int64_t n_pad, int nb, int optin, int& cap) {
+  const int64_t rows = (n_slices + nb - 1) / nb * 32, vec = 5 * rows * (int64_t)sizeof(S);
+  const int64_t avail = (int64_t)optin - 4 * 1024 - vec;   // the kernel's static arrays aside
+  const int64_t entry = (int64_t)sizeof(S) + (int64_t)sizeof(CT), share = (n_pad + nb - 1) / nb;
+  if (avail <= 0 || share * entry > avail) return 0;
+  cap = (int)(min((share + share / 4 + 1024) * entry, avail) / entry) & ~15;
+  return (size_t)(vec + cap * entry);
+}
+
+// One cluster of 16 CTAs (8 where 16 do not fit a GPC) when the system fits
+// its shared memory (2D: to about 29,000 rows), a CTA per SM when it fits that
+// (2D to 270,000 rows, 3D to 130,000), streaming otherwise.  us per iteration,
+// a call's other work included: 64^2 6.5 in a cluster, 10.0 on the grid, 15.0
+// before (atomic barriers, FP64 shuffle trees, divisions in every thread);
+// 256^2 11.0 resident, 16.2 before; 96^3 57 streaming, 65 before.
+template <class S, class CT>
+int sell_launch(int64_t n_slices, int64_t n_pad, SellLaunch& how) {
+  int dev = 0, sms = 0, optin = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return TM_ERR_CUDA;
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  for (int nb = 16; nb >= 8; nb /= 2) {
+    const size_t bytes = resident_bytes<S, CT>(n_slices, n_pad, nb, optin, how.cap);
+    auto kern = pcg_sell_hs_kernel<S, CT, kCluster>;
+    if (!bytes || cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess ||
+        cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
+      continue;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(nb);
+    cfg.blockDim = dim3(kSellThreads);
+    cfg.dynamicSmemBytes = bytes;
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = (unsigned)nb;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    int clusters = 0;
+    if (cudaOccupancyMaxActiveClusters(&clusters, kern, &cfg) != cudaSuccess || clusters < 1) continue;
+    how.mode = kCluster;
+    how.nb = nb;
+    how.bytes = bytes;
+    return TM_OK;
+  }
+  cudaGetLastError();   // a refused attribute or query above only rules the cluster out
+  const int nb = (int)min((int64_t)sms, n_slices);
+  const size_t bytes = nb > 0 ? resident_bytes<S, CT>(n_slices, n_pad, nb, optin, how.cap) : 0;
+  if (bytes && cudaFuncSetAttribute(pcg_sell_hs_kernel<S, CT, kResident>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)bytes) == cudaSuccess) {
+    how.mode = kResident;
+    how.nb = nb;
+    how.bytes = bytes;
+    return TM_OK;
+  }
+  how.nb = sell_blocks(pcg_sell_hs_kernel<S, CT, kGrid>, n_slices);
+  return TM_OK;
 }
 
 template <class S, class CT>
@@ -650,8 +801,14 @@ int launch_pcg_sell(int64_t n, const int64_t* indptr, const int32_t* indices, co
                     const int64_t* sptr, int64_t n_pad, const typename SellT<S>::V* b, typename SellT<S>::V* x,
                     double rtol, double atol, int maxiter, bool pipe, char* w, cudaStream_t s) {
   const int64_t n_slices_all = (n + 31) >> 5;
-  const int nb = pipe ? sell_blocks(pcg_sell_kernel<S, CT>, n_slices_all)
-                      : sell_blocks(pcg_sell_hs_kernel<S, CT>, n_slices_all);
+  SellLaunch how;
+  if (pipe) {
+    how.nb = sell_blocks(pcg_sell_kernel<S, CT>, n_slices_all);
+  } else {
+    const int rc = sell_launch<S, CT>(n_slices_all, n_pad, how);
+    if (rc != TM_OK) return rc;
+  }
+  const int nb = how.nb;
   if (nb <= 0) return TM_ERR_CUDA;
   PcgState* st = reinterpret_cast<PcgState*>(w);
   char* q = w + 256;
@@ -667,7 +824,10 @@ int launch_pcg_sell(int64_t n, const int64_t* indptr, const int32_t* indices, co
   CT* scol = reinterpret_cast<CT*>(q);
   S* dinv = vec[0];
   S* y = vec[5];  // M^-1 x0, read by the first sweep only
-  if (cudaMemsetAsync(st, 0, sizeof(PcgState), s) != cudaSuccess) return TM_ERR_CUDA;
+  // the record, and the words of grid_sum (the first of the partial sums' array)
+  ulonglong2* slots = reinterpret_cast<ulonglong2*>(partials);
+  const size_t clear = pipe ? sizeof(PcgState) : 256 + grid_slot_bytes(nb);
+  if (cudaMemsetAsync(st, 0, clear, s) != cudaSuccess) return TM_ERR_CUDA;
   sell_dinv_kernel<S><<<(unsigned)((n + 255) / 256), 256, 0, s>>>(n, indptr, indices, values, dinv);
   const int64_t n_slices = (n + 31) >> 5;
   sell_fill_kernel<S, CT><<<(unsigned)((n_slices * 32 + 255) / 256), 256, 0, s>>>(n, indptr, indices, values, sptr,
@@ -688,9 +848,25 @@ int launch_pcg_sell(int64_t n, const int64_t* indptr, const int32_t* indices, co
     const S* cy = y;
     void* args[] = {(void*)&n, (void*)&sptr, (void*)&cscol, (void*)&csval, (void*)&cdinv, (void*)&b, (void*)&x,
                     (void*)&xs, (void*)&r, (void*)&qv, (void*)&pt0, (void*)&pt1, (void*)&cy,
-                    (void*)&partials, (void*)&st, (void*)&rtol, (void*)&atol, (void*)&maxiter};
-    e = cudaLaunchCooperativeKernel((const void*)pcg_sell_hs_kernel<S, CT>, dim3(nb), dim3(kSellThreads), args, 0,
-                                    s);
+                    (void*)&slots, (void*)&st, (void*)&rtol, (void*)&atol, (void*)&maxiter, (void*)&how.cap};
+    if (how.mode == kCluster) {
+      cudaLaunchConfig_t cfg{};
+      cfg.gridDim = dim3(nb);
+      cfg.blockDim = dim3(kSellThreads);
+      cfg.dynamicSmemBytes = how.bytes;
+      cfg.stream = s;
+      cudaLaunchAttribute attr{};
+      attr.id = cudaLaunchAttributeClusterDimension;
+      attr.val.clusterDim.x = (unsigned)nb;
+      attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+      cfg.attrs = &attr;
+      cfg.numAttrs = 1;
+      e = cudaLaunchKernelExC(&cfg, (const void*)pcg_sell_hs_kernel<S, CT, kCluster>, args);
+    } else {
+      const void* kern = how.mode == kResident ? (const void*)pcg_sell_hs_kernel<S, CT, kResident>
+                                               : (const void*)pcg_sell_hs_kernel<S, CT, kGrid>;
+      e = cudaLaunchCooperativeKernel(kern, dim3(nb), dim3(kSellThreads), args, how.bytes, s);
+    }
   }
   return e == cudaSuccess ? TM_OK : TM_ERR_CUDA;
 }
@@ -705,7 +881,57 @@ int launch_pcg_sell_any(int64_t n, const int64_t* indptr, const int32_t* indices
   return launch_pcg_sell<S, int32_t>(n, indptr, indices, values, sptr, n_pad, b, x, rtol, atol, maxiter, pipe, w, s);
 }
 
+// grid_sum on given values: thread t of CTA c adds vals[c * kSlotThreads + t] and
+// minus half of it; with `absent` the last CTA leaves without publishing.
+__global__ void __launch_bounds__(kSlotThreads)
+grid_sum_selftest_kernel(const double* __restrict__ vals, ulonglong2* slots, PcgState* st, int absent, int rounds,
+                         long long spins, double* out) {
+  __shared__ int s_red[8 * (kSlotThreads / 32)];
+  __shared__ int s_ok;
+  if (absent && blockIdx.x == gridDim.x - 1) return;
+  const GridSlots gs{slots, gridDim.x};
+  for (int k = 1; k <= rounds; ++k) {
+    double a = vals[(size_t)blockIdx.x * kSlotThreads + threadIdx.x], b = -0.5 * a;
+    const bool ok = grid_sum<true>(st, gs, (unsigned)k, a, b, s_red, spins);
+    if (threadIdx.x == 0) {
+      s_ok = ok;
+      out[2 * blockIdx.x] = a;
+      out[2 * blockIdx.x + 1] = b;
+    }
+    __syncthreads();
+    if (!s_ok) return;
+  }
+}
+
 }  // namespace tmg
+
+extern "C" int tm_selftest_grid_sum(int32_t n_blocks, int32_t absent, int32_t rounds, int64_t spins,
+                                    const double* vals, double* out, int32_t* out_status, void* work,
+                                    int64_t work_bytes, void* stream) {
+  if (n_blocks < 2 || rounds < 1 || spins < 1 || spins > tmg::kSlotSpinLimit || !vals || !out || !out_status || !work)
+    return TM_ERR_INVALID;
+  int dev = 0, sms = 0, per_sm = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return TM_ERR_CUDA;
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, tmg::grid_sum_selftest_kernel, tmg::kSlotThreads, 0);
+  if (n_blocks > sms * per_sm) return TM_ERR_INVALID;
+  const size_t need = 256 + tmg::grid_slot_bytes((unsigned)n_blocks);
+  if (work_bytes < (int64_t)need) return TM_ERR_INDEX;
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  tmg::PcgState* st = static_cast<tmg::PcgState*>(work);
+  if (cudaMemsetAsync(work, 0, need, s) != cudaSuccess) return TM_ERR_CUDA;
+  ulonglong2* slots = reinterpret_cast<ulonglong2*>(static_cast<char*>(work) + 256);
+  long long sp = spins;
+  void* args[] = {(void*)&vals, (void*)&slots, (void*)&st, (void*)&absent, (void*)&rounds, (void*)&sp, (void*)&out};
+  if (cudaLaunchCooperativeKernel((const void*)tmg::grid_sum_selftest_kernel, dim3(n_blocks), dim3(tmg::kSlotThreads),
+                                  args, 0, s) != cudaSuccess)
+    return TM_ERR_CUDA;
+  tmg::PcgState h;
+  if (cudaMemcpyAsync(&h, st, sizeof(h), cudaMemcpyDeviceToHost, s) != cudaSuccess) return TM_ERR_CUDA;
+  if (cudaStreamSynchronize(s) != cudaSuccess) return TM_ERR_CUDA;
+  *out_status = h.status;
+  return TM_OK;
+}
 
 extern "C" int64_t tm_sell_plan(int64_t n, const int64_t* indptr, const int32_t* indices, int64_t* slice_ptr,
                                 int32_t* out_narrow, void* stream) {

@@ -1,0 +1,130 @@
+"""The SELL solver's launch modes (one cluster, a resident grid, streaming) and
+its grid-wide sums: fixed-point sums against exact ones, a wait that runs out,
+and systems whose rows are too uneven for a CTA's shared memory."""
+import ctypes
+import math
+
+import numpy as np
+import pytest
+import torch
+
+import tensormesh_gb300 as tg
+from tensormesh_gb300 import _lib, solve as S
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def grid_sum(vals, blocks, absent=0, rounds=3, spins=1 << 20):
+    out = torch.zeros(2 * blocks, dtype=torch.float64, device=DEV)
+    work = torch.empty(8192 + 64 * blocks, dtype=torch.uint8, device=DEV)
+    status = ctypes.c_int32(-1)
+    st = _lib.call_status("tm_selftest_grid_sum", blocks, absent, rounds, spins, vals.data_ptr(), out.data_ptr(),
+                          ctypes.byref(status), work.data_ptr(), work.numel(),
+                          torch.cuda.current_stream().cuda_stream)
+    assert st == _lib.TM_OK
+    return out.view(blocks, 2).cpu(), status.value
+
+
+@pytest.mark.parametrize("blocks", [2, 5, 32, 33, 152])
+@pytest.mark.parametrize("kind", ["normal", "squares", "wide", "cancel", "zeros", "powers"])
+def test_grid_sums_against_exact(blocks, kind):
+    """Every CTA holds the same bits, within three roundings of 2^-53 (a CTA's,
+    the grid's and the truncations) of the exact sum, relative to the largest
+    partial result."""
+    rng = np.random.default_rng(blocks)
+    n = blocks * 512
+    v = rng.normal(size=n)
+    if kind == "squares":
+        v = v * v
+    elif kind == "wide":
+        v = v * np.exp(30 * rng.normal(size=n))
+    elif kind == "cancel":
+        v[1::2] = -v[::2] * (1 + 1e-9)
+    elif kind == "zeros":
+        v[rng.random(n) < 0.9] = 0.0
+        v[:512] = 0.0
+    elif kind == "powers":
+        v = np.ldexp(1.0, rng.integers(-40, 40, size=n)) * rng.choice([-1, 1], size=n)
+    out, status = grid_sum(torch.tensor(v, device=DEV), blocks)
+    assert status == 0
+    assert torch.equal(out, out[:1].expand(blocks, 2))
+    parts = [math.fsum(c) for c in v.reshape(blocks, 512)]
+    scale = max(max(abs(p) for p in parts), abs(math.fsum(v)), np.abs(v).max())
+    assert abs(float(out[0, 0]) - math.fsum(v)) <= (blocks + 2) * 2.0 ** -53 * scale
+    assert abs(float(out[0, 1]) + 0.5 * math.fsum(v)) <= (blocks + 2) * 2.0 ** -53 * scale
+
+
+def test_grid_sum_of_nan_is_nan():
+    v = torch.ones(4 * 512, dtype=torch.float64, device=DEV)
+    v[700] = float("nan")
+    out, _ = grid_sum(v, 4)
+    assert bool(torch.isnan(out).all())
+
+
+def test_grid_sum_times_out_and_the_context_survives():
+    v = torch.ones(8 * 512, dtype=torch.float64, device=DEV)
+    _, status = grid_sum(v, 8, absent=1, spins=1 << 14)
+    assert status == _lib.TM_ERR_TIMEOUT
+    out, status = grid_sum(v, 8)
+    assert status == 0 and float(out[0, 0]) == 4096.0
+
+
+def poisson(dim, n, dtype):
+    mesh = (tg.Mesh.gen_unit_square if dim == 2 else tg.Mesh.gen_unit_cube)(n, device=DEV, dtype=dtype)
+    K = tg.LaplaceElementAssembler.from_mesh(mesh, quadrature_order=1)(mesh.points)
+    b = tg.const_node_assembler(1.0).from_mesh(mesh, quadrature_order=1)(mesh.points)
+    return tg.Condenser(mesh.boundary_mask)(K, b)
+
+
+# 2 to 16 rows; one cluster; both sides of its shared memory; the resident grid; streaming
+@pytest.mark.parametrize("dim,n", [(2, 2), (2, 3), (2, 64), (2, 150), (2, 190), (3, 40), (2, 600), (3, 80)])
+@pytest.mark.parametrize("dtype", [torch.float64, torch.float32])
+@pytest.mark.filterwarnings("ignore:PCG did not converge")   # float32: the residual's floor, see below
+def test_every_mode_solves(dim, n, dtype):
+    K, f = poisson(dim, n, dtype)
+    rtol = 1e-9 if dtype == torch.float64 else 1e-4
+    u = K.solve(f, rtol=rtol)
+    info = K.last_solve_info
+    # the rounding of K x in the value type floors the residual that can be reached
+    eps = torch.finfo(dtype).eps
+    floor = eps * float(((K.with_values(K.values.abs()) @ u.abs()).norm() / f.norm()))
+    assert info.status == 0 and info.residual <= rtol + 4 * floor
+    assert torch.equal(K.solve(f, rtol=rtol), u)          # bitwise repeatable
+    x = torch.zeros_like(f)
+    S.LAYOUT = "csr"
+    try:
+        ref = S.pcg_jacobi_raw(K.indptr, K.indices, K.values, f, x, rtol, 0.0, 100000)
+    finally:
+        S.LAYOUT = "sell"
+    if info.restarts == ref.restarts == 0:   # corrections at the floor are not comparable
+        assert abs(ref.iterations - info.iterations) <= max(2, ref.iterations // 50)
+    assert float((u - x).norm() / x.norm()) <= (1e-6 if dtype == torch.float64 else 5e-2)
+
+
+@pytest.mark.parametrize("n", [3000, 60000])
+def test_uneven_rows_fall_back_to_global_memory(n):
+    """The first 320 rows hold 200 entries each, the others three: the share of
+    the first CTA exceeds its shared memory's entries."""
+    rng = np.random.default_rng(n)
+    import scipy.sparse as sp
+    rows = np.repeat(np.arange(320), 100)
+    cols = rng.integers(320, n, size=rows.shape[0])
+    A = sp.coo_matrix((rng.uniform(-1, 1, size=rows.shape[0]), (rows, cols)), shape=(n, n))
+    A = A + A.T + sp.diags([np.full(n - 1, -1.0), np.full(n - 1, -1.0)], [1, -1])
+    A = (A + sp.diags(np.asarray(abs(A).sum(1)).ravel() + 0.1)).tocsr()
+    A.sort_indices()
+    b = rng.normal(size=n)
+    K = tg.SparseMatrix(torch.tensor(A.data, device=DEV), shape=(n, n),
+                        indptr=torch.tensor(A.indptr.astype(np.int64), device=DEV),
+                        indices=torch.tensor(A.indices.astype(np.int32), device=DEV))
+    x = K.solve(torch.tensor(b, device=DEV), rtol=1e-11)
+    assert np.linalg.norm(A @ x.cpu().numpy() - b) <= 1e-10 * np.linalg.norm(b)
+
+
+def test_iteration_cap_zero_and_one():
+    K, f = poisson(2, 20, torch.float64)
+    for cap in (0, 1):
+        with pytest.warns(UserWarning, match="did not converge"):
+            K.solve(f, rtol=1e-10, maxiter=cap)
+        assert K.last_solve_info.iterations == cap and K.last_solve_info.status == _lib.TM_ERR_MAXITER
