@@ -9,15 +9,17 @@
 //      the C CTAs), writing CSR values / b directly;
 //   2. runs Jacobi-PCG on the instance's interior dofs (Dirichlet dofs are
 //      masked: x = r = z = p = 0 there, which is CG on K_ii exactly), with
-//      the instance's rows split over the C CTAs.  Dot products reduce per
-//      CTA and are combined through distributed shared memory in a fixed
-//      order after a hardware cluster barrier -- deterministic, and no
-//      spin-wait anywhere (cluster barriers are co-scheduled by construction);
+//      the instance's rows split over the C CTAs.  Dot products are formed in
+//      double-float, added per CTA in fixed point and combined through
+//      distributed shared memory after a hardware cluster barrier
+//      (cluster_sum) -- deterministic, and no spin-wait anywhere (cluster
+//      barriers are co-scheduled by construction);
 //   3. records iterations, recurrence residual and a status per instance.
 // Instances never share rows, so clusters never wait on each other.
 #include <cooperative_groups.h>
 
 #include "assemble_impl.cuh"
+#include "pcg_common.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -51,52 +53,19 @@ struct BatchArgs {
 };
 
 constexpr int kBatchThreads = 512;
+// 256 meshes of 32^2 to 256^2 cells, ms a launch: 2 rows x 4 entries 80.9,
+// 1 x 8 94.8, 2 x 8 90.3, 3 x 4 92.2 (2 x 4 with FP64 dot products: 99.8)
 constexpr int kRowIlp = 4;  // CSR entries fetched together per row and round
 constexpr int kRows = 2;    // rows a thread advances together in the SpMV
 constexpr int kVec = 4;     // rows a thread advances together in the vector update
 
-__device__ __forceinline__ double cta_sum(double v, double* red) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-  if (lane == 0) red[warp] = v;
-  __syncthreads();
-  double t = 0;
-  if (threadIdx.x == 0)
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += red[w];
-  __syncthreads();
-  return t;  // thread 0
-}
-
-// two sums with one pair of barriers; results valid in thread 0
-__device__ __forceinline__ void cta_sum2(double& a, double& b, double (*red)[2]) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    a += __shfl_down_sync(0xffffffffu, a, o);
-    b += __shfl_down_sync(0xffffffffu, b, o);
-  }
-  if (lane == 0) {
-    red[warp][0] = a;
-    red[warp][1] = b;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    a = b = 0;
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) {
-      a += red[w][0];
-      b += red[w][1];
-    }
-  }
-  __syncthreads();
-}
-
-// combine one partial per CTA of the cluster, in rank order (same value everywhere)
-__device__ __forceinline__ double cluster_combine(cg::cluster_group& cl, double* slot) {
-  double s = 0;
-  const unsigned n = cl.num_blocks();
-  for (unsigned j = 0; j < n; ++j) s += *cl.map_shared_rank(slot, j);
-  return s;
+// acc += a b of two floats: the product exactly (FMA), the sum in double-float.
+// The products were added in native FP64 before, whose conversions and
+// multiply-adds (nine warp instructions a row and iteration at ~18 cycles each
+// on an SM) took more time than the rest of the iteration.
+TM_D void dot_add(df64& acc, float a, float b) {
+  const float p = __fmul_rn(a, b);
+  acc = acc + df64{p, __fmaf_rn(a, b, -p)};
 }
 
 template <int EL>
@@ -105,9 +74,13 @@ __global__ void __launch_bounds__(kBatchThreads, 2) batched_assemble_pcg_kernel(
   const unsigned rank = cl.block_rank();
   const unsigned C = cl.num_blocks();
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ double red[32];
-  __shared__ double red2[32][2];
-  __shared__ double part[2][3];  // [parity][pq, rz, rr]
+  static_assert(kBatchThreads == kSlotThreads, "cluster_sum's CTA size");
+  __shared__ int s_red[8 * (kSlotThreads / 32)];
+  __shared__ double s_slot[2 * 16 * 2];
+  __shared__ float s_scalar;   // alpha, then beta
+  __shared__ float s_scale[2];
+  __shared__ int s_stop;       // -1: go on, else the instance's status
+  unsigned gen = 0;
   __shared__ int task;
 
   for (;;) {
@@ -138,50 +111,55 @@ __global__ void __launch_bounds__(kBatchThreads, 2) batched_assemble_pcg_kernel(
     const int64_t r0 = rb + min(n, (int64_t)rank * per), r1 = rb + min(n, (int64_t)(rank + 1) * per);
     const float* val = static_cast<const float*>(A.mat.out);
     const float* b = static_cast<const float*>(A.load.out);
-    double rz_l = 0, rr_l = 0, bb_l = 0;
-    for (int64_t row = r0 + threadIdx.x; row < r1; row += kBatchThreads) {
-      const bool fixed = A.dirichlet[row] != 0;
-      float d = 1.f;
-      for (int64_t kk = A.indptr[row]; kk < A.indptr[row + 1]; ++kk)
-        if (A.indices[kk] == row) d = val[kk];
-      const float di = (fixed || d == 0.f) ? 0.f : 1.f / d;
-      const float rv = fixed ? 0.f : b[row];  // x0 = 0
-      const float zv = di * rv;
-      A.dinv[row] = di;
-      A.x[row] = 0.f;
-      A.r[row] = rv;
-      A.z[row] = zv;
-      A.p0[row] = zv;
-      rz_l += (double)rv * zv;
-      rr_l += (double)rv * rv;
-      bb_l += (double)rv * rv;
+    // the first sums in native FP64: they set the powers of two that bring r and
+    // z near 1 in the float products below (any units of the data)
+    double rz = 0.0, rr = 0.0, bb = 0.0, tol2 = 0.0;   // kept by thread 0
+    {
+      double rz_l = 0, rr_l = 0;
+      for (int64_t row = r0 + threadIdx.x; row < r1; row += kBatchThreads) {
+        const bool fixed = A.dirichlet[row] != 0;
+        float d = 1.f;
+        for (int64_t kk = A.indptr[row]; kk < A.indptr[row + 1]; ++kk)
+          if (A.indices[kk] == row) d = val[kk];
+        const float di = (fixed || d == 0.f) ? 0.f : 1.f / d;
+        const float rv = fixed ? 0.f : b[row];  // x0 = 0
+        const float zv = di * rv;
+        A.dinv[row] = di;
+        A.x[row] = 0.f;
+        A.r[row] = rv;
+        A.z[row] = zv;
+        A.p0[row] = zv;
+        rz_l += (double)rv * zv;
+        rr_l += (double)rv * rv;
+      }
+      cluster_sum<true>(++gen, C, rz_l, rr_l, s_red, s_slot);
+      if (threadIdx.x == 0) {
+        rz = rz_l;
+        rr = bb = rr_l;
+        tol2 = (double)A.rtol * A.rtol * bb;
+        auto half_exp = [](double v) {   // the exponent of sqrt(v), 0 for unusable v
+          const int e = fix_exp(v);
+          return e > 0 && e < 2047 ? (e - 1023) / 2 : 0;
+        };
+        const double nn = (double)(n > 0 ? n : 1);
+        const int er = half_exp(bb / nn);
+        const int ez = bb > 0.0 && rz > 0.0 ? er + fix_exp(rz / bb) - 1023 : er;
+        s_scale[0] = tm_pow2f(max(-126, min(126, -er)));
+        s_scale[1] = tm_pow2f(max(-126, min(126, -ez)));
+        s_stop = rr <= tol2 ? TM_OK : (A.maxiter <= 0 ? TM_ERR_MAXITER : -1);
+      }
+      __syncthreads();
     }
-    double t0 = cta_sum(rz_l, red), t1 = cta_sum(rr_l, red), t2 = cta_sum(bb_l, red);
-    if (threadIdx.x == 0) {
-      part[0][0] = t0;
-      part[0][1] = t1;
-      part[0][2] = t2;
-    }
-    __threadfence();
-    cl.sync();
-    double rz = cluster_combine(cl, &part[0][0]);
-    double rr = cluster_combine(cl, &part[0][1]);
-    const double bb = cluster_combine(cl, &part[0][2]);
-    const double tol2 = (double)A.rtol * A.rtol * bb;
-    cl.sync();  // part[0] is rewritten below
+    const float sr = s_scale[0], sz = s_scale[1];
+    // what a sum of scaled products is divided by
+    const double un_rr = 1.0 / ((double)sr * sr), un_rz = 1.0 / ((double)sr * sz);
 
     float beta = 0.f;
     float* pold = A.p0;
     float* pnew = A.p1;
-    int it = 0, st = TM_ERR_MAXITER;
-    int par = 1;
-    for (; it <= A.maxiter; ++it) {
-      if (rr <= tol2) {
-        st = TM_OK;
-        break;
-      }
-      if (it == A.maxiter) break;
-      double pq_l = 0;
+    int it = 0, st = s_stop;
+    while (st < 0) {
+      df64 pq_l{0.f, 0.f};
       // one thread per row, kRows rows at a time (rows row, row + T, ...), each
       // row's entries fetched kRowIlp at a time with every load of the round
       // issued before the first use: a warp keeps 32 x kRows x kRowIlp
@@ -226,22 +204,26 @@ __global__ void __launch_bounds__(kBatchThreads, 2) batched_assemble_pcg_kernel(
             const float pv = A.z[row] + beta * pold[row];
             const float qv = fixed ? 0.f : s[u];
             A.q[row] = qv;
-            pq_l += (double)pv * qv;
+            dot_add(pq_l, pv * sz, qv * sr);
           }
         }
       }
-      t0 = cta_sum(pq_l, red);
-      if (threadIdx.x == 0) part[par][0] = t0;
-      // the cluster barrier's arrive/wait carry release/acquire semantics at
-      // cluster scope: the q rows written above are visible to the other CTAs
-      cl.sync();
-      const double pq = cluster_combine(cl, &part[par][0]);
-      if (!(pq > 0.0)) {
-        st = TM_ERR_BREAKDOWN;
-        break;
+      {
+        // the cluster barrier's arrive/wait carry release/acquire semantics at
+        // cluster scope: the q rows written above are visible to the other CTAs
+        double pq = tm_to_double(pq_l), none;
+        cluster_sum<false>(++gen, C, pq, none, s_red, s_slot);
+        if (threadIdx.x == 0) {
+          pq *= un_rz;
+          if (!(pq > 0.0)) s_stop = TM_ERR_BREAKDOWN;
+          else s_scalar = (float)(rz / pq);
+        }
+        __syncthreads();
       }
-      const float alpha = (float)(rz / pq);
-      double rz_n = 0, rr_n = 0;
+      st = s_stop;
+      if (st >= 0) break;
+      const float alpha = s_scalar;
+      df64 rz_n{0.f, 0.f}, rr_n{0.f, 0.f};
       // kVec rows per round, every load of the round before any store (the
       // vectors are distinct arrays, but the compiler cannot know that and
       // would otherwise serialise the rows behind one another's stores)
@@ -269,32 +251,35 @@ __global__ void __launch_bounds__(kBatchThreads, 2) batched_assemble_pcg_kernel(
             A.x[row] = xx[u] + alpha * pv;
             A.r[row] = rv;
             A.z[row] = zv;
-            rz_n += (double)rv * zv;
-            rr_n += (double)rv * rv;
+            dot_add(rz_n, rv * sr, zv * sz);
+            dot_add(rr_n, rv * sr, rv * sr);
           }
         }
       }
-      cta_sum2(rz_n, rr_n, red2);
+      double rzs = tm_to_double(rz_n), rrs = tm_to_double(rr_n);
+      cluster_sum<true>(++gen, C, rzs, rrs, s_red, s_slot);
+      ++it;
       if (threadIdx.x == 0) {
-        part[par][1] = rz_n;
-        part[par][2] = rr_n;
+        rzs *= un_rz;
+        rr = rrs * un_rr;
+        s_scalar = (float)(rzs / rz);
+        rz = rzs;
+        if (rr <= tol2) s_stop = TM_OK;
+        else if (it == A.maxiter) s_stop = TM_ERR_MAXITER;
       }
-      cl.sync();
-      const double rzn = cluster_combine(cl, &part[par][1]);
-      rr = cluster_combine(cl, &part[par][2]);
-      beta = (float)(rzn / rz);
-      rz = rzn;
+      __syncthreads();
+      st = s_stop;
+      beta = s_scalar;
       float* tmp = pold;
       pold = pnew;
       pnew = tmp;
-      par ^= 1;
     }
     if (rank == 0 && threadIdx.x == 0) {
       A.status[k] = st;
       A.iters[k] = it;
       A.resid[k] = (float)sqrt(rr / (bb > 0 ? bb : 1.0));
     }
-    cl.sync();  // task / part reuse
+    cl.sync();  // task reuse
   }
 }
 

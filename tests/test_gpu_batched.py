@@ -82,3 +82,18 @@ def test_autotuner_picks_and_caches(tmp_path, monkeypatch):
     assert bp2.config["n_big"] == best["n_big"]
     u, info = bp2(k)
     assert int(info.status.max()) == 0
+
+
+@pytest.mark.parametrize("exponent", [-60, 40])
+def test_units_of_the_source_scale_the_solution_exactly(exponent):
+    """The dot products are formed in float pairs on values scaled by powers of
+    two, so a source in units 2^-60 or 2^40 gives the same bits, scaled."""
+    from tensormesh_gb300.batched import BatchedPoisson
+    meshes = [tg.Mesh.gen_unit_square(n, device=DEV) for n in (5, 20, 33)]
+    kappa = torch.exp(torch.randn(sum(m.n_elements for m in meshes), device=DEV,
+                                  generator=torch.Generator(DEV).manual_seed(2)))
+    base, info = BatchedPoisson(meshes)(kappa)
+    base, its = base.clone(), info.iterations.clone()
+    x, info = BatchedPoisson(meshes, source=2.0 ** exponent)(kappa)
+    assert bool((info.status == 0).all()) and torch.equal(info.iterations, its)
+    assert torch.equal(x, base * 2.0 ** exponent)
