@@ -222,8 +222,10 @@ __device__ __forceinline__ void cluster_sum(unsigned gen, unsigned nb, double& a
 // a and b (b with kTwo) become their sums over all threads of the grid, valid in
 // warp 0 of every CTA, the same bits everywhere.  Every thread of the CTA calls
 // it; the caller's __syncthreads after it completes the barrier.  Returns false
-// in warp 0 when the wait ran out (st->status is set).
-template <bool kTwo>
+// in warp 0 when the wait ran out (st->status is set).  kFence = false: only
+// the sums are exchanged; what the CTAs stored before becomes visible at the
+// next sum with fences.
+template <bool kTwo, bool kFence = true>
 __device__ __forceinline__ bool grid_sum(PcgState* st, const GridSlots& sl, unsigned gen, double& a, double& b,
                                          int* s_red, long long spin_limit = kSlotSpinLimit) {
   cta_sum<kTwo>(a, b, s_red);
@@ -232,7 +234,7 @@ __device__ __forceinline__ bool grid_sum(PcgState* st, const GridSlots& sl, unsi
   ulonglong2* set = sl.w + (gen & 1u) * 2 * (size_t)sl.nb;
   {
     if (lane == 0) {
-      __threadfence();   // the CTA's vector stores before its words
+      if (kFence) __threadfence();   // the CTA's vector stores before its words
       slot_store(set + 2 * blockIdx.x, a, gen);
       if (kTwo) slot_store(set + 2 * blockIdx.x + 1, b, gen);
     }
@@ -294,7 +296,7 @@ __device__ __forceinline__ bool grid_sum(PcgState* st, const GridSlots& sl, unsi
       }
     }
     if (ok) {
-      __threadfence();   // the other CTAs' stores before the totals
+      if (kFence) __threadfence();   // the other CTAs' stores before the totals
       if (lane < (int)kTotals) {
         slot_store(tot + lane * 8, a, gen);
         if (kTwo) slot_store(tot + lane * 8 + 1, b, gen);
@@ -317,7 +319,7 @@ __device__ __forceinline__ bool grid_sum(PcgState* st, const GridSlots& sl, unsi
       }
     }
   }
-  __threadfence();     // what the other CTAs stored before their words
+  if (kFence) __threadfence();     // what the other CTAs stored before their words
   if (!ok && lane == 0) atomicExch(&st->status, TM_ERR_TIMEOUT);
   return ok;
 }
