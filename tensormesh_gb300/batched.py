@@ -29,6 +29,7 @@ from __future__ import annotations
 
 import ctypes
 import hashlib
+import heapq
 import json
 import os
 from dataclasses import dataclass
@@ -40,6 +41,39 @@ from . import _lib, element as E_
 from .plan import PatchPlan, node_pattern
 
 from .autotune import load_cache as _load_cache, store_cache as _store_cache
+
+
+# One PCG iteration of an instance of n rows on a cluster of C CTAs, in us:
+# _ITER_US + _ROW_US[dim] * n / C.  From single instances at C = 1 .. 16 on a
+# GB300: triangles 10.7 / 6.8 / 6.6 us at 1,681 rows (C = 1 / 4 / 16),
+# 167.5 / 48.5 / 17.3 us at 66,049 rows; tetrahedra 178.9 / 52.6 / 18.2 us at
+# 15,625 rows.
+_ITER_US = 6.0
+_ROW_US = {2: 2.6e-3, 3: 11.0e-3}
+
+
+def choose_cluster(rows: Sequence[int], dim: int, slots: dict) -> int:
+    """Cluster size for a batch: the C of ``slots`` (C -> resident clusters)
+    whose estimated time is the smallest.  Instances go, largest first, to the
+    cluster that is free first, as the launch's queue hands them out; Jacobi-CG
+    takes a number of iterations that grows with the nodes along one axis.
+    Small clusters win where the batch has many times more instances than the
+    chip has clusters, large ones where a few instances set the time: 64 square
+    meshes of 32^2 .. 160^2 cells ran 26.8 / 14.8 / 9.5 / 13.4 ms at C = 2 / 4 /
+    8 / 16, 256 of 32^2 .. 256^2 cells 123.8 / 80.2 / 85.5 / 114.2 ms, 20 of
+    20^2 .. 140^2 cells 16.8 / 10.3 / 6.4 / 4.4 ms, and 200 of 20^2 cells 0.61 /
+    0.95 / 1.43 ms at C = 1 / 2 / 4.  The estimate picks the fastest of each.
+    Within 5 % the smaller C is taken: the estimate is no closer than that, and
+    on tiny systems (8 of 16^2 cells: 0.34 / 0.39 / 0.40 ms at C = 1 / 4 / 16)
+    a larger cluster only costs its barrier."""
+    rows = sorted(rows, reverse=True)
+    span = {}
+    for c, n_slots in slots.items():
+        free = [0.0] * min(n_slots, len(rows))
+        for n in rows:
+            heapq.heapreplace(free, free[0] + n ** (1.0 / dim) * (_ITER_US + _ROW_US[dim] * n / c))
+        span[c] = max(free)
+    return min(c for c in span if span[c] <= 1.05 * min(span.values()))
 
 
 @dataclass
@@ -123,7 +157,8 @@ class BatchedPoisson:
                    n_big: int = 0):
         """Patch size, cluster size of the main launch, and the big group: the
         ``n_big`` largest instances on clusters of ``cluster_big`` CTAs (no big
-        group when n_big is 0 or cluster_big is None)."""
+        group when n_big is 0 or cluster_big is None).  ``cluster=None``: 4
+        beside a big group, else by the batch's sizes (``choose_cluster``)."""
         lib = _lib.load()
         plan, pstruct, pbeg = self._plan(slot_budget)
         chunk = 128
@@ -131,9 +166,16 @@ class BatchedPoisson:
                                            _lib.TM_COEF_ELEMENT, chunk),
                    lib.tm_patch_smem_bytes(self.el_id, _lib.TM_FORM_LOAD, 1, _lib.TM_F32, ctypes.byref(pstruct),
                                            _lib.TM_COEF_SCALAR, chunk))
-        cluster = cluster or 4
         n_big = int(n_big) if cluster_big else 0
         n_big = max(0, min(n_big, self.n_inst - 1))
+        if not cluster:
+            cluster = 4
+            if n_big == 0:
+                slots = {c: lib.tm_batched_max_clusters(self.el_id, c, smem) for c in (1, 2, 4, 8, 16)}
+                slots = {c: n for c, n in slots.items() if n > 0}   # 16 is not portable: a refusal leaves it out
+                if slots:
+                    cluster = choose_cluster([b - a for a, b in zip(self.node_ptr, self.node_ptr[1:])], self.dim,
+                                             slots)
         cap = lib.tm_batched_max_clusters(self.el_id, cluster, smem)
         if cap <= 0:
             raise _lib.TensorMeshCudaError("tm_batched_max_clusters", -cap if cap < 0 else 6)

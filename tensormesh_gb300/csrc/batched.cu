@@ -358,7 +358,11 @@ extern "C" int tm_batched_max_clusters(int32_t element, int32_t cluster, int64_t
   } else {
     return -TM_ERR_UNSUPPORTED;
   }
-  return e == cudaSuccess ? n : -TM_ERR_CUDA;
+  if (e != cudaSuccess) {
+    cudaGetLastError();  // a shape that the device refuses is an answer, not an error for the next launch to report
+    return -TM_ERR_CUDA;
+  }
+  return n;
 }
 
 extern "C" int tm_batched_assemble_pcg(const tm_batched_args* a, void* stream) {
