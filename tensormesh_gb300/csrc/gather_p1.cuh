@@ -292,36 +292,68 @@ TM_D void cp_async16(void* smem, const void* gmem) {
 }
 TM_D void cp_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
-// Copies the NV values of the group's elements into shared memory, element i
-// at s_val[i * kStride]; consecutive threads copy consecutive words, so
-// elements that are neighbours in memory are read in full lines.
+// A group's element numbers, kBlk blocks of 32 per warp in registers: loaded
+// with the group's other first loads, so that the copies of the values start
+// one memory latency after the group's offsets are known.
+template <int kThreads, int kBlk> struct ElemRefs {
+  int e[kBlk];
+  TM_D void load(const int32_t* __restrict__ gelem, int n) {
+#pragma unroll
+    for (int j = 0; j < kBlk; ++j) {
+      const int i = j * kThreads + (int)threadIdx.x;
+      e[j] = i < n ? gelem[i] : 0;
+    }
+  }
+};
+
+// Copies the NV values of 32 elements (element i's in lane i's el, the first m
+// of them) to dst; consecutive lanes copy consecutive words, so elements that
+// are neighbours in memory are read in full lines.  Whole warps call it.
 template <class S, int NV, int kStride>
-TM_D void load_elements(const int32_t* __restrict__ gelem, int n, const S* __restrict__ vals, S* s_val,
-                        int nthreads) {
+TM_D void copy_elements(int el, int m, const S* __restrict__ vals, S* dst_) {
   constexpr int kBytes = NV * (int)sizeof(S);
   constexpr int kStep = kStride * (int)sizeof(S);
   constexpr int kWord = kBytes % 16 == 0 && kStep % 16 == 0 ? 16 : kBytes % 8 == 0 && kStep % 8 == 0 ? 8 : 4;
   constexpr int W = kBytes / kWord;
   const unsigned char* src = reinterpret_cast<const unsigned char*>(vals);
-  unsigned char* dst = reinterpret_cast<unsigned char*>(s_val);
-  for (int i = threadIdx.x; i < n * W; i += nthreads) {
-    const int l = i / W, w = i - l * W;
-    const void* g = src + (int64_t)gelem[l] * kBytes + w * kWord;
-    void* d = dst + (size_t)l * kStride * sizeof(S) + w * kWord;
-    if constexpr (kWord == 16) cp_async16(d, g);
-    else if constexpr (kWord == 8) cp_async8(d, g);
-    else cp_async4(d, g);
+  unsigned char* dst = reinterpret_cast<unsigned char*>(dst_);
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int s = 0; s < W; ++s) {
+    const int i = s * 32 + lane, l = i / W, w = i - l * W;
+    const int e = __shfl_sync(0xffffffffu, el, l);
+    if (l < m) {
+      const void* g = src + (int64_t)e * kBytes + w * kWord;
+      void* d = dst + l * kStep + w * kWord;
+      if constexpr (kWord == 16) cp_async16(d, g);
+      else if constexpr (kWord == 8) cp_async8(d, g);
+      else cp_async4(d, g);
+    }
   }
 }
 
-// Starts the copy of a group's elements, then the rows' value offsets:
-// s_row[k] entries before local row k, s_out[k] the row's first value minus
-// that, so that entry t of row k is value s_out[k] + t of the matrix.
-template <class St, int NV, int kStride>
-TM_D void open_group(const tm_gather_plan& plan, int g, const int32_t* __restrict__ gelem, int ne,
-                     const St* __restrict__ vals, St* s_val, int* s_row, int64_t* s_out, int nthreads) {
-  load_elements<St, NV, kStride>(gelem, ne, vals, s_val, nthreads);
-  const int r0 = g * plan.rows_per_cta, nr = min(plan.rows_per_cta, plan.n_points - r0);
+// Starts the copies of the group's n elements, element i to s_val[i * kStride].
+template <class S, int NV, int kStride, int kThreads, int kBlk>
+TM_D void load_elements(const ElemRefs<kThreads, kBlk>& refs, const int32_t* __restrict__ gelem, int n,
+                        const S* __restrict__ vals, S* s_val) {
+  const int lane = threadIdx.x & 31, w0 = (int)threadIdx.x - lane;
+#pragma unroll
+  for (int j = 0; j < kBlk; ++j) {
+    const int i0 = j * kThreads + w0;
+    if (i0 < n) copy_elements<S, NV, kStride>(refs.e[j], n - i0, vals, s_val + (size_t)i0 * kStride);
+  }
+  for (int i0 = kBlk * kThreads + w0; i0 < n; i0 += kThreads)
+    copy_elements<S, NV, kStride>(i0 + lane < n ? gelem[i0 + lane] : 0, n - i0, vals, s_val + (size_t)i0 * kStride);
+}
+
+// The value offsets of the group's rows (warp 0): s_row[k] entries before
+// local row k, s_out[k] the row's first value minus that, so that entry t of
+// row k is value s_out[k] + t of the matrix.  `first` is the lane's row of the
+// first 32, loaded ahead with `group_row`.
+TM_D int group_row(const tm_gather_plan& plan, int r0, int nr) {
+  return (int)threadIdx.x < 32 && (int)threadIdx.x < nr ? plan.order[r0 + threadIdx.x] : 0;
+}
+TM_D void row_offsets(const tm_gather_plan& plan, int r0, int nr, int first, int* s_row, int64_t* s_out) {
   const int lane = threadIdx.x & 31;
   if ((int)threadIdx.x < 32) {  // exclusive scan of the row lengths (at most 64 rows)
     int carry = 0;
@@ -330,7 +362,7 @@ TM_D void open_group(const tm_gather_plan& plan, int g, const int32_t* __restric
       int d = 0;
       int64_t p = 0;
       if (k < nr) {
-        const int r = plan.order[r0 + k];
+        const int r = b ? plan.order[r0 + k] : first;
         p = plan.indptr[r];
         d = (int)(plan.indptr[r + 1] - p);
       }
@@ -363,10 +395,13 @@ TM_D void group_wide(const int32_t* __restrict__ gelem, int ne, const uint32_t* 
 // values are copied to shared memory in full lines; one thread per entry adds
 // its list, four records a load, and writes its value; four lanes per row
 // then form the diagonal: minus the row's sum, or (kDiagList) the sum of the
-// node's diagonal values.  Bound by the latency of its load chain (element
-// list, values, records): 124 us and 354 MB of DRAM traffic for 80^3 cells
-// (2.9 TB/s).  Reading the values from global memory per record instead took
-// 148 us there and four times as many L1 sectors.
+// node's diagonal values.  No single unit bounds it: 115 us and 354 MB of DRAM
+// traffic for 80^3 cells (3.1 TB/s), issue slots 57 %, the shared-memory pipe
+// 54 % (four-way conflicts of the records' reads), the rest the latency of the
+// three dependent loads at eight CTAs an SM.  124 us with the element numbers
+// loaded a word at a time, before the entries' and rows' first loads; 148 us
+// with the values read from global memory per record, and four times as many
+// L1 sectors.
 template <class T, int B, bool kDiagList, bool kWide>
 TM_D void group_rows(const tm_gather_plan& plan, const typename Sto<T>::S* __restrict__ vals,
                      const typename Sto<T>::S* __restrict__ diag, const uint32_t* __restrict__ wide, int S,
@@ -385,9 +420,6 @@ TM_D void group_rows(const tm_gather_plan& plan, const typename Sto<T>::S* __res
   St* s_val = reinterpret_cast<St*>(s_row + 68);         // [max_elems * NV + 1], the last a zero
   St* s_sum = s_val + (((size_t)plan.max_elems * NV + 4) & ~size_t(3));        // [max_entries]
   uint32_t* s_wide = reinterpret_cast<uint32_t*>(s_sum + plan.max_entries);  // kWide: [max_elems / 32]
-  open_group<St, NV, NV>(plan, g, gelem, ne, vals, s_val, s_row, s_out, kGrpThreads);
-  if constexpr (kWide) group_wide(gelem, ne, wide, s_wide, kGrpThreads);
-  if (tid == 0) s_val[ne * NV] = St{};
   const int r0 = g * plan.rows_per_cta, nr = min(plan.rows_per_cta, plan.n_points - r0);
   const uint32_t* __restrict__ ent = plan.gent + tb;
   const uint2* __restrict__ recs = reinterpret_cast<const uint2*>(plan.grec + rb);
@@ -403,25 +435,38 @@ TM_D void group_rows(const tm_gather_plan& plan, const typename Sto<T>::S* __res
     const A v0 = value(r.x & 0xffffu), v1 = value(r.x >> 16), v2 = value(r.y & 0xffffu), v3 = value((r.y >> 16) & 0x7fffu);
     return Ar<A>::add(Ar<A>::add(v0, v1), Ar<A>::add(v2, v3));
   };
-  // kAhead entries per thread at a time; the words and first records of the
-  // first round are in flight while the elements arrive
+  // kAhead entries per thread at a time.  The first loads (elements, words,
+  // rows) go out together, then what they point to (records, values, offsets).
   constexpr int kAhead = 4;
   uint32_t w[kAhead];
   uint2 rec[kAhead];
-  auto fetch = [&](int t0) {
+  auto words = [&](int t0) {
 #pragma unroll
     for (int j = 0; j < kAhead; ++j) {
       const int t = t0 + j * kGrpThreads + tid;
       w[j] = t < nt ? ent[t] : kDiag;
     }
+  };
+  auto records = [&] {
 #pragma unroll
     for (int j = 0; j < kAhead; ++j) rec[j] = w[j] != kDiag ? recs[w[j] & 0xffffu] : make_uint2(0u, 0x80000000u);
   };
-  fetch(0);
+  ElemRefs<kGrpThreads, 4> refs;
+  refs.load(gelem, ne);
+  words(0);
+  const int row = group_row(plan, r0, nr);
+  load_elements<St, NV, NV>(refs, gelem, ne, vals, s_val);
+  records();
+  row_offsets(plan, r0, nr, row, s_row, s_out);
+  if constexpr (kWide) group_wide(gelem, ne, wide, s_wide, kGrpThreads);
+  if (tid == 0) s_val[ne * NV] = St{};
   cp_async_wait();
   __syncthreads();
   for (int t0 = 0; t0 < nt; t0 += kAhead * kGrpThreads) {
-    if (t0) fetch(t0);
+    if (t0) {
+      words(t0);
+      records();
+    }
 #pragma unroll
     for (int j = 0; j < kAhead; ++j) {
       const int t = t0 + j * kGrpThreads + tid;
@@ -524,13 +569,17 @@ TM_D void group_blocks(const tm_gather_plan& plan, const typename Sto<T>::S* __r
   uint32_t* s_wide = reinterpret_cast<uint32_t*>(s_dpos + 64);   // [64] (2048 elements)
   unsigned char* s_lrow = reinterpret_cast<unsigned char*>(s_wide + 64);   // [512] local row of each entry
   St* s_val = reinterpret_cast<St*>(s_lrow + kBlkGrpThreads);   // [max_elems][kStride], then [max_entries][HH]
-  open_group<St, NV, kStride>(plan, g, gelem, ne, vals, s_val + D, s_row, s_out, kBlkGrpThreads);
-  if constexpr (kWide) group_wide(gelem, ne, wide, s_wide, kBlkGrpThreads);
   const int r0 = g * plan.rows_per_cta, nr = min(plan.rows_per_cta, plan.n_points - r0);
   const uint16_t* __restrict__ recs = plan.grec + rb;
+  ElemRefs<kBlkGrpThreads, 1> refs;
+  refs.load(gelem, ne);
   const uint32_t w = tid < nt ? plan.gent[tb + tid] : kDiag;
+  const int row = group_row(plan, r0, nr);
+  load_elements<St, NV, kStride>(refs, gelem, ne, vals, s_val + D);
   const uint16_t* __restrict__ rec = recs + (w & 0xffffu);
   unsigned r = w != kDiag ? *rec : 0u;   // in flight while the elements arrive
+  row_offsets(plan, r0, nr, row, s_row, s_out);
+  if constexpr (kWide) group_wide(gelem, ne, wide, s_wide, kBlkGrpThreads);
   cp_async_wait();
   __syncthreads();
   // C_0 = -(C_1 + .. + C_D), once per element
