@@ -1,5 +1,7 @@
 """ElementAssembler / NodeAssembler with the reference's interface, backed by
-the CUDA patch-assembly kernels.
+the CUDA assembly kernels: element-once (every element integrated a single
+time, CSR entries summed from lists) or, on small meshes and in native FP64,
+one launch over patches of rows.
 
 Interface parity (TensorMesh):
   * ``ElementAssembler.from_mesh(mesh, quadrature_order=2, project='reduce',
@@ -18,7 +20,7 @@ Error behaviour follows the reference: AssertionError for shape mismatches,
 ValueError for a forward parameter that no data provides
 (element_assembler.py:364), NotImplementedError for an integrand that has no
 GPU kernel.  ``batch_size`` is accepted and ignored: it is a memory knob of
-the reference's quadrature chunking, and the fused kernel never materialises
+the reference's quadrature chunking, and the kernels never materialise
 per-quadrature-point tensors.
 """
 from __future__ import annotations
@@ -62,11 +64,10 @@ class MeshTopology:
         self._plans = {}
         self._gather = None
         self.scratch_bytes = {}
-        # what the calls on this mesh run on: lists of the element-once
-        # kernels, or the patch plan (each is built on first use otherwise)
-        if self.element_once:
-            self.gather.struct(1)
-        else:
+        # what the calls on this mesh run on, built here so that a first call
+        # can be captured: the lists of the element-once kernels, or the patch
+        # plan (the rest is built on first use)
+        if not self.element_once or self.gather.struct(0) is None or self.gather.struct(1) is None:
             self.plan_for(1)
         self._block = {}
         self._incidence = None
@@ -402,7 +403,9 @@ def _autotune_assembler(asm, call, dtype, budgets, reps, use_cache):
 def _assembler_autotune(self, points=None, element_data=None, point_data=None, scalar_data=None,
                         budgets=(512, 1024, 2048, 4096, 6144), reps: int = 3, use_cache: bool = True) -> dict:
     """Pick the patch size (accumulator budget per patch) that assembles
-    fastest for these inputs on this GPU; the choice is cached as JSON."""
+    fastest for these inputs on this GPU; the choice is cached as JSON.  Only
+    the patch kernels read it: where assembly runs element-once
+    (``MeshTopology.element_once``) every size takes the same time."""
     pts = self.points if points is None else points
     return _autotune_assembler(self, lambda: self(pts, element_data=element_data, point_data=point_data,
                                                   scalar_data=scalar_data), pts.dtype, budgets, reps, use_cache)

@@ -1,6 +1,7 @@
-// Specialised kernel of the headline case: P1 tetrahedra, Laplace form with a
-// scalar, per-element, nodal or per-quadrature-point coefficient, float64
-// (double-float arithmetic on the FP32 pipe) or float32.
+// Patch kernel of P1 tetrahedra (meshes below the element-once size, and
+// tm_assemble's callers): Laplace form with a scalar, per-element, nodal or
+// per-quadrature-point coefficient, float64 (double-float arithmetic on the
+// FP32 pipe) or float32.
 //
 // Same patch decomposition and deterministic row-owner accumulation as the
 // generic kernel (assemble_impl.cuh); what is specific:

@@ -1,4 +1,4 @@
-"""Mesh-only precomputation for the deterministic patch assembly.
+"""Mesh-only precomputation for the deterministic assembly kernels.
 
 This replaces the reference's ``from_mesh`` pattern build
 (assemble/element_assembler.py:838-875: scipy coo->csr->coo dedup of the
@@ -12,10 +12,12 @@ plan by torch ops) that produces:
   (RCB); each patch owns a set of CSR rows and lists every element touching
   them, with a patch-local vertex table and, for each owned row, its
   incidences (element, local vertex) sorted by element together with the
-  position of every column inside the row.
+  position of every column inside the row (``PatchPlan``);
+* the record lists of the element-once kernels (``GatherPlan``, built by the
+  project's own kernels).
 
-Everything is computed with torch ops, so it runs on the GPU when the mesh
-lives there (and on the CPU in unit tests).
+The pattern's host definition and the patch plan are torch ops, so they run on
+the GPU when the mesh lives there and on the CPU in unit tests.
 """
 from __future__ import annotations
 
