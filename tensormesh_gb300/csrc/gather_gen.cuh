@@ -1,5 +1,6 @@
-// Element-once assembly with quadrature: every form on P2 simplices, mass
-// matrices and loads on P1 ones (gather.cuh has the scheme).  A CTA integrates
+// Element-once assembly with quadrature: every form on P2 simplices and mass
+// matrices on P1 ones; the node sums of the loads (gather.cuh has the scheme,
+// gather_load.cuh the loads of P1 elements).  A CTA integrates
 // 32 elements in three phases with one barrier each:
 //   0  edge vectors and coefficients with their exponents, to shared memory;
 //   1  one thread per (quadrature point, element): Jacobian, its adjugate, the
@@ -15,7 +16,7 @@
 // Laplace, 7200 for elasticity) and so runs with few threads: calls at 27^3
 // cells 2730 -> 242 us (Laplace), 3072 elements 6916 -> 108 us (elasticity).
 #pragma once
-#include "gather_sum.cuh"
+#include "gather_load.cuh"
 
 namespace tmg {
 namespace ga {
@@ -340,7 +341,8 @@ gen_element_kernel(int64_t n_el, const int32_t* __restrict__ el, tm_assemble_arg
     // s_sexp: INT_MIN for pairs, else the exponent of the plain doubles
     const int em = s_emax[tid], ec = s_cexp[tid];
     if constexpr (kPairsT) {
-      const bool ok = em >= 200 && em <= 1846 && ec != 2047;
+      // (below 2^-923 a zero among the coefficients could not be scaled)
+      const bool ok = em >= 200 && em <= 1846 && ec != 2047 && (ec == 0 || ec > 100);
       const int em1 = ok ? em : 1023, ec1 = ok && ec ? ec : 1023;
       const int s = elem_exp(em1, ec1, G::power);
       const int r = ec == 0 ? 0 : s - head->S;
@@ -661,11 +663,17 @@ int launch_gen(const tm_gather_plan& plan, const tm_assemble_args& args, void* w
   S* diag = reinterpret_cast<S*>(sc.diag);
   if constexpr (sizeof(T) == 8)
     gen_head_kernel<T><<<1, 1, 0, s>>>(G::D, G::B, G::HC, G::power, plan.elements, args, sc.head);
-  const size_t bytes = gen_smem<EL, FORM, H, T>(args.n_quad);
-  int st = with_smem(gen_element_kernel<EL, FORM, H, T>, bytes);
-  if (st != TM_OK) return st;
-  gen_element_kernel<EL, FORM, H, T><<<(unsigned)((n + kGenEl - 1) / kGenEl), kGenThreads, bytes, s>>>(
-      n, plan.elements, args, sc.head, sc.wide, vals, diag);
+  int st = TM_OK;
+  if constexpr (G::kLoad && G::kP1) {
+    auto kern = args.coef_kind == TM_COEF_POINT ? p1_load_kernel<T, G::D, H, true> : p1_load_kernel<T, G::D, H, false>;
+    kern<<<(unsigned)((n + kElThreads - 1) / kElThreads), kElThreads, 0, s>>>(n, plan.elements, args, sc.head, sc.wide,
+                                                                              diag);
+  } else {
+    const size_t bytes = gen_smem<EL, FORM, H, T>(args.n_quad);
+    if ((st = with_smem(gen_element_kernel<EL, FORM, H, T>, bytes)) != TM_OK) return st;
+    gen_element_kernel<EL, FORM, H, T><<<(unsigned)((n + kGenEl - 1) / kGenEl), kGenThreads, bytes, s>>>(
+        n, plan.elements, args, sc.head, sc.wide, vals, diag);
+  }
   T* out = static_cast<T*>(args.out);
   if constexpr (G::kLoad) {
     sum_nodes_kernel<T, G::B, H><<<(unsigned)(((int64_t)plan.n_points * H + 255) / 256), 256, 0, s>>>(

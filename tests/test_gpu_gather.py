@@ -264,6 +264,41 @@ def test_loads_match_oracle(etype, n, q, dtype):
         assert err <= (1e-12 if dtype == torch.float64 else 1e-5), err
 
 
+@pytest.mark.parametrize("etype", ["triangle", "tetra"])
+@pytest.mark.parametrize("q", [1, 2, 4])
+@pytest.mark.parametrize("far", [1.0, 1e-150, 1e150, 1e-285])
+def test_p1_loads_of_slivers_far_units_and_far_sources(etype, q, far):
+    """Needle elements (native FP64), meshes in extreme units, and sources that
+    are tiny, huge, or zero at some points, one to three components: 1e-12 of
+    the largest entry (order 4 has more points than a thread keeps)."""
+    ring = 33
+    t = np.arange(ring) * 2 * np.pi / ring
+    if etype == "tetra":
+        pts = np.concatenate([[[0.0, 0.0, -200.0], [0.0, 0.0, 200.0]],
+                              np.stack([np.cos(t), np.sin(t), 0.1 * np.sin(3 * t)], 1)])
+        el = np.array([[0, 2 + k, 2 + (k + 1) % ring, 1] for k in range(ring)], dtype=np.int64)
+    else:
+        pts = np.concatenate([[[0.0, 3e5]], np.stack([np.cos(t), np.sin(t)], 1)])
+        el = np.array([[0, 1 + k, 1 + (k + 1) % ring] for k in range(ring)], dtype=np.int64)
+    ragged_pts, ragged_el = ragged(etype, 6 if etype == "triangle" else 4, 7)
+    for p, e, scale in ((pts, el, 1.0), (ragged_pts, ragged_el, 1e-9), (ragged_pts, ragged_el, 1e9)):
+        if far == 1e-285 and scale < 1.0:
+            continue   # subnormal results
+        p = p * scale
+        mesh = tg.Mesh(points=torch.tensor(p, device=DEV), cells={etype: torch.tensor(e, device=DEV)})
+        for H in (1, 2, 3):
+            class PointLoad(tg.NodeAssembler):
+                def forward(self, v, f):
+                    return v * f
+
+            f = far * np.random.default_rng(H).normal(size=(p.shape[0], H))
+            f[::3] = 0.0
+            got = PointLoad.from_mesh(mesh, quadrature_order=q)(
+                mesh.points, point_data={"f": torch.tensor(f[:, 0] if H == 1 else f, device=DEV)}).cpu().numpy()
+            ref = fem.assemble_load(p, e, etype, q, "point", f)
+            assert np.max(np.abs(got - ref)) <= 1e-12 * np.max(np.abs(ref)), (scale, H)
+
+
 # -- backward ----------------------------------------------------------------------
 def torch_values(pts, el, kappa, form, q_weight):
     """CSR values of a P1 mesh by plain torch (differentiable), canonical order."""
