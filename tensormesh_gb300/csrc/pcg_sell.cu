@@ -299,20 +299,29 @@ TM_D void sell_rows(const int64_t* __restrict__ sptr, const CT* scol, const S* s
   for (int u = 0; u < kSellRows; ++u) acc[u] = Tr::done(sum[u]);
 }
 
-// Standard (Hestenes-Stiefel) Jacobi-PCG over the SELL-32 copy of A M, two
-// grid barriers per iteration.  With pt = M^-1 p (so that A p = (A M) pt and
-// pt_new = r + beta pt_old), an iteration is
-//   sweep 1: q = (A M)(r + beta pt_old), gathering r and pt_old and forming
-//            the combination per column; pt_new (own rows) to the other half
-//            of a double buffer; partial (p, q) = sum M pt q       [barrier]
+// Standard (Hestenes-Stiefel) Jacobi-PCG over the SELL-32 copy of A M.  With
+// pt = M^-1 p (so that A p = (A M) pt and pt_new = r + beta pt_old), an
+// iteration is
+//   sweep 1: q = (A M) pt_new; partial (p, q) = sum M pt q         [barrier]
 //   sweep 2: alpha = rz / (p, q); x += alpha M pt; r -= alpha q; partial
 //            rz = sum M r^2 and rr = sum r^2                        [barrier]
+// pt_new: kResident and kCluster gather r and pt_old in sweep 1 and form the
+// combination per column (own rows go to the other half of a double buffer):
+// their iterations are barriers, and a third would cost more than it saves.
+// kGrid updates pt in a sweep of its own, with a barrier after it, and gathers
+// one value per entry instead of two and a multiply-add.
 // The iterates are those of tm_pcg_jacobi's recurrence (z = M r, p = z +
 // beta p), so its rounding behaviour is that of standard PCG.  The barriers are
 // the grid sums (grid_sum); the scalars' FP64 divisions and the square root run
 // in one thread of a CTA.
 //
-// kMode kGrid streams the matrix.  kResident: a CTA's share of the matrix, x, q, M and its own rows of r and pt stay
+// kMode kGrid streams the matrix; of its own-row vectors the first `cap` of r,
+// q, x and M stay in shared memory.  Bound by the latency of the gathers and
+// the matrix stream.  us per iteration, a call's other work included, with r
+// and pt_old gathered and every vector in global memory / pt in a sweep of its
+// own / vectors in shared memory as well: 64^3 Poisson 21.3 / 20.4 / 19.0, 96^3
+// 53.5 / 53.5 / 46.3, 128^3 116 / 109 / 102, 1000^2 38.9 / - / 30.1, 40^3
+// elasticity 42.6 / 39.4 / 28.8.  kResident: a CTA's share of the matrix, x, q, M and its own rows of r and pt stay
 // in shared memory for the whole solve, and an iteration reads only the
 // gathered r and pt from L2.  kCluster: the same in one cluster, whose barriers
 // take a microsecond instead of three.  Chosen by launch_pcg_sell; a CTA whose
@@ -372,13 +381,26 @@ pcg_sell_hs_kernel(int64_t n, const int64_t* __restrict__ sptr, const CT* __rest
       mcol = mc - k0;
     }
     __syncthreads();
+  } else {
+    const int64_t rows = per * 32;
+    S* s = reinterpret_cast<S*>(smem_raw);
+    if (cap > 0) orr = s - row0;
+    if (cap > 1) oq = s + rows - row0;
+    if (cap > 2) ox = s + 2 * rows - row0;
+    if (cap > 3) {
+      S* d = s + 3 * rows - row0;
+      for (int64_t i = row0 + threadIdx.x; i < min(n, s_hi * 32); i += kSellThreads) d[i] = dinv[i];
+      od = d;
+      __syncthreads();
+    }
   }
   auto product = [&](const auto& g, int64_t sl, A (&acc)[kSellRows]) {
     sell_rows<S, CT, kRes>(sptr, mcol, mval, g, sl, s_hi, acc);
   };
   // one sum, no fences: sweep 2 reads and writes own rows only, and a CTA's sum
   // is published after its gathers of sweep 1 have returned; the stores of both
-  // sweeps become visible at barrier2
+  // sweeps become visible at barrier2 (kGrid: others read pt alone, which has
+  // its own barrier, so barrier2 needs no fences either)
   auto barrier1 = [&](double& a) -> bool {
     double b = 0.0;
     if constexpr (kMode == kCluster) {
@@ -393,7 +415,7 @@ pcg_sell_hs_kernel(int64_t n, const int64_t* __restrict__ sptr, const CT* __rest
       cluster_sum<true>(++gen, nb, a, b, s_red, s_slot);
       return true;
     } else {
-      return grid_sum<true>(st, gs, ++gen, a, b, s_red);
+      return grid_sum<true, kRes>(st, gs, ++gen, a, b, s_red);
     }
   };
   // Ends a barrier: lane 0 of warp 0 runs f on the sums (it sets s_scalar and s_stop).
@@ -420,9 +442,9 @@ pcg_sell_hs_kernel(int64_t n, const int64_t* __restrict__ sptr, const CT* __rest
         const int64_t row = row_of(sl, u);
         const A b = Tr::in(bv[row]);
         const A rv = b - acc[u];
-        Tr::st(r, row, rv);
+        Tr::st(orr, row, rv);
         if constexpr (kRes) {
-          Tr::st(orr, row, rv);
+          Tr::st(r, row, rv);
           Tr::st(op, row, Tr::zero());
         }
         Tr::st(ox, row, Tr::in(xv[row]));
@@ -458,19 +480,35 @@ pcg_sell_hs_kernel(int64_t n, const int64_t* __restrict__ sptr, const CT* __rest
   int it = 0;
   int status = s_stop;
   while (status < 0) {
+    if constexpr (!kRes) {
+      // pt = r + beta pt, own rows
+      for (int64_t sl = s_lo + warp; sl < s_hi; sl += kSellWarps) {
+        const int64_t row = sl * 32 + lane;
+        if (row < n) Tr::st(pt0, row, Tr::axpy(Tr::ld(orr, row), beta, Tr::ld(pt0, row)));
+      }
+      double a = 0.0, b = 0.0;
+      const bool ok = grid_sum<false, true>(st, gs, ++gen, a, b, s_red);
+      if (!finish(ok, [] {})) return;
+    }
     // sweep 1
     A pq_l = Tr::zero();
     const S* cpold = pold;
     for (int64_t sl = s_lo + warp; sl < s_hi; sl += (int64_t)kSellRows * kSellWarps) {
       A acc[kSellRows];
-      product([&](int c) { return Tr::axpy(Tr::ld(r, c), beta, Tr::ld(cpold, c)); }, sl, acc);
+      if constexpr (kRes) product([&](int c) { return Tr::axpy(Tr::ld(r, c), beta, Tr::ld(cpold, c)); }, sl, acc);
+      else product([&](int c) { return Tr::ld(pt0, c); }, sl, acc);
 #pragma unroll
       for (int u = 0; u < kSellRows; ++u) {
         if (!valid(sl, u)) continue;
         const int64_t row = row_of(sl, u);
-        const A pv = Tr::axpy(Tr::ld(orr, row), beta, Tr::ld(kRes ? op : cpold, row));
-        Tr::st(pnew, row, pv);
-        if constexpr (kRes) Tr::st(op, row, pv);
+        A pv;
+        if constexpr (kRes) {
+          pv = Tr::axpy(Tr::ld(orr, row), beta, Tr::ld(op, row));
+          Tr::st(pnew, row, pv);
+          Tr::st(op, row, pv);
+        } else {
+          pv = Tr::ld(pt0, row);
+        }
         Tr::st(oq, row, acc[u]);
         pq_l += Tr::ld(od, row) * pv * acc[u];
       }
@@ -490,12 +528,12 @@ pcg_sell_hs_kernel(int64_t n, const int64_t* __restrict__ sptr, const CT* __rest
     for (int64_t sl = s_lo + warp; sl < s_hi; sl += kSellWarps) {
       const int64_t row = sl * 32 + lane;
       if (row >= n) continue;
-      const A di = Tr::ld(od, row), pv = Tr::ld(kRes ? op : pnew, row), qv = Tr::ld(oq, row);
+      const A di = Tr::ld(od, row), pv = Tr::ld(kRes ? op : pt0, row), qv = Tr::ld(oq, row);
       const A xo = Tr::ld(ox, row), ro = Tr::ld(orr, row);
       const A rn = ro - alpha * qv;
       Tr::st(ox, row, xo + alpha * (di * pv));
-      Tr::st(r, row, rn);
-      if constexpr (kRes) Tr::st(orr, row, rn);
+      Tr::st(orr, row, rn);
+      if constexpr (kRes) Tr::st(r, row, rn);
       rz_l += di * rn * rn;
       rr_l += rn * rn;
     }
@@ -748,6 +786,12 @@ constexpr int kSellMaxBlocks = 4096;
 // 128^3 127 / 172, 64^3 31.2 / 27.3).
 constexpr int kSlicesPerCta = 48;
 
+// Own-row vectors in shared memory, an SM: what they take, the L1 loses, and
+// the gathers live on it.  128^3 (54 KB a vector and CTA): 109 us an iteration
+// with none, 102 with r, 118 with r and q (216 KB); 96^3 with all four (180 KB)
+// 46, with none 54.
+constexpr size_t kGridVectorBytes = 184 * 1024;
+
 template <class K>
 int sell_blocks(K kern, int64_t n_slices) {
   int dev = 0, sms = 0, per_sm = 0;
@@ -783,7 +827,7 @@ size_t resident_bytes(int64_t n_slices, int64_t n_pad, int nb, int optin, int& c
 // (2D to 270,000 rows, 3D to 130,000), streaming otherwise.  us per iteration,
 // a call's other work included: 64^2 6.5 in a cluster, 10.0 on the grid, 15.0
 // before (atomic barriers, FP64 shuffle trees, divisions in every thread);
-// 256^2 11.0 resident, 16.2 before; 96^3 57 streaming, 65 before.
+// 256^2 9.3 resident, 16.2 before; 96^3 46 streaming, 65 before.
 template <class S, class CT>
 int sell_launch(int64_t n_slices, int64_t n_pad, SellLaunch& how) {
   int dev = 0, sms = 0, optin = 0;
@@ -823,7 +867,23 @@ int sell_launch(int64_t n_slices, int64_t n_pad, SellLaunch& how) {
     how.bytes = bytes;
     return TM_OK;
   }
-  how.nb = sell_blocks(pcg_sell_hs_kernel<S, CT, kGrid>, n_slices);
+  auto kern = pcg_sell_hs_kernel<S, CT, kGrid>;
+  how.nb = sell_blocks(kern, n_slices);
+  if (how.nb <= 0) return TM_OK;
+  how.cap = 0;   // kGrid: vectors in shared memory
+  const int per_sm = how.nb > sms ? 2 : 1;
+  const size_t vec = (size_t)((n_slices + how.nb - 1) / how.nb) * 32 * sizeof(S);
+  for (int k = 4; k > 0; --k) {
+    int fit = 0;
+    if (k * vec > (size_t)optin || k * vec * per_sm > kGridVectorBytes ||
+        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(k * vec)) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, kern, kSellThreads, k * vec) != cudaSuccess || fit < per_sm)
+      continue;
+    how.cap = k;
+    how.bytes = k * vec;
+    break;
+  }
+  cudaGetLastError();   // a refused size only leaves a vector out
   return TM_OK;
 }
 

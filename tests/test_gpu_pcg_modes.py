@@ -128,3 +128,32 @@ def test_iteration_cap_zero_and_one():
         with pytest.warns(UserWarning, match="did not converge"):
             K.solve(f, rtol=1e-10, maxiter=cap)
         assert K.last_solve_info.iterations == cap and K.last_solve_info.status == _lib.TM_ERR_MAXITER
+
+
+@pytest.mark.parametrize("n", [600_001, 1_000_000, 1_500_033, 2_500_000, 3_800_001])
+@pytest.mark.parametrize("far", [1000, 40_000])
+@pytest.mark.parametrize("dtype", [torch.float64, torch.float32])
+def test_streaming_grid_sizes(n, far, dtype):
+    """Systems too large for shared memory, with four to none of the own-row
+    vectors held there, 16-bit and 32-bit columns: the residual, formed by
+    torch in float64, against the tolerance asked for (condition number below
+    nine, so float32 reaches 1e-4 with a rounding floor near 1e-6)."""
+    i = torch.arange(n, device=DEV)
+    offs = torch.tensor([-far, -1, 0, 1, far], device=DEV)
+    cols = i[:, None] + offs
+    inside = (cols >= 0) & (cols < n)
+    g = torch.Generator(device=DEV).manual_seed(n)
+    scale = torch.exp(torch.randn(n, generator=g, device=DEV, dtype=torch.float64))   # Jacobi undoes it
+    base = torch.tensor([-1.0, -1.0, 5.0, -1.0, -1.0], device=DEV, dtype=torch.float64).expand(n, 5)
+    vals = (base * (scale[:, None] * scale[cols.clamp(0, n - 1)]).sqrt())[inside].to(dtype)
+    indptr = torch.zeros(n + 1, dtype=torch.int64, device=DEV)
+    indptr[1:] = torch.cumsum(inside.sum(1), 0)
+    K = tg.SparseMatrix(vals, shape=(n, n), indptr=indptr, indices=cols[inside].to(torch.int32))
+    b = torch.randn(n, generator=g, device=DEV, dtype=torch.float64).to(dtype)
+    rtol = 1e-9 if dtype == torch.float64 else 1e-4
+    x = K.solve(b, rtol=rtol)
+    assert K.last_solve_info.status == 0
+    A = torch.sparse_csr_tensor(indptr, K.indices.long(), vals.double(), size=(n, n))
+    res = b.double() - (A @ x.double()[:, None])[:, 0]
+    assert float(res.norm() / b.double().norm()) <= rtol * (1.0 if dtype == torch.float64 else 1.1)
+    assert torch.equal(K.solve(b, rtol=rtol), x)
