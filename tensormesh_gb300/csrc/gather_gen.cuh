@@ -643,8 +643,10 @@ int with_smem(K kern, size_t bytes) {
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
   if (bytes > (size_t)optin) return TM_ERR_INDEX;
+  // the most a block may have, not `bytes`: another thread's smaller plan must
+  // not lower it between here and the launch
   if (bytes > 48 * 1024 &&
-      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess)
+      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, optin) != cudaSuccess)
     return TM_ERR_CUDA;
   return TM_OK;
 }

@@ -711,8 +711,10 @@ int launch_group(K kern, const tm_gather_plan& plan, int threads, size_t bytes, 
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
   if (bytes > (size_t)optin) return TM_ERR_INDEX;
+  // the most a block may have, not `bytes`: another thread's smaller plan must
+  // not lower it between here and the launch
   if (bytes > 48 * 1024 &&
-      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess)
+      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, optin) != cudaSuccess)
     return TM_ERR_CUDA;
   const int grid = (plan.n_points + plan.rows_per_cta - 1) / plan.rows_per_cta;
   kern<<<grid, threads, bytes, s>>>(plan, args...);

@@ -834,10 +834,13 @@ int sell_launch(int64_t n_slices, int64_t n_pad, SellLaunch& how) {
   if (cudaGetDevice(&dev) != cudaSuccess) return TM_ERR_CUDA;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  // the attribute is set to the most any launch takes, not to this one's bytes:
+  // another thread's smaller system must not lower it before the launch
+  const int most = optin - 4 * 1024;
   for (int nb = 16; nb >= 8; nb /= 2) {
     const size_t bytes = resident_bytes<S, CT>(n_slices, n_pad, nb, optin, how.cap);
     auto kern = pcg_sell_hs_kernel<S, CT, kCluster>;
-    if (!bytes || cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess ||
+    if (!bytes || cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, most) != cudaSuccess ||
         cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
       continue;
     cudaLaunchConfig_t cfg{};
@@ -861,7 +864,7 @@ int sell_launch(int64_t n_slices, int64_t n_pad, SellLaunch& how) {
   const int nb = (int)min((int64_t)sms, n_slices);
   const size_t bytes = nb > 0 ? resident_bytes<S, CT>(n_slices, n_pad, nb, optin, how.cap) : 0;
   if (bytes && cudaFuncSetAttribute(pcg_sell_hs_kernel<S, CT, kResident>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)bytes) == cudaSuccess) {
+                                    most) == cudaSuccess) {
     how.mode = kResident;
     how.nb = nb;
     how.bytes = bytes;
@@ -875,8 +878,8 @@ int sell_launch(int64_t n_slices, int64_t n_pad, SellLaunch& how) {
   const size_t vec = (size_t)((n_slices + how.nb - 1) / how.nb) * 32 * sizeof(S);
   for (int k = 4; k > 0; --k) {
     int fit = 0;
-    if (k * vec > (size_t)optin || k * vec * per_sm > kGridVectorBytes ||
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(k * vec)) != cudaSuccess ||
+    if (k * vec > (size_t)most || k * vec * per_sm > kGridVectorBytes ||
+        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, most) != cudaSuccess ||
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, kern, kSellThreads, k * vec) != cudaSuccess || fit < per_sm)
       continue;
     how.cap = k;
