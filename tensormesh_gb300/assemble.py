@@ -63,10 +63,12 @@ class MeshTopology:
         self._coords = points.detach()
         self._plans = {}
         self._gather = None
+        self._lock = threading.Lock()
         self.scratch_bytes = {}
-        # what the calls on this mesh run on, built here so that a first call
-        # can be captured: the lists of the element-once kernels, or the patch
-        # plan (the rest is built on first use)
+        # what scalar forms and loads run on, built here so that their first
+        # call can be captured: the lists of the element-once kernels, or the
+        # patch plan.  The first call or gradient of another kind (H x H blocks,
+        # gradients of patch forms) builds what it needs.
         if not self.element_once or self.gather.struct(0) is None or self.gather.struct(1) is None:
             self.plan_for(1)
         self._block = {}
@@ -97,10 +99,13 @@ class MeshTopology:
     @property
     def gather(self) -> GatherPlan:
         if self._gather is None:
-            self._refusals()
-            t0 = _now(self.elements.device)
-            self._gather = GatherPlan(self.elements, self._coords, self.pattern)
-            self.timings["gather_s"] = _now(self.elements.device) - t0
+            with self._lock:
+                if self._gather is None:
+                    self._refusals()
+                    t0 = _now(self.elements.device)
+                    lists = GatherPlan(self.elements, self._coords, self.pattern)
+                    self.timings["gather_s"] = _now(self.elements.device) - t0
+                    self._gather = lists   # complete on every stream, as plan_for's plans are
         return self._gather
 
     def _refusals(self):

@@ -22,6 +22,7 @@ the GPU when the mesh lives there and on the CPU in unit tests.
 from __future__ import annotations
 
 import math
+import threading
 from dataclasses import dataclass
 
 import torch
@@ -445,6 +446,7 @@ class GatherPlan:
         dev = elements.device
         self.pattern, self.elements = pattern, elements
         self._structs = {}
+        self._lock = threading.Lock()
         self.p1 = B <= 4
         self.ok = dev.type == "cuda" and E > 0 and E * B < 2**31 - 1 and pattern.nnz < 2**31 - 1 and \
             E * (B * (B - 1) // 2) < (1 << 30) - 1 and not self._repeats(elements)
@@ -480,7 +482,13 @@ class GatherPlan:
         if not self.ok:
             return None
         if H not in self._structs:
-            self._structs[H] = self._groups(H)
+            with self._lock:
+                if H not in self._structs:
+                    s = self._groups(H)
+                    # complete before any call sees it: the next one may run on
+                    # another stream, which nothing orders behind the fill
+                    torch.cuda.synchronize(self.elements.device)
+                    self._structs[H] = s
         s = self._structs[H]
         return None if s is None else s[0]
 

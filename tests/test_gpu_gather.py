@@ -350,3 +350,50 @@ def test_p1_gradients_match_torch(etype, n, form, data, dtype):
         assert err <= (1e-11 if dtype == torch.float64 else 1e-4), err
     again = torch.autograd.grad(asm(xg, **{data: {"kappa": kg}}).values, (xg, kg), G.to(dtype))
     assert all(torch.equal(a, b) for a, b in zip(got, again))
+
+
+# -- streams -------------------------------------------------------------------------
+@pytest.mark.parametrize("etype,n,H", [("triangle", 5, 1), ("tetra", 4, 1), ("tetra", 4, 3), ("tetra10", 2, 1)])
+def test_lists_are_complete_when_they_become_visible(etype, n, H, monkeypatch):
+    """The stream that built the lists is idle when ``struct`` returns, even
+    where the last kernels of the build take long: a call on any other stream
+    may read them at once."""
+    pts, el = (curved if etype == "tetra10" else ragged)(etype, n, 3)
+    mesh = tg.Mesh(points=torch.tensor(pts, device=DEV), cells={etype: torch.tensor(el, device=DEV)})
+    topo = KappaLaplace.from_mesh(mesh).topology
+    plan = tg.plan.GatherPlan(topo.elements, mesh.points, topo.pattern)
+    inner, fills = tg._lib.call, []
+
+    def slow_fill(name, *args):
+        inner(name, *args)
+        if name in ("tm_group_fill", "tm_gather_fill"):
+            fills.append(name)
+            torch.cuda._sleep(100_000_000)
+
+    monkeypatch.setattr(tg._lib, "call", slow_fill)
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        assert plan.struct(H) is not None
+        assert fills and side.query()
+
+
+@pytest.mark.parametrize("etype,n,form", [("tetra", 6, "laplace"), ("tetra", 6, "elasticity"), ("tetra10", 3, "laplace"),
+                                          ("tetra10", 3, "elasticity")])
+def test_first_calls_of_a_mesh_on_two_streams(etype, n, form):
+    """A mesh's first call on one stream and its second on another, with no
+    order between the two, give the values of a later call on the device's
+    default stream."""
+    pts, el = (curved if etype == "tetra10" else ragged)(etype, n, 5)
+    x, k = torch.tensor(pts, device=DEV), torch.rand(el.shape[0], dtype=torch.float64, device=DEV) + 0.5
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    torch.cuda.synchronize()
+    with torch.cuda.stream(streams[0]):
+        asm = FORMS[form].from_mesh(tg.Mesh(points=x, cells={etype: torch.tensor(el, device=DEV)}), 2)
+    got = []
+    for s in streams[::-1] + streams:
+        with torch.cuda.stream(s):
+            got.append(asm(x, element_data={"kappa": k}).values)
+    torch.cuda.synchronize()
+    ref = asm(x, element_data={"kappa": k}).values
+    assert all(torch.equal(v, ref) for v in got)
