@@ -190,10 +190,15 @@ __device__ __forceinline__ void cta_sum(double& a, double& b, int* s_red /* [8][
   if (kTwo) b = total(5, eb);
 }
 
+__device__ __forceinline__ void cluster_barrier() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
 // The same over a cluster: every CTA writes its sums into the shared memory of
 // all of them (s_slot[2 sets][16][2], alternating like the grid's words) and
 // one hardware cluster barrier, which also orders the CTAs' global stores,
-// stands between the writes and the reads.
+// stands between the writes and the reads.  The caller has passed a cluster
+// barrier before its first sum, so that all of them have started.
 template <bool kTwo>
 __device__ __forceinline__ void cluster_sum(unsigned gen, unsigned nb, double& a, double& b, int* s_red,
                                             double* s_slot) {
@@ -207,7 +212,7 @@ __device__ __forceinline__ void cluster_sum(unsigned gen, unsigned nb, double& a
     asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(dst), "d"(a) : "memory");
     if (kTwo) asm volatile("st.shared::cluster.f64 [%0+8], %1;" ::"r"(dst), "d"(b) : "memory");
   }
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+  cluster_barrier();
   if (threadIdx.x < 32) {
     auto sum = [&](int k) {
       const double d = lane < (int)nb ? set[2 * lane + k] : 0.0;

@@ -346,6 +346,9 @@ pcg_sell_hs_kernel(int64_t n, const int64_t* __restrict__ sptr, const CT* __rest
   const GridSlots gs{slots, nb};
   unsigned gen = 0;        // the host zeroes the slots before the launch
   if (*((volatile int*)&st->status) != TM_OK) return;  // slice plan rejected by the fill kernel
+  // every CTA of the cluster runs before one writes into another's shared
+  // memory: a CTA without rows reaches its first cluster_sum at once
+  if constexpr (kMode == kCluster) cluster_barrier();
   const int64_t n_slices = (n + 31) >> 5;
   const int64_t per = (n_slices + nb - 1) / nb;
   const int64_t s_lo = min(n_slices, (int64_t)blockIdx.x * per), s_hi = min(n_slices, s_lo + per);

@@ -157,3 +157,27 @@ def test_streaming_grid_sizes(n, far, dtype):
     res = b.double() - (A @ x.double()[:, None])[:, 0]
     assert float(res.norm() / b.double().norm()) <= rtol * (1.0 if dtype == torch.float64 else 1.1)
     assert torch.equal(K.solve(b, rtol=rtol), x)
+
+
+@pytest.mark.parametrize("n", [1, 2, 31, 32, 33, 64, 65, 96, 255, 257, 480, 511, 512, 513])
+@pytest.mark.parametrize("dtype", [torch.float64, torch.float32])
+def test_clusters_with_ctas_that_own_no_rows(n, dtype):
+    """Fewer slices than the cluster has CTAs, many launches in a row: the
+    same bits each time, and the tridiagonal system's dense solution."""
+    i = torch.arange(n, device=DEV)
+    cols = i[:, None] + torch.tensor([-1, 0, 1], device=DEV)
+    inside = (cols >= 0) & (cols < n)
+    vals = torch.tensor([-1.0, 4.0, -1.0], device=DEV, dtype=dtype).expand(n, 3)[inside]
+    indptr = torch.zeros(n + 1, dtype=torch.int64, device=DEV)
+    indptr[1:] = torch.cumsum(inside.sum(1), 0)
+    K = tg.SparseMatrix(vals, shape=(n, n), indptr=indptr, indices=cols[inside].to(torch.int32))
+    b = torch.randn(n, generator=torch.Generator(device=DEV).manual_seed(n), device=DEV, dtype=torch.float64).to(dtype)
+    rtol = 1e-12 if dtype == torch.float64 else 1e-5
+    x = K.solve(b, rtol=rtol)
+    A = 4.0 * torch.eye(n, dtype=torch.float64, device=DEV)
+    A -= torch.diag(torch.ones(n - 1, dtype=torch.float64, device=DEV), 1)
+    A -= torch.diag(torch.ones(n - 1, dtype=torch.float64, device=DEV), -1)
+    ref = torch.linalg.solve(A, b.double())
+    # the residual's relative size times the condition number (below three), and the value type's rounding
+    assert float((x.double() - ref).norm() / ref.norm()) <= 3 * rtol + 16 * torch.finfo(dtype).eps
+    assert all(torch.equal(K.solve(b, rtol=rtol), x) for _ in range(20))
