@@ -168,6 +168,8 @@ int tm_assemble(const tm_patch_plan* plan, const tm_assemble_args* args, void* s
  *   ent[nnz], rec[]
  * max_entries, max_elems: most CSR entries and elements of one group (P2:
  * entries of one CTA's rows).  Calls that run at the same time need a work array each.
+ * Alignment: work 16 bytes, elements 16 bytes for TM_TET4, grec 8 bytes
+ * (TM_ERR_INVALID otherwise).
  */
 typedef struct tm_gather_plan {
   int32_t n_elements;

@@ -53,6 +53,9 @@ class MeshTopology:
             f"{element_type} elements have {self.n_basis} nodes, but the connectivity has {elements.shape[1]} columns"
         check_connectivity(elements, int(points.shape[0]))
         self.elements = elements.to(torch.int32).contiguous()
+        if self.elements.data_ptr() % 16:   # a view into a larger array: the kernels read four nodes at once
+            self.elements = self.elements.clone()
+        self._source = elements   # kept: topology_for knows a connectivity by its address
         self._elements_long = elements.long()
         self.n_points = int(points.shape[0])
         self.n_elements = int(elements.shape[0])

@@ -77,6 +77,10 @@ extern "C" int tm_assemble_gather(const tm_gather_plan* plan, const tm_assemble_
     }
   }
   if (work_bytes < need) return TM_ERR_INDEX;
+  // the widest accesses: a tetrahedron's four nodes, quads of records, runs of values
+  auto off = [](const void* p, uintptr_t to) { return reinterpret_cast<uintptr_t>(p) % to != 0; };
+  if (off(work, 16) || (args->element == TM_TET4 && off(plan->elements, 16))) return TM_ERR_INVALID;
+  if (args->form != TM_FORM_LOAD && is_p1(args->element) && off(plan->grec, 8)) return TM_ERR_INVALID;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (closed_form(args->element, args->form)) return assemble_p1(*plan, *args, work, s);
   switch (args->element) {

@@ -65,3 +65,28 @@ def test_null_pointers_unknown_dtypes_and_flags_are_rejected(lib):
 def test_network_entries_reject_negative_sizes(lib):
     assert lib.tm_mpnn_input_fwd(-1, FAKE, FAKE, FAKE, FAKE, FAKE, FAKE, FAKE, None) == INV
     assert lib.tm_gather_axpy_f32(-1, FAKE, FAKE, FAKE, FAKE, FAKE, FAKE, FAKE, None) == INV
+
+
+def gather_call(element=_lib.TM_TET4, form=_lib.TM_FORM_LAPLACE, n_comp=1):
+    """Arguments of a tm_assemble_gather call that names every array."""
+    plan = _lib.GatherPlan()
+    plan.n_elements, plan.n_points, plan.rows_per_cta, plan.max_entries, plan.max_elems = 8, 20, 8, 100, 8
+    for name in ("elements", "indptr", "nptr", "nrec", "order", "base", "gelem", "gent", "grec", "ent", "rec"):
+        setattr(plan, name, FAKE)
+    a = _lib.AssembleArgs()
+    a.element, a.form, a.dtype, a.precision = element, form, _lib.TM_F64, _lib.TM_PREC_EMULATED
+    a.coef_kind, a.n_comp, a.n_quad = _lib.TM_COEF_SCALAR, n_comp, 1
+    a.tables = a.points = a.out = FAKE
+    return plan, a
+
+
+def test_element_once_arrays_of_wrong_alignment_are_rejected(lib):
+    for off in (4, 8, 12):
+        for form in (_lib.TM_FORM_LAPLACE, _lib.TM_FORM_ELASTICITY, _lib.TM_FORM_MASS, _lib.TM_FORM_LOAD):
+            plan, a = gather_call(form=form)
+            assert lib.tm_assemble_gather(plan, a, FAKE + off, 1 << 20, None) == INV
+            plan.elements = FAKE + off
+            assert lib.tm_assemble_gather(plan, a, FAKE, 1 << 20, None) == INV
+    plan, a = gather_call(element=_lib.TM_TRI3)
+    plan.grec = FAKE + 4
+    assert lib.tm_assemble_gather(plan, a, FAKE, 1 << 20, None) == INV

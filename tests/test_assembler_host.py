@@ -42,3 +42,16 @@ def test_facet_topology_groups_pairs_by_node_in_order():
         assert bool((nodes[group] == n).all())
         assert bool((group[1:] > group[:-1]).all())
     assert int(topo.ptr[-1]) == nodes.numel()
+
+
+@pytest.mark.parametrize("word", [1, 2, 3])
+def test_connectivity_at_an_odd_address_is_copied(word):
+    """A connectivity that is a view into a larger int32 array, at any word."""
+    mesh = tg.Mesh.gen_unit_cube(2)
+    el = mesh.cells["tetra"].to(torch.int32)
+    flat = torch.zeros(el.numel() + word, dtype=torch.int32)
+    flat[word:] = el.reshape(-1)
+    view = flat[word:].view(-1, 4)
+    assert view.data_ptr() % 16 and view.is_contiguous()
+    topo = tg.assemble.MeshTopology(view, mesh.points, "tetra")
+    assert topo.elements.data_ptr() % 16 == 0 and torch.equal(topo.elements, el)

@@ -397,3 +397,25 @@ def test_first_calls_of_a_mesh_on_two_streams(etype, n, form):
     torch.cuda.synchronize()
     ref = asm(x, element_data={"kappa": k}).values
     assert all(torch.equal(v, ref) for v in got)
+
+
+# -- alignment ---------------------------------------------------------------------
+@pytest.mark.parametrize("word", [1, 2, 3])
+def test_connectivity_at_an_odd_address(word):
+    """A tetrahedral connectivity that starts at any word of a larger array:
+    loads, matrices and gradients are those of a connectivity of its own."""
+    pts, el = ragged("tetra", 4, word)
+    x, own = torch.tensor(pts, device=DEV), torch.tensor(el, device=DEV, dtype=torch.int32)
+    flat = torch.zeros(own.numel() + word, dtype=torch.int32, device=DEV)
+    flat[word:] = own.reshape(-1)
+    view = flat[word:].view(-1, 4)
+    load = tg.const_node_assembler(2.0)
+    assert torch.equal(load.from_elements(x, {"tetra": view}, 2, DEV, torch.float64)(x),
+                       load.from_elements(x, {"tetra": own}, 2, DEV, torch.float64)(x))
+    k = torch.rand(el.shape[0], dtype=torch.float64, device=DEV) + 0.5
+    got = []
+    for cells in (view, own):
+        xg = x.clone().requires_grad_(True)
+        v = KappaLaplace(tg.assemble.topology_for(cells, x, "tetra"), x, 2)(xg, element_data={"kappa": k}).values
+        got.append((v, *torch.autograd.grad(v.square().sum(), xg)))
+    assert all(torch.equal(a, b) for a, b in zip(*got))
