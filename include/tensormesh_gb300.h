@@ -168,6 +168,8 @@ int tm_assemble(const tm_patch_plan* plan, const tm_assemble_args* args, void* s
  *   ent[nnz], rec[]
  * max_entries, max_elems: most CSR entries and elements of one group (P2:
  * entries of one CTA's rows).  Calls that run at the same time need a work array each.
+ * Limits of P1 groups (TM_ERR_INVALID beyond): 64 rows; elasticity 512 entries
+ * and 2048 elements; scalar forms 32767 elements times node pairs.
  * Alignment: work 16 bytes, elements 16 bytes for TM_TET4, grec 8 bytes
  * (TM_ERR_INVALID otherwise).
  */
@@ -206,7 +208,7 @@ int tm_assemble_gather(const tm_gather_plan* plan, const tm_assemble_args* args,
  * consumes cnt.  Limits: E * B * (B - 1) / 2 < 2^30 - 1.  *bad is set when an
  * element repeats a node (no lists then).
  * tm_group_count writes [distinct elements, entries, records] of every group
- * and sets *bad when a group exceeds the record format (use fewer rows); base
+ * and sets *bad when a group exceeds the limits above (use fewer rows); base
  * is the exclusive scan of the sizes, cnt[nnz] is scratch that tm_group_fill
  * consumes.  quads = 1: the records of scalar forms, 0: of elasticity blocks.
  * rows_per_group <= 64.

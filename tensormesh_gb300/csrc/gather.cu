@@ -72,6 +72,12 @@ extern "C" int tm_assemble_gather(const tm_gather_plan* plan, const tm_assemble_
     if (is_p1(args->element)) {
       if (!plan->order || !plan->base || !plan->gelem || !plan->gent || !plan->grec || plan->max_elems < 1)
         return TM_ERR_INVALID;
+      // what a group's records and its CTA hold
+      const bool blocks = args->form == TM_FORM_ELASTICITY;
+      const int64_t pairs = args->element == TM_TRI3 ? 3 : 6;
+      if (plan->rows_per_cta > kGroupRows || (blocks ? plan->max_entries > kBlockEntries || plan->max_elems > kBlockElems
+                                                     : plan->max_elems * pairs > kPairValues))
+        return TM_ERR_INVALID;
     } else if (!plan->ent || !plan->rec) {
       return TM_ERR_INVALID;
     }

@@ -34,6 +34,11 @@ constexpr uint32_t kEnd = 0x80000000u;    // record: last of its list
 constexpr uint32_t kFlip = 0x40000000u;   // record: local pair (a, b), a < b, has node a > node b
 constexpr uint32_t kIdx = 0x3fffffffu;    // record: element * pairs + pair
 constexpr int kWindow = 60;
+// groups of P1 rows
+constexpr int kGroupRows = 64;       // rows: six bits of an entry word
+constexpr int kBlockEntries = 512;   // entries of a group of blocks: one thread each (group_blocks)
+constexpr int kBlockElems = 2048;    // its elements: eleven bits of a record
+constexpr int kPairValues = 32767;   // elements times pairs of a scalar group: fifteen bits of a record
 
 struct Head {
   int S;              // common exponent of the pairs in the scratch

@@ -129,7 +129,6 @@ __global__ void node_sort_kernel(int64_t n_points, const int64_t* __restrict__ n
 //           node = b), bit 15 on the last record
 constexpr int kGroupThreads = 256;
 constexpr int kGroupInc = 4096;    // incidences of one group's rows
-constexpr int kGroupRows = 64;
 
 // Sorted distinct elements of group g in s_e[0, n); returns n, or -1 when the
 // group holds too many incidences.  s_off[k]: incidences before row k.
@@ -227,8 +226,9 @@ group_count_kernel(int rows_per_group, int n_points, int B, int quads, const int
   }
   __syncthreads();
   if (tid != 0) return;
-  const bool over = n < 0 || s_sum[0] > 65535 ||
-                    (quads ? (n * (B * (B - 1) / 2) > 32767 || s_sum[1] / 4 > 65535) : (n > 2048 || s_sum[1] > 65535));
+  const bool over = n < 0 || s_sum[0] > (quads ? 65535 : kBlockEntries) ||
+                    (quads ? (n * (B * (B - 1) / 2) > kPairValues || s_sum[1] / 4 > 65535)
+                           : (n > kBlockElems || s_sum[1] > 65535));
   if (over) atomicExch(bad, 1);
   sizes[3 * g] = over ? 0 : n;
   sizes[3 * g + 1] = over ? 0 : s_sum[0];

@@ -546,7 +546,7 @@ template <class T, int B> size_t group_rows_smem(const tm_gather_plan& p) {
 // nine double-float multiply-adds per record; 380 us at 64^3, where the patch
 // kernel, which forms all sixteen blocks of an element from staged values,
 // takes 1390 us.
-constexpr int kBlkGrpThreads = 512;
+constexpr int kBlkGrpThreads = kBlockEntries;
 
 template <class T, int D, bool kWide>
 TM_D void group_blocks(const tm_gather_plan& plan, const typename Sto<T>::S* __restrict__ vals,

@@ -436,9 +436,9 @@ class GatherPlan:
     # elements, 21 KB of staged values, so eight 128-thread CTAs share an SM:
     # 124 us at 80^3 against 136 us for 64 rows and 256 threads); as many rows
     # of blocks as have at most 512 entries, one for each thread of the CTA
+    # (tm_group_count refuses more)
     ROWS = {1: (32, 16, 8, 4, 2, 1), 2: (64, 56, 48, 40, 32, 24, 16, 8, 4, 2, 1),
             3: (34, 32, 30, 28, 26, 24, 22, 20, 16, 12, 8, 4, 2, 1)}
-    BLOCK_ENTRIES = 512
     SMEM_BYTES = 200 * 1024
 
     def __init__(self, elements: torch.Tensor, points: torch.Tensor, pattern: NodePattern):
@@ -551,7 +551,7 @@ class GatherPlan:
                 words = most[0] * (B * (B - 1) // 2 + 2) + most[1]    # float64 words, head-room included
             else:
                 words = max(most[0] * 14, most[1] * H * H)
-            if not most[3] and 8 * words <= self.SMEM_BYTES and (H == 1 or most[1] <= self.BLOCK_ENTRIES):
+            if not most[3] and 8 * words <= self.SMEM_BYTES:
                 break
         else:
             return None

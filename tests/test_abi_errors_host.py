@@ -90,3 +90,20 @@ def test_element_once_arrays_of_wrong_alignment_are_rejected(lib):
     plan, a = gather_call(element=_lib.TM_TRI3)
     plan.grec = FAKE + 4
     assert lib.tm_assemble_gather(plan, a, FAKE, 1 << 20, None) == INV
+
+
+def test_element_once_groups_beyond_their_limits_are_rejected(lib):
+    """A thread of the block kernel owns one entry, a record holds so many bits."""
+    def status(form, element=_lib.TM_TET4, **sizes):
+        plan, a = gather_call(element, form)
+        for k, v in sizes.items():
+            setattr(plan, k, v)
+        return lib.tm_assemble_gather(plan, a, FAKE, 1 << 20, None)
+
+    for element in (_lib.TM_TRI3, _lib.TM_TET4):
+        assert status(_lib.TM_FORM_ELASTICITY, element, max_entries=513) == INV
+        assert status(_lib.TM_FORM_ELASTICITY, element, max_elems=2049) == INV
+        for form in (_lib.TM_FORM_LAPLACE, _lib.TM_FORM_MASS, _lib.TM_FORM_ELASTICITY):
+            assert status(form, element, rows_per_cta=65) == INV
+    assert status(_lib.TM_FORM_LAPLACE, max_elems=32767 // 6 + 1) == INV
+    assert status(_lib.TM_FORM_MASS, _lib.TM_TRI3, max_elems=32767 // 3 + 1) == INV

@@ -419,3 +419,19 @@ def test_connectivity_at_an_odd_address(word):
         v = KappaLaplace(tg.assemble.topology_for(cells, x, "tetra"), x, 2)(xg, element_data={"kappa": k}).values
         got.append((v, *torch.autograd.grad(v.square().sum(), xg)))
     assert all(torch.equal(a, b) for a, b in zip(*got))
+
+
+# -- limits ------------------------------------------------------------------------
+def test_block_groups_of_too_many_entries_are_marked():
+    """34 rows of a regular mesh have about 510 entries, 64 of them about 960:
+    the count refuses what a CTA of 512 threads does not hold."""
+    mesh = tg.Mesh.gen_unit_cube(8, device=DEV)
+    topo = KappaLaplace.from_mesh(mesh).topology
+    g, pat = topo.gather, topo.pattern
+    for rows, quads, refused in ((64, 0, 1), (16, 0, 0), (64, 1, 0)):
+        sizes = torch.empty((-(-topo.n_points // rows), 3), dtype=torch.int32, device=DEV)
+        cnt, bad = torch.empty(pat.nnz, dtype=torch.int32, device=DEV), torch.empty(1, dtype=torch.int32, device=DEV)
+        tg._lib.call("tm_group_count", 4, topo.n_points, rows, quads, g.order.data_ptr(), g.nptr.data_ptr(),
+                     g.nrec.data_ptr(), pat.indptr.data_ptr(), pat.slots.data_ptr(), cnt.data_ptr(),
+                     sizes.data_ptr(), bad.data_ptr(), tg._lib.stream_handle(torch.device(DEV)))
+        assert int(bad) == refused
