@@ -109,7 +109,7 @@ def csr_diagonal(A) -> torch.Tensor:
 
 
 class PCGWorkspace:
-    """Device scratch for tm_pcg_jacobi, reused across solves of one size."""
+    """Device scratch of one tm_pcg_jacobi solve."""
 
     def __init__(self, n: int, nnz: int, dtype: torch.dtype, device):
         lib = _lib.load()
@@ -121,7 +121,7 @@ class PCGWorkspace:
 
 
 class SellWorkspace:
-    """Device scratch for tm_pcg_jacobi_sell (n rows, n_pad SELL-32 entries)."""
+    """Device scratch of one tm_pcg_jacobi_sell solve (n rows, n_pad SELL-32 entries)."""
 
     def __init__(self, n: int, n_pad: int, dtype: torch.dtype, device):
         lib = _lib.load()
@@ -130,22 +130,6 @@ class SellWorkspace:
         if self.nbytes < 0:
             raise _lib.TensorMeshCudaError("tm_pcg_sell_workspace_bytes", -self.nbytes)
         self.buf = torch.empty(self.nbytes, dtype=torch.uint8, device=device)
-
-
-_WS = {}
-
-
-def _cached(key, make):
-    ws = _WS.get(key)
-    if ws is None:
-        if len(_WS) > 4:
-            _WS.clear()
-        ws = _WS[key] = make()
-    return ws
-
-
-def workspace(n, nnz, dtype, device) -> PCGWorkspace:
-    return _cached(("csr", n, nnz, dtype, str(device)), lambda: PCGWorkspace(n, nnz, dtype, device))
 
 
 def sell_plan(indptr: torch.Tensor, indices: torch.Tensor):
@@ -182,7 +166,11 @@ def pcg_jacobi_raw(indptr, indices, values, b, x, rtol=1e-8, atol=0.0, maxiter=1
     double-float, whose ~48-bit products floor the attainable residual near
     cond(K) * 2^-48 -- each restart is one step of iterative refinement: the
     residual r = b - K x in the value type, a solve K d = r from zero to the
-    accuracy the remaining gap needs, and x += d."""
+    accuracy the remaining gap needs, and x += d.
+
+    The scratch (solver record, barrier words, vectors, matrix copy) is this
+    solve's own, from torch's allocator on the calling stream: solves of one
+    shape may run at the same time on several threads and streams."""
     n = b.shape[0]
     dev = values.device
     s = _lib.stream_handle(dev)
@@ -190,7 +178,7 @@ def pcg_jacobi_raw(indptr, indices, values, b, x, rtol=1e-8, atol=0.0, maxiter=1
     pipelined = LAYOUT == "sell-pipelined"
     if LAYOUT in ("sell", "sell-pipelined"):
         sp, n_pad, narrow = sell_plan(indptr, indices)
-        ws = _cached(("sell", n, n_pad, values.dtype, str(dev)), lambda: SellWorkspace(n, n_pad, values.dtype, dev))
+        ws = SellWorkspace(n, n_pad, values.dtype, dev)
         method = (_lib.TM_PCG_PIPELINED if pipelined else _lib.TM_PCG_STANDARD) | (_lib.TM_PCG_NARROW if narrow else 0)
 
         def launch(rhs, sol, rt, at, budget):
@@ -198,7 +186,7 @@ def pcg_jacobi_raw(indptr, indices, values, b, x, rtol=1e-8, atol=0.0, maxiter=1
                       sp.data_ptr(), n_pad, rhs.data_ptr(), sol.data_ptr(), rt, at, budget, method,
                       ws.buf.data_ptr(), ws.nbytes, s)
     else:
-        ws = workspace(n, int(values.shape[0]), values.dtype, dev)
+        ws = PCGWorkspace(n, int(values.shape[0]), values.dtype, dev)
 
         def launch(rhs, sol, rt, at, budget):
             _lib.call("tm_pcg_jacobi", code, n, indptr.data_ptr(), indices.data_ptr(), values.data_ptr(),

@@ -162,3 +162,46 @@ def test_bounded_grid_barrier_times_out_and_context_survives():
     K_ii, f_i = tg.Condenser(mesh.boundary_mask)(K, b)
     K_ii.solve(f_i, rtol=1e-10)
     assert K_ii.last_solve_info.status == 0 and K_ii.last_solve_info.residual <= 1e-10
+
+
+@pytest.mark.parametrize("layout", ["sell", "csr"])
+def test_two_threads_solve_systems_of_one_shape(layout, monkeypatch):
+    """Two threads, each on its own stream, solve different systems of the
+    same shape again and again: the bits of solves one after the other."""
+    import threading
+    from tensormesh_gb300 import solve as S
+
+    class Kappa(tg.ElementAssembler):
+        def forward(self, gradu, gradv, kappa):
+            return kappa * (gradu @ gradv)
+
+    monkeypatch.setattr(S, "LAYOUT", layout)
+    mesh = tg.Mesh.gen_unit_square(40, device=DEV, dtype=torch.float64)
+    asm, cond = Kappa.from_mesh(mesh, 1), tg.Condenser(mesh.boundary_mask)
+    b = tg.const_node_assembler(1.0).from_mesh(mesh, 1)(mesh.points)
+    g = torch.Generator(device=DEV).manual_seed(3)
+    systems = []
+    for _ in range(2):
+        k = torch.exp(torch.randn(mesh.n_elements, generator=g, device=DEV, dtype=torch.float64))
+        systems.append(cond(asm(mesh.points, element_data={"kappa": k}), b))
+    ref = [K.solve(f, rtol=1e-10) for K, f in systems]
+    torch.cuda.synchronize()
+    got, failed = [[], []], []
+
+    def work(i):
+        try:
+            with torch.cuda.stream(torch.cuda.Stream()):
+                for _ in range(30):
+                    got[i].append(systems[i][0].solve(systems[i][1], rtol=1e-10))
+                torch.cuda.current_stream().synchronize()
+        except Exception as e:  # reported by the main thread
+            failed.append(e)
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failed, failed
+    for i in range(2):
+        assert len(got[i]) == 30 and all(torch.equal(x, ref[i]) for x in got[i])
