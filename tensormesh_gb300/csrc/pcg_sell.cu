@@ -843,9 +843,12 @@ int sell_launch(int64_t n_slices, int64_t n_pad, SellLaunch& how) {
   for (int nb = 16; nb >= 8; nb /= 2) {
     const size_t bytes = resident_bytes<S, CT>(n_slices, n_pad, nb, optin, how.cap);
     auto kern = pcg_sell_hs_kernel<S, CT, kCluster>;
-    if (!bytes || cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, most) != cudaSuccess ||
-        cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
+    if (!bytes) continue;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, most) != cudaSuccess ||
+        cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
+      cudaGetLastError();   // a refusal rules this size out; the launch must not report it
       continue;
+    }
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(nb);
     cfg.blockDim = dim3(kSellThreads);
@@ -857,13 +860,15 @@ int sell_launch(int64_t n_slices, int64_t n_pad, SellLaunch& how) {
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
     int clusters = 0;
-    if (cudaOccupancyMaxActiveClusters(&clusters, kern, &cfg) != cudaSuccess || clusters < 1) continue;
+    if (cudaOccupancyMaxActiveClusters(&clusters, kern, &cfg) != cudaSuccess || clusters < 1) {
+      cudaGetLastError();
+      continue;
+    }
     how.mode = kCluster;
     how.nb = nb;
     how.bytes = bytes;
     return TM_OK;
   }
-  cudaGetLastError();   // a refused attribute or query above only rules the cluster out
   const int nb = (int)min((int64_t)sms, n_slices);
   const size_t bytes = nb > 0 ? resident_bytes<S, CT>(n_slices, n_pad, nb, optin, how.cap) : 0;
   if (bytes && cudaFuncSetAttribute(pcg_sell_hs_kernel<S, CT, kResident>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -873,6 +878,7 @@ int sell_launch(int64_t n_slices, int64_t n_pad, SellLaunch& how) {
     how.bytes = bytes;
     return TM_OK;
   }
+  cudaGetLastError();
   auto kern = pcg_sell_hs_kernel<S, CT, kGrid>;
   how.nb = sell_blocks(kern, n_slices);
   if (how.nb <= 0) return TM_OK;

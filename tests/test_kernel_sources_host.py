@@ -25,3 +25,13 @@ def test_clusters_meet_before_they_write_each_others_shared_memory():
     assert solve.index("cluster_barrier()") < solve.index("cluster_sum<")
     batch = body("batched.cu", "batched_assemble_pcg_kernel(BatchArgs A)")
     assert batch.index("cl.sync()") < batch.index("cluster_sum<")
+
+
+def test_a_refused_cluster_size_leaves_no_error_for_the_launch():
+    """A CUDA error stays until it is read.  Every refusal inside the search
+    for a cluster size reads it, so that a smaller size launches cleanly."""
+    search = body("pcg_sell.cu", "int sell_launch(int64_t n_slices")
+    loop = search[search.index("for (int nb = 16"):search.index("how.mode = kCluster")]
+    refusals = re.findall(r"if \(([^;{]*cuda[^;{]*)\) \{\s*cudaGetLastError\(\);\s*continue;\s*\}", loop)
+    calls = re.findall(r"cuda(?:FuncSetAttribute|OccupancyMaxActiveClusters)\(", loop)
+    assert len(calls) == 3 and sum(c.count("cudaSuccess") for c in refusals) == 3
