@@ -17,7 +17,8 @@
 // The scratch holds them as float pairs relative to a call-wide exponent S,
 // that of element 0, as long as |s - S| <= kWindow; an element outside the
 // window stores plain doubles instead, sets its bit in `wide` and raises
-// `head->any`, and the summing kernel then adds in native FP64.
+// `head->any`.  Where that is raised, every group of rows looks at its elements'
+// bits, and those that hold such an element add in native FP64 (loads: nodes).
 // An ill-conditioned element (the bound of the patch kernels) is computed in
 // native FP64 by the same thread or block.
 #pragma once

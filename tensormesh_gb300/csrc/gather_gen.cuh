@@ -433,8 +433,13 @@ sum_nodes_kernel(int64_t n, const int64_t* __restrict__ nptr, const uint32_t* __
   if (i >= n * H) return;
   if constexpr (sizeof(T) == 8) {
     if (head->any) {
-      sum_nodes<T, B, H, true>(i, nptr, nrec, diag, wide, head->S, out);
-      return;
+      const int64_t r = i / H;
+      bool any = false;
+      for (int64_t k = nptr[r]; k < nptr[r + 1]; ++k) any = any || wide_of(wide, nrec[k] / B);
+      if (any) {
+        sum_nodes<T, B, H, true>(i, nptr, nrec, diag, wide, head->S, out);
+        return;
+      }
     }
     sum_nodes<T, B, H, false>(i, nptr, nrec, diag, wide, head->S, out);
   } else {
@@ -448,6 +453,25 @@ sum_nodes_kernel(int64_t n, const int64_t* __restrict__ nptr, const uint32_t* __
 // them would not pay); the CTA's rows are consecutive, their sums staged for
 // the diagonal and a coalesced write.
 constexpr int kSumThreads = 256;
+
+// Whether an element of the CTA's rows stored plain doubles (read only when
+// some element of the call did; every thread of the CTA calls it).
+template <int B>
+TM_D bool rows_any_wide(const tm_gather_plan& plan, const uint32_t* __restrict__ wide) {
+  const int r0 = blockIdx.x * plan.rows_per_cta, r1 = min(plan.n_points, r0 + plan.rows_per_cta);
+  bool any = false;
+  for (int64_t t = plan.indptr[r0] + threadIdx.x; t < plan.indptr[r1]; t += blockDim.x) {
+    const uint32_t w = plan.ent[t];
+    if (w == kDiag) continue;   // a row's elements are all in its lists off the diagonal
+    const uint32_t* __restrict__ rec = plan.rec + (w & kIdx);
+    uint32_t r;
+    do {
+      r = *rec++;
+      any = any || wide_of(wide, (r & kIdx) / Pairs<B>::P);
+    } while (!(r & kEnd));
+  }
+  return __syncthreads_or(any);
+}
 
 template <class T, int B, bool kDiagList, bool kWide>
 TM_D void sum_rows(const tm_gather_plan& plan, const typename Sto<T>::S* __restrict__ vals,
@@ -529,7 +553,7 @@ sum_rows_kernel(tm_gather_plan plan, const typename Sto<T>::S* __restrict__ vals
   extern __shared__ __align__(16) unsigned char smem_raw[];
   auto* s_val = reinterpret_cast<typename Sto<T>::S*>(smem_raw);
   if constexpr (sizeof(T) == 8) {
-    if (head->any) {
+    if (head->any && rows_any_wide<B>(plan, wide)) {
       sum_rows<T, B, kDiagList, true>(plan, vals, diag, wide, head->S, out, s_val);
       return;
     }
@@ -627,7 +651,7 @@ sum_blocks_kernel(tm_gather_plan plan, const typename Sto<T>::S* __restrict__ va
   extern __shared__ __align__(16) unsigned char smem_raw[];
   auto* s_val = reinterpret_cast<typename Sto<T>::S*>(smem_raw);
   if constexpr (sizeof(T) == 8) {
-    if (head->any) {
+    if (head->any && rows_any_wide<B>(plan, wide)) {
       sum_blocks<T, D, B, true>(plan, vals, wide, head->S, lam, mu, out, s_val);
       return;
     }

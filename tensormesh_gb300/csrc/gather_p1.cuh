@@ -391,6 +391,16 @@ TM_D void group_wide(const int32_t* __restrict__ gelem, int ne, const uint32_t* 
   }
 }
 
+// Whether one of the group's elements stored plain doubles (read only when
+// some element of the call did; every thread of the CTA calls it).
+TM_D bool group_any_wide(const tm_gather_plan& plan, const uint32_t* __restrict__ wide) {
+  const int64_t e1 = plan.base[3 * (int64_t)blockIdx.x + 3];
+  bool any = false;
+  for (int64_t i = plan.base[3 * (int64_t)blockIdx.x] + threadIdx.x; i < e1; i += blockDim.x)
+    any = any || wide_of(wide, (uint32_t)plan.gelem[i]);
+  return __syncthreads_or(any);
+}
+
 // Sums of the scalar CSR entries of one group (one CTA).  The group's element
 // values are copied to shared memory in full lines; one thread per entry adds
 // its list, four records a load, and writes its value; four lanes per row
@@ -521,7 +531,7 @@ group_rows_kernel(tm_gather_plan plan, const typename Sto<T>::S* __restrict__ va
                   const uint32_t* __restrict__ wide, T* __restrict__ out) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   if constexpr (sizeof(T) == 8) {
-    if (head->any) {
+    if (head->any && group_any_wide(plan, wide)) {
       group_rows<T, B, kDiagList, true>(plan, vals, diag, wide, head->S, out, smem_raw);
       return;
     }
@@ -689,7 +699,7 @@ group_blocks_kernel(tm_gather_plan plan, const typename Sto<T>::S* __restrict__ 
                     const uint32_t* __restrict__ wide, double lam, double mu, T* __restrict__ out) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   if constexpr (sizeof(T) == 8) {
-    if (head->any) {
+    if (head->any && group_any_wide(plan, wide)) {
       group_blocks<T, D, true>(plan, vals, wide, head->S, lam, mu, out, smem_raw);
       return;
     }

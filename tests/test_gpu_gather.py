@@ -435,3 +435,45 @@ def test_block_groups_of_too_many_entries_are_marked():
                      g.nrec.data_ptr(), pat.indptr.data_ptr(), pat.slots.data_ptr(), cnt.data_ptr(),
                      sizes.data_ptr(), bad.data_ptr(), tg._lib.stream_handle(torch.device(DEV)))
         assert int(bad) == refused
+
+
+# -- elements outside the common exponent's window -----------------------------------
+@pytest.mark.parametrize("etype,n,forms", [("tetra", 8, ("laplace", "mass", "elasticity")),
+                                           ("triangle", 24, ("laplace", "mass", "elasticity")),
+                                           ("tetra10", 4, ("laplace", "mass", "elasticity")),
+                                           ("triangle6", 9, ("laplace",))])
+def test_a_far_coefficient_changes_its_own_surroundings_only(etype, n, forms):
+    """One element outside the window makes the rows near it add in native
+    FP64; the others keep the bits they have without it."""
+    base = tg.Mesh.gen_unit_square(n) if etype.startswith("tri") else tg.Mesh.gen_unit_cube(n)
+    mesh = (base.to_p2() if etype in ("tetra10", "triangle6") else base).to(DEV)
+    cells = mesh.cells[etype]
+    g = torch.Generator(device=DEV).manual_seed(n)
+    x = mesh.points + 0.1 / n * torch.rand(mesh.points.shape, generator=g, device=DEV, dtype=torch.float64)
+    k = torch.exp(torch.randn(cells.shape[0], generator=g, device=DEV, dtype=torch.float64))
+    far = k.clone()
+    far[-1] *= 2.0 ** 70
+    near = cells[-1].long()
+    for form in forms:
+        asm = FORMS[form].from_mesh(mesh, 2)
+        a, b = (asm(x, element_data={"kappa": c}) for c in (k, far))
+        H = a.shape[0] // x.shape[0]
+        plan = asm.topology.gather
+        group = torch.arange(x.shape[0], device=DEV)
+        if plan.p1:
+            group[plan.order.long()] = group.clone()
+        group //= plan.struct(H).rows_per_cta
+        rows = ~torch.isin(group, group[near]).repeat_interleave(H)[a.row]
+        assert int(rows.sum()) > 500 and torch.equal(a.values[rows], b.values[rows])
+
+    class PointLoad(tg.NodeAssembler):
+        def forward(self, v, f):
+            return v * f
+
+    load, f = PointLoad.from_mesh(mesh, 2), torch.rand(x.shape[0], generator=g, device=DEV, dtype=torch.float64)
+    f2 = f.clone()
+    f2[cells[-1, 0].long()] *= 2.0 ** 70
+    a, b = (load(x, point_data={"f": c}) for c in (f, f2))
+    touched = torch.isin(cells, cells[-1, 0]).any(1)
+    away = ~torch.isin(torch.arange(x.shape[0], device=DEV), cells[touched])
+    assert int(away.sum()) > 100 and torch.equal(a[away], b[away])
