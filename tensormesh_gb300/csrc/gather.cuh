@@ -20,7 +20,7 @@
 // `head->any`.  Where that is raised, every group of rows looks at its elements'
 // bits, and those that hold such an element add in native FP64 (loads: nodes).
 // An ill-conditioned element (the bound of the patch kernels) is computed in
-// native FP64 by the same thread or block.
+// native FP64 by the same thread or block, and kept as plain doubles too.
 #pragma once
 #include "p1tet_fast.cuh"
 #include <climits>

@@ -187,8 +187,8 @@ TM_D bool gen_pass(const tm_assemble_args& args, int64_t e0, int ne, double* s_c
     if constexpr (!kPairsT) {
       return tm_scale_pow2(v, sexp);
     } else {
-      if (sexp == INT_MIN) return pair_of(v);
       if constexpr (std::is_same<A, double>::value) return bits_of(tm_scale_pow2(v, sexp));
+      else if (sexp == INT_MIN) return pair_of(v);
       else return bits_of(tm_scale_pow2(tm_to_double(df64{v.h, v.l}), sexp));
     }
   };
@@ -367,8 +367,16 @@ gen_element_kernel(int64_t n_el, const int32_t* __restrict__ el, tm_assemble_arg
   if (gen_pass<EL, FORM, H, T, A, kPairsT>(args, e0, ne, s_cq, words, s_v, s_emax, s_cexp, s_sexp, s_r, vals, diag))
     return;
   if constexpr (kPairsT) {
-    if (tid < kGenEl && s_r[tid] == INT_MIN)
-      s_r[tid] = s_sexp[tid] == INT_MIN ? elem_exp(s_emax[tid], s_cexp[tid], G::power) - head->S : 0;
+    // the CTA's elements in native FP64, kept as plain doubles (a flat
+    // element's values leave float's range)
+    if (tid < kGenEl) {
+      s_sexp[tid] = elem_exp(s_emax[tid], s_cexp[tid], G::power);
+      s_r[tid] = 0;
+      if (tid == 0) {
+        wide_bits[blockIdx.x] = 0xffffffffu >> (kGenEl - ne);
+        atomicOr(&head->any, 1u);
+      }
+    }
     __syncthreads();
     gen_pass<EL, FORM, H, T, double, false>(args, e0, ne, s_cq, words, s_v, s_emax, s_cexp, s_sexp, s_r, vals, diag);
   }

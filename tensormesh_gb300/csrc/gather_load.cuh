@@ -115,7 +115,7 @@ p1_load_kernel(int64_t n_el, const int32_t* __restrict__ el, tm_assemble_args ar
     const bool ok = ed.ok() && ec != 2047 && (ec == 0 || ec > 100);
     const int em = ok ? ed.emax : 1023, ecn = ok && ec ? ec : 1023;
     const int s_exp = elem_exp(em, ecn, D), r = ec == 0 ? 0 : s_exp - head->S;
-    const bool wide = r > kWindow || r < -kWindow;
+    bool wide = r > kWindow || r < -kWindow;
     A d[D][D], adet, t[NV];
 #pragma unroll
     for (int k = 0; k < D; ++k)
@@ -132,19 +132,18 @@ p1_load_kernel(int64_t n_el, const int32_t* __restrict__ el, tm_assemble_args ar
         so[i] = wide ? bits_of(tm_scale_pow2(tm_to_double(df64{x.h, x.l}), s_exp)) : pair_of(x);
       }
     } else {
-      // ill-conditioned, degenerate or non-finite: the element in native FP64
+      // ill-conditioned, degenerate or non-finite: the element in native FP64,
+      // kept as plain doubles (a flat element's values leave float's range)
+      wide = true;
       double dd[D][D], vol, tn[NV];
 #pragma unroll
       for (int k = 0; k < D; ++k)
 #pragma unroll
         for (int j = 0; j < D; ++j) dd[k][j] = tm_scale_pow2(ed.d[k][j], 1023 - em);
       simplex_volume<double, D>(dd, vol);
-      sums(0.0, [&](double c) { return tm_scale_pow2(c, 1023 - ecn + (wide ? 0 : r)); }, [&](int i) { return N[i]; }, tn);
+      sums(0.0, [&](double c) { return tm_scale_pow2(c, 1023 - ecn); }, [&](int i) { return N[i]; }, tn);
 #pragma unroll
-      for (int i = 0; i < NV; ++i) {
-        const double x = tn[i] * vol;
-        so[i] = wide ? bits_of(tm_scale_pow2(x, s_exp)) : pair_of(x);
-      }
+      for (int i = 0; i < NV; ++i) so[i] = bits_of(tm_scale_pow2(tn[i] * vol, s_exp));
     }
     const unsigned bits = __ballot_sync(0xffffffffu, wide && e_raw < n_el);
     if (lane == 0 && e_raw < n_el) {

@@ -197,7 +197,8 @@ p1_element_kernel(int64_t n_el, const int32_t* __restrict__ el, tm_assemble_args
   if constexpr (kPairs) {
     const double c = p1_coef<NB>(args, e, v, head->wsum);
     const int ec = dexp(c);
-    int s_exp = elem_exp(ed.emax, ec, kPower), r = s_exp - head->S;
+    int s_exp = elem_exp(ed.emax, ec, kPower);
+    int r = s_exp - head->S;
     if (ec == 0) r = 0;  // zero values (a subnormal coefficient takes the native path)
     wide = r > kWindow || r < -kWindow;
     const float p2 = tm_pow2f(wide ? 0 : r);
@@ -209,34 +210,30 @@ p1_element_kernel(int64_t n_el, const int32_t* __restrict__ el, tm_assemble_args
     const A cw = l2_mul(Ar<L2>::scale2(l2_scaled(c, ec ? ec : 1023), p2), L2{head->w.x, head->w.y});
     const bool good = p1_element<A, D, kElast>(d, cw, out) && ed.ok() && ec != 2047 &&
                       (ec != 0 || (__double_as_longlong(c) << 1) == 0);
+    S* so = s_out[warp] + lane * NV;
+    // plain doubles in real units; elasticity's cofactors stay O(1)
+    auto plain = [&](double x, int i) { return bits_of(kElast && i < NV - 1 ? x : tm_scale_pow2(x, s_exp)); };
     if (!good) {
-      // ill-conditioned, degenerate or non-finite: the element in native FP64
+      // ill-conditioned, degenerate or non-finite: the element in native FP64,
+      // kept as plain doubles (a flat element's values leave float's range)
       const int em = ed.ok() ? ed.emax : 1023;
       const int ecn = ec > 0 && ec < 2047 ? ec : 1023;
       s_exp = elem_exp(em, ecn, kPower);
-      r = s_exp - head->S;
-      if ((__double_as_longlong(c) << 1) == 0) r = 0;
-      wide = r > kWindow || r < -kWindow;
+      wide = true;
       double dd[D][D], on[NV];
 #pragma unroll
       for (int k = 0; k < D; ++k)
 #pragma unroll
         for (int j = 0; j < D; ++j) dd[k][j] = tm_scale_pow2(ed.d[k][j], 1023 - em);
-      p1_element<double, D, kElast>(dd, tm_scale_pow2(c, 1023 - ecn + (wide ? 0 : r)) * head->wsum, on);
+      p1_element<double, D, kElast>(dd, tm_scale_pow2(c, 1023 - ecn) * head->wsum, on);
 #pragma unroll
-      for (int i = 0; i < NV; ++i) out[i] = l2_from(tm_from_double(on[i]));
-    }
-    S* so = s_out[warp] + lane * NV;
-    if (!wide) {
+      for (int i = 0; i < NV; ++i) so[i] = plain(on[i], i);
+    } else if (!wide) {
 #pragma unroll
       for (int i = 0; i < NV; ++i) so[i] = make_float2(out[i].h, out[i].l);
     } else {
-      // elasticity keeps the O(1) cofactors as pairs: only s leaves the window
 #pragma unroll
-      for (int i = 0; i < NV; ++i) {
-        if (kElast && i < NV - 1) so[i] = make_float2(out[i].h, out[i].l);
-        else so[i] = bits_of(tm_scale_pow2(tm_to_double(df64{out[i].h, out[i].l}), s_exp));
-      }
+      for (int i = 0; i < NV; ++i) so[i] = plain(tm_to_double(df64{out[i].h, out[i].l}), i);
     }
     const unsigned bits = __ballot_sync(0xffffffffu, wide && e_raw < n_el);
     if (lane == 0 && e_raw < n_el) {
@@ -592,15 +589,23 @@ TM_D void group_blocks(const tm_gather_plan& plan, const typename Sto<T>::S* __r
   if constexpr (kWide) group_wide(gelem, ne, wide, s_wide, kBlkGrpThreads);
   cp_async_wait();
   __syncthreads();
+  auto wide_elem = [&](unsigned l) { return kWide && ((s_wide[l >> 5] >> (l & 31)) & 1u); };
   // C_0 = -(C_1 + .. + C_D), once per element
   for (int i = tid; i < ne * D; i += kBlkGrpThreads) {
     const int l = i / D, j = i - l * D;
     St* v = s_val + (size_t)l * kStride + j;
     if constexpr (sizeof(T) == 8) {
-      L2 t{v[D].x, v[D].y};
+      if (wide_elem(l)) {
+        double t = double_of(v[D]);
 #pragma unroll
-      for (int k = 2; k <= D; ++k) t = l2_add(t, L2{v[k * D].x, v[k * D].y});
-      v[0] = make_float2(-t.h, -t.l);
+        for (int k = 2; k <= D; ++k) t += double_of(v[k * D]);
+        v[0] = bits_of(-t);
+      } else {
+        L2 t{v[D].x, v[D].y};
+#pragma unroll
+        for (int k = 2; k <= D; ++k) t = l2_add(t, L2{v[k * D].x, v[k * D].y});
+        v[0] = make_float2(-t.h, -t.l);
+      }
     } else {
       float t = v[D];
 #pragma unroll
@@ -609,8 +614,8 @@ TM_D void group_blocks(const tm_gather_plan& plan, const typename Sto<T>::S* __r
     }
   }
   __syncthreads();
-  auto cof = [](const St x) -> A {
-    if constexpr (kWide) return tm_to_double(df64{x.x, x.y});
+  auto cof = [](const St x, bool we) -> A {
+    if constexpr (kWide) return we ? double_of(x) : tm_to_double(df64{x.x, x.y});
     else return M::get(x);
   };
   A acc[D][D];
@@ -624,13 +629,14 @@ TM_D void group_blocks(const tm_gather_plan& plan, const typename Sto<T>::S* __r
       const unsigned l = (r >> 4) & 0x7ffu, a = (r >> 2) & 3u, b = r & 3u;
       if (!last) r = *++rec;
       const St* v = s_val + l * kStride;
+      const bool we = wide_elem(l);
       A cb[D];
 #pragma unroll
-      for (int d = 0; d < D; ++d) cb[d] = cof(v[b * D + d]);
-      const A s = M::ld(v[B * D], kWide && ((s_wide[l >> 5] >> (l & 31)) & 1u), S);
+      for (int d = 0; d < D; ++d) cb[d] = cof(v[b * D + d], we);
+      const A s = M::ld(v[B * D], we, S);
 #pragma unroll
       for (int i = 0; i < D; ++i) {
-        const A si = Pa::mul(s, cof(v[a * D + i]));
+        const A si = Pa::mul(s, cof(v[a * D + i], we));
 #pragma unroll
         for (int j = 0; j < D; ++j) acc[i][j] = Pa::add(acc[i][j], Pa::mul(si, cb[j]));
       }

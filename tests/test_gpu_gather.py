@@ -477,3 +477,135 @@ def test_a_far_coefficient_changes_its_own_surroundings_only(etype, n, forms):
     touched = torch.isin(cells, cells[-1, 0]).any(1)
     away = ~torch.isin(torch.arange(x.shape[0], device=DEV), cells[touched])
     assert int(away.sum()) > 100 and torch.equal(a[away], b[away])
+
+
+# -- flat elements: native FP64, kept as doubles -----------------------------------------
+FLAT = {"triangle": [[0, 0], [1, 0], [0.25, 1]], "tetra": [[0, 0, 0], [1, 0, 0], [0.5, 1, 0], [0.25, 0.25, 1]]}
+
+
+def flat_mesh(etype, heights):
+    """Disjoint elements of the given heights (their last coordinate's factor),
+    every coordinate and edge a short dyadic number."""
+    corners = np.array(FLAT["triangle" if etype.startswith("tri") else "tetra"])
+    pts, el = [], []
+    for i, h in enumerate(heights):
+        x = corners * np.array([1.0] * (corners.shape[1] - 1) + [h])
+        x[:, 0] += 4.0 * i
+        pts.append(x)
+        el.append(np.arange(len(x)) + i * len(x))
+    mesh = tg.Mesh(points=torch.tensor(np.concatenate(pts)),
+                   cells={"triangle" if corners.shape[1] == 2 else "tetra": torch.tensor(np.array(el))})
+    mesh = mesh.to_p2() if etype in ("triangle6", "tetra10") else mesh
+    return mesh.points.numpy(), mesh.cells[etype].numpy()
+
+
+def longdouble_elements(pts, el, etype, form, q, coef, lam=0.0, mu=0.0):
+    """Element matrices (load: vectors) in extended precision from the double
+    tables, weights and coefficients the kernels are given."""
+    L = np.longdouble
+    t = tg.element.kernel_tables(etype, q, torch.device("cpu")).double().numpy().astype(L)
+    Q, B, D = tg.element.n_quadrature(etype, q), el.shape[1], pts.shape[1]
+    w, N, dN = t[:Q], t[Q:Q + Q * B].reshape(Q, B), t[Q + Q * B:Q + Q * B + Q * B * D].reshape(Q, B, D)
+    x = (pts[el] - pts[el[:, :1]]).astype(L)
+    total = 0
+    for k in range(Q):
+        J = np.einsum("bi,ebj->eij", dN[k], x)
+        if D == 2:
+            adj = np.stack([np.stack([J[:, 1, 1], -J[:, 0, 1]], 1), np.stack([-J[:, 1, 0], J[:, 0, 0]], 1)], 1)
+        else:
+            adj = np.stack([np.cross(J[:, 1], J[:, 2]), np.cross(J[:, 2], J[:, 0]), np.cross(J[:, 0], J[:, 1])], 2)
+        det = (J[:, 0] * adj[:, :, 0]).sum(1)
+        g = np.einsum("bi,eji->ebj", dN[k], adj)
+        s, v = coef.astype(L) * w[k] / abs(det), coef.astype(L) * w[k] * abs(det)
+        if form == "load":
+            total = total + v[:, None] * N[k]
+        elif form == "mass":
+            total = total + v[:, None, None] * (N[k][:, None] * N[k])
+        elif form == "laplace":
+            total = total + s[:, None, None] * np.einsum("eaj,ebj->eab", g, g)
+        else:
+            blk = L(lam) * np.einsum("eai,ebj->eaibj", g, g) + L(mu) * np.einsum("eaj,ebi->eaibj", g, g)
+            blk = blk + L(mu) * np.einsum("eab,ij->eaibj", np.einsum("eaj,ebj->eab", g, g), np.eye(D))
+            total = total + s[:, None, None, None, None] * blk
+    return total
+
+
+def element_values(pts, el, etype, form, q, coef):
+    """(values [E, ...] of the disjoint elements as assembled, lam, mu)."""
+    mesh = tg.Mesh(points=torch.tensor(pts, device=DEV), cells={etype: torch.tensor(el, device=DEV)})
+    E, B, D = el.shape[0], el.shape[1], pts.shape[1]
+    c = torch.tensor(coef, device=DEV)
+    if form == "load":
+        class PointLoad(tg.NodeAssembler):
+            def forward(self, v, f):
+                return v * f
+
+        nodal = torch.zeros(pts.shape[0], dtype=torch.float64, device=DEV)
+        nodal[mesh.cells[etype].long()] = c[:, None].expand(E, B)
+        out = PointLoad.from_mesh(mesh, q)(mesh.points, point_data={"f": nodal})
+        return out.cpu().numpy()[el], 0.0, 0.0
+    asm = FORMS[form].from_mesh(mesh, q)
+    K = asm(mesh.points, element_data={"kappa": c})
+    f = next(iter(asm._form_cache.values()))
+    H = D if form == "elasticity" else 1
+    dense = torch.zeros(E, B * H, B * H, dtype=torch.float64, device=DEV)
+    where = torch.empty(pts.shape[0], 2, dtype=torch.int64, device=DEV)
+    where[mesh.cells[etype].long()] = torch.stack(torch.meshgrid(torch.arange(E, device=DEV), torch.arange(
+        B, device=DEV), indexing="ij"), 2)
+    r, s = where[K.row // H], where[K.col // H]
+    dense[r[:, 0], r[:, 1] * H + K.row % H, s[:, 1] * H + K.col % H] = K.values
+    dense = dense.cpu().numpy()
+    return (dense.reshape(E, B, D, B, D) if H > 1 else dense), f.lam, f.mu
+
+
+@pytest.mark.parametrize("etype,form", [("triangle", "laplace"), ("triangle", "elasticity"), ("tetra", "laplace"),
+                                        ("tetra", "elasticity"), ("tetra", "mass"), ("tetra", "load"),
+                                        ("tetra10", "laplace"), ("tetra10", "elasticity")])
+def test_flat_elements_keep_the_bits_of_fp64(etype, form):
+    """Flat elements of dyadic shape (heights 2^-8 .. 2^-30: all of them past
+    the double-float bound): cofactors, determinants and their products are
+    exact in FP64, which leaves a handful of roundings: eight units of 2^-53 of
+    an element's largest entry (the order-1 tables of a tetrahedron are exact
+    but for the weight)."""
+    h = 2.0 ** -np.linspace(8, 30, 40).round()
+    pts, el = flat_mesh(etype, h)
+    coef = np.exp(np.random.default_rng(4).normal(size=len(h)))
+    got, lam, mu = element_values(pts, el, etype, form, 1, coef)
+    ref = longdouble_elements(pts, el, etype, form, 1, coef, lam, mu)
+    big = np.abs(ref).reshape(len(h), -1).max(1).reshape([-1] + [1] * (ref.ndim - 1))
+    assert float((np.abs(got - ref) / big).max()) <= 8 * 2.0 ** -53
+
+
+@pytest.mark.parametrize("etype", ["triangle", "triangle6", "tetra", "tetra10"])
+@pytest.mark.parametrize("form", ["laplace", "elasticity", "mass", "load"])
+def test_values_of_flat_elements_outside_floats_range(etype, form):
+    """Stiffness of heights near 1e-27 with large coefficients (values past
+    1e38), mass and loads of heights near 1e-51 (below 1e-45): finite, and
+    within 1e-12 of the element's largest entry.  The first element is regular
+    and sets the common exponent."""
+    stiff = form in ("laplace", "elasticity")
+    h = np.array([1.0] + [2.0 ** -(90 if stiff else 170)] * 5)
+    pts, el = flat_mesh(etype, h)
+    coef = np.array([1.0] + [2.0 ** (59 if stiff else 0) * 1.1] * 5)
+    got, lam, mu = element_values(pts, el, etype, form, 2, coef)
+    ref = longdouble_elements(pts, el, etype, form, 2, coef, lam, mu)
+    big = np.abs(ref).reshape(len(h), -1).max(1).reshape([-1] + [1] * (ref.ndim - 1))
+    assert np.isfinite(got).all() and float((np.abs(got - ref) / big).max()) <= 1e-12
+
+
+@pytest.mark.parametrize("etype", ["triangle", "tetra"])
+@pytest.mark.parametrize("form", ["laplace", "elasticity"])
+@pytest.mark.parametrize("height", [20.0, 200.0, 3e5])
+def test_slivers_of_p1_matrices(etype, form, height):
+    """Fans of needles, most of them past the double-float bound, that share
+    their rows: the element kernel's native branch."""
+    ring = 30
+    t = np.arange(ring) * 2 * np.pi / ring
+    if etype == "tetra":
+        pts = np.concatenate([[[0.0, 0.0, -height], [0.0, 0.0, height]],
+                              np.stack([np.cos(t), np.sin(t), 0.1 * np.sin(3 * t)], 1)])
+        el = np.array([[0, 2 + k, 2 + (k + 1) % ring, 1] for k in range(ring)], dtype=np.int64)
+    else:
+        pts = np.concatenate([[[0.0, height]], np.stack([np.cos(t), np.sin(t)], 1)])
+        el = np.array([[0, 1 + k, 1 + (k + 1) % ring] for k in range(ring)], dtype=np.int64)
+    check(pts, el, etype, form, np.exp(np.random.default_rng(ring).normal(size=ring)))
