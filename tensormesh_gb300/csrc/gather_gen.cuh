@@ -35,13 +35,15 @@ struct Gen {
   static constexpr int off = kLoad ? 0 : (FORM == TM_FORM_ELASTICITY ? P * D * D : P);   // values per element
   static constexpr int diag = kLoad ? B * H : (kMass ? B : 0);
   static constexpr int stage = FORM == TM_FORM_ELASTICITY ? 0 : off + diag;
+  // a point's table: N_a, or for mass matrices N_a N_b of every pair and node
+  static constexpr int NT = kMass ? P + B : B;
 };
 
 // Shared-memory words (of the storage type) of one CTA.
 template <int EL, int FORM, int H>
 constexpr size_t gen_words(int Q) {
   using G = Gen<EL, FORM, H>;
-  return kMaxQuad * (G::B + G::B * G::D) + (size_t)(G::B - 1) * G::D * kGenEl +
+  return kMaxQuad * (G::NT + G::B * G::D) + (size_t)(G::B - 1) * G::D * kGenEl +
          (G::kStiff ? (size_t)Q * G::B * G::D * kGenEl : 0) + (size_t)Q * G::HC * kGenEl + (size_t)kGenEl * G::stage;
 }
 template <int EL, int FORM, int H, class T>
@@ -56,6 +58,18 @@ template <class A> struct Word;
 template <> struct Word<L2> { using S = float2; };
 template <> struct Word<double> { using S = double; };
 template <> struct Word<float> { using S = float; };
+
+// Nodes of a stored value: the pairs a < b, then the nodes themselves.
+template <int B>
+TM_D void pair_of_value(int i, int& a, int& b) {
+  if (i >= Pairs<B>::P) {
+    a = b = i - Pairs<B>::P;
+    return;
+  }
+  a = 0;
+  while (i >= B - 1 - a) i -= B - 1 - a, ++a;
+  b = a + 1 + i;
+}
 
 // Phases 1 and 2 in arithmetic A.  Returns false on every thread when an
 // element needs native FP64.
@@ -72,12 +86,23 @@ TM_D bool gen_pass(const tm_assemble_args& args, int64_t e0, int ne, double* s_c
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int Q = args.n_quad;
   W* s_N = reinterpret_cast<W*>(words);
-  W* s_dN = s_N + kMaxQuad * B;
+  W* s_dN = s_N + kMaxQuad * G::NT;
   W* s_X = s_dN + kMaxQuad * B * D;               // [(B - 1) D][32]
   W* s_G = s_X + (B - 1) * D * kGenEl;            // [Q][B D][32]
   W* s_s = s_G + (G::kStiff ? Q * B * D * kGenEl : 0);  // [Q][HC][32]
   St* s_out = reinterpret_cast<St*>(s_s + Q * HC * kGenEl);   // [32][off + diag]
-  for (int i = tid; i < Q * B; i += kGenThreads) s_N[i] = Pa::st(Pa::in(args.tables[Q + i]));
+  if constexpr (G::kMass) {
+    // products in double: formed from pairs their rounding was the same for
+    // every element, and so did not average out
+    for (int i = tid; i < Q * G::NT; i += kGenThreads) {
+      const int q = i / G::NT;
+      int a, b;
+      pair_of_value<B>(i - q * G::NT, a, b);
+      s_N[i] = Pa::st(Pa::in(args.tables[Q + q * B + a] * args.tables[Q + q * B + b]));
+    }
+  } else {
+    for (int i = tid; i < Q * B; i += kGenThreads) s_N[i] = Pa::st(Pa::in(args.tables[Q + i]));
+  }
   for (int i = tid; i < Q * B * D; i += kGenThreads) s_dN[i] = Pa::st(Pa::in(args.tables[Q + Q * B + i]));
   const T* __restrict__ pts = static_cast<const T*>(args.points);
   for (int i = tid; i < (B - 1) * kGenEl; i += kGenThreads) {
@@ -201,26 +226,15 @@ TM_D bool gen_pass(const tm_assemble_args& args, int64_t e0, int ne, double* s_c
       s_out[lane * G::stage + i] = put(t);
     }
   } else if constexpr (FORM == TM_FORM_MASS) {
-    for (int i = warp; i < G::P + B; i += kGenThreads / 32) {
-      int a, b;
-      if (i < G::P) {
-        a = 0;
-        b = i;
-        while (b >= B - 1 - a) b -= B - 1 - a, ++a;
-        b += a + 1;
-      } else {
-        a = b = i - G::P;
-      }
+    for (int i = warp; i < G::NT; i += kGenThreads / 32) {
       A t = Pa::zero();
-      for (int q = 0; q < Q; ++q)
-        t = Pa::add(t, Pa::mul(s_of(q, 0), Pa::mul(Pa::ld(s_N[q * B + a]), Pa::ld(s_N[q * B + b]))));
+      for (int q = 0; q < Q; ++q) t = Pa::add(t, Pa::mul(s_of(q, 0), Pa::ld(s_N[q * G::NT + i])));
       s_out[lane * G::stage + i] = put(t);
     }
   } else {
     for (int i = warp; i < G::P; i += kGenThreads / 32) {
-      int a = 0, b = i;
-      while (b >= B - 1 - a) b -= B - 1 - a, ++a;
-      b += a + 1;
+      int a, b;
+      pair_of_value<B>(i, a, b);
       if constexpr (FORM == TM_FORM_LAPLACE) {
         A t = Pa::zero();
         for (int q = 0; q < Q; ++q) {

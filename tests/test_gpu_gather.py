@@ -609,3 +609,61 @@ def test_slivers_of_p1_matrices(etype, form, height):
         pts = np.concatenate([[[0.0, height]], np.stack([np.cos(t), np.sin(t)], 1)])
         el = np.array([[0, 1 + k, 1 + (k + 1) % ring] for k in range(ring)], dtype=np.int64)
     check(pts, el, etype, form, np.exp(np.random.default_rng(ring).normal(size=ring)))
+
+
+# -- accuracy against the patch kernels ---------------------------------------------------
+def exact_values(x, cells, etype, form, q, k, asm):
+    """CSR values in float64 by plain torch (form's Lame constants as given)."""
+    w, N = tg.element.shape_values(etype, q)
+    xi = tg.element.quadrature(etype, q)[1]
+    dN = torch.tensor(tg.element.shape_tables(etype, xi)[1], device=x.device)
+    N, D = torch.tensor(N, device=x.device), x.shape[1]
+    X, total = x[cells], 0
+    for i in range(len(w)):
+        J = torch.einsum("bi,ebj->eij", dN[i], X - X[:, :1])
+        g, det = torch.einsum("bi,eji->ebj", dN[i], torch.linalg.inv(J)), torch.linalg.det(J).abs()
+        cw = (k * float(w[i]) * det)[:, None, None]
+        if form == "mass":
+            total = total + cw * (N[i][:, None] * N[i])
+        elif form == "laplace":
+            total = total + cw * (g @ g.transpose(1, 2))
+        else:
+            f = next(iter(asm._form_cache.values()))
+            blk = f.lam * torch.einsum("eai,ebj->eaibj", g, g) + f.mu * torch.einsum("eaj,ebi->eaibj", g, g)
+            blk = blk + f.mu * torch.einsum("eab,ij->eaibj", g @ g.transpose(1, 2), torch.eye(D, device=x.device).double())
+            total = total + cw[..., None, None] * blk
+    n = x.shape[0]
+    if form == "elasticity":
+        cells = (cells[:, :, None] * D + torch.arange(D, device=x.device)).reshape(cells.shape[0], -1)
+        total, n = total.reshape(cells.shape[0], cells.shape[1], -1), n * D
+    uniq, inv = torch.unique((cells[:, :, None] * n + cells[:, None, :]).reshape(-1), return_inverse=True)
+    return torch.zeros(uniq.shape[0], dtype=x.dtype, device=x.device).index_add(0, inv, total.reshape(-1))
+
+
+def both_routes(etype, n, form, q, monkeypatch):
+    """Relative 2-norm errors of the float64 values, (all, diagonal), of the
+    element-once and of the patch kernels, over four jittered meshes."""
+    base = (tg.Mesh.gen_unit_square if etype.startswith("tri") else tg.Mesh.gen_unit_cube)(n)
+    mesh = (base.to_p2() if etype in ("triangle6", "tetra10") else base).to(DEV)
+    cells, err = mesh.cells[etype].long(), np.zeros((2, 2))
+    move = 0.05 if etype in ("triangle6", "tetra10") else 0.2
+    for seed in range(4):
+        g = torch.Generator(device=DEV).manual_seed(seed)
+        x = mesh.points + move / n * (2 * torch.rand(mesh.points.shape, generator=g, device=DEV, dtype=torch.float64) - 1)
+        k = torch.exp(torch.randn(cells.shape[0], generator=g, device=DEV, dtype=torch.float64))
+        asm = FORMS[form].from_mesh(mesh, q)
+        for route, least in enumerate((0, 1 << 40)):
+            monkeypatch.setattr("tensormesh_gb300.assemble._GATHER_MIN_ELEMENTS", {etype: least})
+            assert asm.topology.element_once == (least == 0)
+            K = asm(x, element_data={"kappa": k})
+            ref = exact_values(x, cells, etype, form, q, k, asm)
+            d, on = K.values - ref, K.row == K.col
+            err[route] += float(d.norm() / ref.norm()), float(d[on].norm() / ref[on].norm())
+    return err
+
+
+@pytest.mark.parametrize("etype,n", [("triangle", 60), ("tetra", 12), ("triangle6", 24), ("tetra10", 6)])
+@pytest.mark.parametrize("q", [1, 2])
+def test_mass_matrices_are_as_accurate_as_the_patch_kernels(etype, n, q, monkeypatch):
+    once, patch = both_routes(etype, n, "mass", q, monkeypatch)
+    assert (once <= patch).all(), (once, patch)
