@@ -667,3 +667,11 @@ def both_routes(etype, n, form, q, monkeypatch):
 def test_mass_matrices_are_as_accurate_as_the_patch_kernels(etype, n, q, monkeypatch):
     once, patch = both_routes(etype, n, "mass", q, monkeypatch)
     assert (once <= patch).all(), (once, patch)
+
+
+@pytest.mark.parametrize("etype,n", [("triangle", 60), ("tetra", 12)])
+@pytest.mark.parametrize("form", ["laplace", "elasticity"])
+@pytest.mark.parametrize("q", [1, 2])
+def test_p1_stiffness_is_as_accurate_as_the_patch_kernels(etype, n, form, q, monkeypatch):
+    once, patch = both_routes(etype, n, form, q, monkeypatch)
+    assert (once <= patch).all(), (once, patch)
