@@ -675,3 +675,11 @@ def test_mass_matrices_are_as_accurate_as_the_patch_kernels(etype, n, q, monkeyp
 def test_p1_stiffness_is_as_accurate_as_the_patch_kernels(etype, n, form, q, monkeypatch):
     once, patch = both_routes(etype, n, form, q, monkeypatch)
     assert (once <= patch).all(), (once, patch)
+
+
+@pytest.mark.parametrize("etype,n", [("triangle6", 24), ("tetra10", 6)])
+@pytest.mark.parametrize("form", ["laplace", "elasticity"])
+@pytest.mark.parametrize("q", [1, 2, 3])
+def test_p2_stiffness_is_as_accurate_as_the_patch_kernels(etype, n, form, q, monkeypatch):
+    once, patch = both_routes(etype, n, form, q, monkeypatch)
+    assert (once <= patch).all(), (once, patch)
