@@ -181,3 +181,60 @@ def test_clusters_with_ctas_that_own_no_rows(n, dtype):
     # the residual's relative size times the condition number (below three), and the value type's rounding
     assert float((x.double() - ref).norm() / ref.norm()) <= 3 * rtol + 16 * torch.finfo(dtype).eps
     assert all(torch.equal(K.solve(b, rtol=rtol), x) for _ in range(20))
+
+
+def two_sum(a, b):
+    s = a + b
+    t = s - a
+    return s, (a - (s - t)) + (b - t)
+
+
+def renorm(h, l):
+    s = h + l
+    return s, l - (s - h)
+
+
+def pair_add(a, b):
+    s, e = two_sum(a[0], b[0])
+    return renorm(s, e + (a[1] + b[1]))
+
+
+def pair_mul(a, b):
+    def fma(x, y, z):
+        return (x.astype(np.float64) * y.astype(np.float64) + z.astype(np.float64)).astype(np.float32)
+    p = a[0] * b[0]
+    return renorm(p, fma(a[1], b[0], fma(a[0], b[1], fma(a[0], b[0], -p))))
+
+
+@pytest.mark.parametrize("n,per", [(1500, 7), (3000, 15), (60_000, 15), (900_000, 7)])
+def test_row_sums_have_the_error_of_normalised_pairs(n, per):
+    """b - A x0 of the kernel's first sweep (a solve of no iterations) where it
+    is nothing but the rounding of the row sums: its norm is that of the same
+    sums in normalised float pairs on the host.  The last bits of a conversion
+    may differ: 5 %, where sums normalised only at the end are at 170 %."""
+    rng = np.random.default_rng(n)
+    far = min(n // per, 4000)
+    cols = (np.arange(n)[:, None] + far * np.arange(per)) % n
+    vals = np.exp(rng.normal(size=(n, per))) * rng.choice([-1.0, 1.0], (n, per))
+    vals[:, 0] = 1.0                                    # the diagonal: the Jacobi scaling is the identity
+    order = np.argsort(cols, 1)
+    cols, vals = np.take_along_axis(cols, order, 1), np.take_along_axis(vals, order, 1)
+    x = rng.normal(size=n)
+    b = (vals.astype(np.longdouble) * x[cols]).sum(1).astype(np.float64)
+
+    def pair(v):
+        h = v.astype(np.float32)
+        return h, (v - h).astype(np.float32)
+
+    acc = (np.zeros(n, np.float32), np.zeros(n, np.float32))
+    for j in range(per):
+        acc = pair_add(acc, pair_mul(pair(vals[:, j]), pair(x[cols[:, j]])))
+    r = pair_add(pair(b), (-acc[0], -acc[1]))
+    expect = np.linalg.norm(r[0].astype(np.float64) + r[1]) / np.linalg.norm(b)
+    K = tg.SparseMatrix(torch.tensor(vals.reshape(-1), device=DEV), shape=(n, n),
+                        indptr=torch.arange(0, n * per + 1, per, device=DEV),
+                        indices=torch.tensor(cols.reshape(-1).astype(np.int32), device=DEV))
+    with pytest.warns(UserWarning, match="did not converge"):
+        K.solve(torch.tensor(b, device=DEV), x0=torch.tensor(x, device=DEV), rtol=1e-18, maxiter=0)
+    got = K.last_solve_info.recurrence_residual
+    assert abs(got - expect) <= 0.05 * expect, (got, expect)
