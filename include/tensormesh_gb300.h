@@ -585,6 +585,10 @@ int tm_selftest_barrier_timeout(int32_t n_blocks, int64_t spins, int32_t* out_st
 int tm_selftest_grid_sum(int32_t n_blocks, int32_t absent, int32_t rounds, int64_t spins, const double* vals,
                          double* out, int32_t* out_status, void* work, int64_t work_bytes, void* stream);
 
+/* Self-test of the batched solver's dot products: out[t] = sum_k a[k][t] b[k][t]
+ * (k < len, t < n), each in one thread. */
+int tm_selftest_dot(int32_t n, int32_t len, const float* a, const float* b, double* out, void* stream);
+
 /* 1/diag(A) with missing diagonals taken as 1 (torch_solve.py:24-59). */
 int tm_csr_diagonal_inverse(int32_t dtype, int64_t n, const int64_t* indptr, const int32_t* indices,
                             const void* values, void* out, void* stream);

@@ -45,7 +45,7 @@ EXPORTS = [
     "tm_sell_fill", "tm_spmv_sell",
     "tm_gather_workspace_bytes", "tm_assemble_gather", "tm_gather_count", "tm_gather_fill", "tm_node_lists",
     "tm_group_count", "tm_group_fill", "tm_check_finite",
-    "tm_backward_gather", "tm_node_sum", "tm_selftest_grid_sum",
+    "tm_backward_gather", "tm_node_sum", "tm_selftest_grid_sum", "tm_selftest_dot",
 ]
 
 P = ctypes.c_void_p
@@ -139,6 +139,7 @@ def _declare(lib):
         "tm_backward_gather": [ctypes.POINTER(GatherPlan), P, ctypes.POINTER(AssembleArgs), P, P, P, P],
         "tm_node_sum": [i32, i64, P, P, i32, P, P, P],
         "tm_selftest_grid_sum": [i32, i32, i32, i64, P, P, ctypes.POINTER(i32), P, i64, P],
+        "tm_selftest_dot": [i32, i32, P, P, P, P],
         "tm_check_finite": [i32, i64, P, i32, i64, P, P, P],
         "tm_quadrature_points": [i32, i32, i32, P, P, P, i64, P, P],
         "tm_spmv_csr": [i32, i64, i64, P, P, P, P, P, P],

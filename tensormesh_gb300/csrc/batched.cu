@@ -10,7 +10,7 @@
 //   2. runs Jacobi-PCG on the instance's interior dofs (Dirichlet dofs are
 //      masked: x = r = z = p = 0 there, which is CG on K_ii exactly), with
 //      the instance's rows split over the C CTAs.  Dot products are formed in
-//      double-float, added per CTA in fixed point and combined through
+//      three floats a thread, added per CTA in fixed point and combined through
 //      distributed shared memory after a hardware cluster barrier
 //      (cluster_sum) -- deterministic, and no spin-wait anywhere (cluster
 //      barriers are co-scheduled by construction);
@@ -59,13 +59,31 @@ constexpr int kRowIlp = 4;  // CSR entries fetched together per row and round
 constexpr int kRows = 2;    // rows a thread advances together in the SpMV
 constexpr int kVec = 4;     // rows a thread advances together in the vector update
 
-// acc += a b of two floats: the product exactly (FMA), the sum in double-float.
-// The products were added in native FP64 before, whose conversions and
-// multiply-adds (nine warp instructions a row and iteration at ~18 cycles each
-// on an SM) took more time than the rest of the iteration.
-TM_D void dot_add(df64& acc, float a, float b) {
+// Running dot product of float vectors in three floats, s + c + d.  Every
+// product is exact (FMA) and every sum error-free (TwoSum) but d's, which holds
+// what c rounds away: a thread's sum is as good as one in FP64, whose
+// conversions and multiply-adds (nine warp instructions a row and iteration at
+// ~18 cycles each on an SM) took more time than the rest of the iteration.
+struct Dot3 {
+  float s, c, d;
+};
+TM_D void dot_add(Dot3& acc, float a, float b) {
   const float p = __fmul_rn(a, b);
-  acc = acc + df64{p, __fmaf_rn(a, b, -p)};
+  const df64 s = tm_two_sum(acc.s, p);
+  const df64 c = tm_two_sum(acc.c, s.lo);
+  const df64 e = tm_two_sum(c.hi, __fmaf_rn(a, b, -p));
+  acc = Dot3{s.hi, e.hi, __fadd_rn(acc.d, __fadd_rn(c.lo, e.lo))};
+}
+// The sum as a double, within a unit of its last place: s + c is rounded to
+// 53 bits, d is added in units of the last of them.
+TM_D double dot_value(Dot3 a) {
+  const df64 t = tm_two_sum(a.s, a.c);
+  const double v = tm_to_double(t);
+  const int e = (int)(((unsigned)__double2hiint(v) >> 20) & 0x7ffu);
+  if (e == 0 || e == 2047) return v;
+  const int up = 1075 - e;   // d 2^up, in two factors within float's range
+  const int k = __float2int_rn(__fmul_rn(__fmul_rn(a.d, tm_pow2f(up / 2)), tm_pow2f(up - up / 2)));
+  return __longlong_as_double(__double_as_longlong(v) + (__double2hiint(v) < 0 ? -(long long)k : (long long)k));
 }
 
 template <int EL>
@@ -159,7 +177,7 @@ __global__ void __launch_bounds__(kBatchThreads, 2) batched_assemble_pcg_kernel(
     float* pnew = A.p1;
     int it = 0, st = s_stop;
     while (st < 0) {
-      df64 pq_l{0.f, 0.f};
+      Dot3 pq_l{0.f, 0.f, 0.f};
       // one thread per row, kRows rows at a time (rows row, row + T, ...), each
       // row's entries fetched kRowIlp at a time with every load of the round
       // issued before the first use: a warp keeps 32 x kRows x kRowIlp
@@ -211,7 +229,7 @@ __global__ void __launch_bounds__(kBatchThreads, 2) batched_assemble_pcg_kernel(
       {
         // the cluster barrier's arrive/wait carry release/acquire semantics at
         // cluster scope: the q rows written above are visible to the other CTAs
-        double pq = tm_to_double(pq_l), none;
+        double pq = dot_value(pq_l), none;
         cluster_sum<false>(++gen, C, pq, none, s_red, s_slot);
         if (threadIdx.x == 0) {
           pq *= un_rz;
@@ -223,7 +241,7 @@ __global__ void __launch_bounds__(kBatchThreads, 2) batched_assemble_pcg_kernel(
       st = s_stop;
       if (st >= 0) break;
       const float alpha = s_scalar;
-      df64 rz_n{0.f, 0.f}, rr_n{0.f, 0.f};
+      Dot3 rz_n{0.f, 0.f, 0.f}, rr_n{0.f, 0.f, 0.f};
       // kVec rows per round, every load of the round before any store (the
       // vectors are distinct arrays, but the compiler cannot know that and
       // would otherwise serialise the rows behind one another's stores)
@@ -256,7 +274,7 @@ __global__ void __launch_bounds__(kBatchThreads, 2) batched_assemble_pcg_kernel(
           }
         }
       }
-      double rzs = tm_to_double(rz_n), rrs = tm_to_double(rr_n);
+      double rzs = dot_value(rz_n), rrs = dot_value(rr_n);
       cluster_sum<true>(++gen, C, rzs, rrs, s_red, s_slot);
       ++it;
       if (threadIdx.x == 0) {
@@ -283,6 +301,16 @@ __global__ void __launch_bounds__(kBatchThreads, 2) batched_assemble_pcg_kernel(
   }
 }
 
+// out[t] = sum_k a[k][t] b[k][t], one thread each.
+__global__ void __launch_bounds__(256) dot_selftest_kernel(int n, int len, const float* __restrict__ a,
+                                                           const float* __restrict__ b, double* __restrict__ out) {
+  const int t = blockIdx.x * 256 + threadIdx.x;
+  if (t >= n) return;
+  Dot3 acc{0.f, 0.f, 0.f};
+  for (int k = 0; k < len; ++k) dot_add(acc, a[(int64_t)k * n + t], b[(int64_t)k * n + t]);
+  out[t] = dot_value(acc);
+}
+
 template <int EL>
 int launch_batched(const BatchArgs& A, int cluster, int n_clusters, size_t smem, cudaStream_t s) {
   auto kern = batched_assemble_pcg_kernel<EL>;
@@ -306,6 +334,14 @@ int launch_batched(const BatchArgs& A, int cluster, int n_clusters, size_t smem,
 }
 
 }  // namespace tmg
+
+extern "C" int tm_selftest_dot(int32_t n, int32_t len, const float* a, const float* b, double* out, void* stream) {
+  if (n < 0 || len < 0) return TM_ERR_INVALID;
+  if (n == 0) return TM_OK;
+  if (!a || !b || !out) return TM_ERR_INVALID;
+  tmg::dot_selftest_kernel<<<(n + 255) / 256, 256, 0, static_cast<cudaStream_t>(stream)>>>(n, len, a, b, out);
+  return cudaPeekAtLastError() == cudaSuccess ? TM_OK : TM_ERR_CUDA;
+}
 
 extern "C" int64_t tm_patch_smem_bytes(int32_t element, int32_t form, int32_t n_comp, int32_t dtype,
                                        const tm_patch_plan* plan, int32_t coef_kind, int32_t chunk) {

@@ -97,3 +97,32 @@ def test_units_of_the_source_scale_the_solution_exactly(exponent):
     x, info = BatchedPoisson(meshes, source=2.0 ** exponent)(kappa)
     assert bool((info.status == 0).all()) and torch.equal(info.iterations, its)
     assert torch.equal(x, base * 2.0 ** exponent)
+
+
+@pytest.mark.parametrize("length", [1, 2, 7, 33, 64])
+@pytest.mark.parametrize("kind", ["normal", "squares", "cancel", "small"])
+def test_dot_products_of_a_thread_are_as_good_as_fp64(length, kind):
+    """A thread's sum of products against the exact one: a unit in the last
+    place of a double for the conversion, and the roundings of the third
+    float, whose terms are below 2^-47 of the partial sums."""
+    import math
+    from tensormesh_gb300 import _lib
+    rng = np.random.default_rng(length)
+    n = 300
+    a = rng.normal(size=(length, n)).astype(np.float32)
+    b = rng.normal(size=(length, n)).astype(np.float32)
+    if kind == "squares":
+        b = a.copy()
+    elif kind == "cancel":
+        b[1::2], a[1::2] = b[:-1:2][:length // 2], -a[:-1:2][:length // 2] * np.float32(1 + 2.0 ** -20)
+    elif kind == "small":
+        a, b = a * np.float32(2.0 ** -30), b * np.float32(2.0 ** -20)
+    out = torch.empty(n, dtype=torch.float64, device=DEV)
+    ta, tb = torch.tensor(a, device=DEV), torch.tensor(b, device=DEV)
+    _lib.call("tm_selftest_dot", n, length, ta.data_ptr(), tb.data_ptr(), out.data_ptr(),
+              torch.cuda.current_stream().cuda_stream)
+    for t in range(n):
+        terms = [float(x) * float(y) for x, y in zip(a[:, t], b[:, t])]   # exact: 48 bits
+        exact, size = math.fsum(terms), math.fsum(abs(v) for v in terms)
+        bound = 2.0 ** -52 * abs(exact) + length ** 2 * 2.0 ** -71 * size
+        assert abs(float(out[t]) - exact) <= bound, (t, float(out[t]) - exact, bound)
