@@ -49,14 +49,12 @@ _KERNEL_DTYPES = {torch.float32: 0, torch.float64: 1}   # TM_F32, TM_F64
 _LOCAL = threading.local()
 
 
-def _flag_buffer(device):
-    """This thread's pinned flags and event for ``device``."""
-    table = _LOCAL.__dict__.setdefault("flags", {})
-    key = str(device)
-    if key not in table:
-        flags = torch.zeros(2, dtype=torch.int32, pin_memory=True)
-        table[key] = (flags, flags.numpy(), torch.cuda.Event())
-    return table[key]
+def _flag_buffers(device) -> list:
+    """This thread's idle (pinned flags, their numpy view, event) for
+    ``device``.  A check takes one until its answer has been read: the body
+    may run further checks (a saved-tensor hook that calls an assembler), and
+    those take another."""
+    return _LOCAL.__dict__.setdefault("flags", {}).setdefault(str(device), [])
 
 
 class finite_check:
@@ -84,23 +82,32 @@ class finite_check:
             check_finite(self.items)
             return self
         from . import _lib
-        flags, view, event = _flag_buffer(dev)
+        idle = _flag_buffers(dev)
+        if idle:
+            buffer = idle.pop()
+        else:
+            pinned = torch.zeros(2, dtype=torch.int32, pin_memory=True)
+            buffer = (pinned, pinned.numpy(), torch.cuda.Event())
+        flags, view, event = buffer
         view[:] = 0
         (_, a), (_, b) = named[0], (named[1] if len(named) > 1 else (None, None))
         _lib.call("tm_check_finite", _KERNEL_DTYPES[a.dtype], a.numel(), a.data_ptr(),
                   _KERNEL_DTYPES[a.dtype if b is None else b.dtype], 0 if b is None else b.numel(),
                   0 if b is None else b.data_ptr(), flags.data_ptr(), _lib.stream_handle(dev))
         event.record(torch.cuda.current_stream(dev))
-        self.pending = (named, view, event)
+        self.pending = (named, buffer, idle)
         return self
 
     def __exit__(self, kind, *_):
         if self.pending is None:
             return
-        named, view, event = self.pending
-        event.synchronize()   # also when the body raised: the flags serve this thread's next check
-        if kind is None and view.any():
-            raise ValueError(f"{named[0 if view[0] else 1][0]} holds a non-finite value (nan or inf)")
+        named, buffer, idle = self.pending
+        view, event = buffer[1:]
+        event.synchronize()   # also when the body raised: the flags serve another check next
+        bad = [bool(v) for v in view]
+        idle.append(buffer)
+        if kind is None and any(bad):
+            raise ValueError(f"{named[0 if bad[0] else 1][0]} holds a non-finite value (nan or inf)")
 
 
 def check_finite(items: Iterable[Tuple[str, Optional[torch.Tensor]]]) -> None:

@@ -65,3 +65,41 @@ def test_rejects_bad_arguments():
     for args in ((0, -1, x.data_ptr(), 0, 0, 0), (0, 4, 0, 0, 0, 0), (7, 4, x.data_ptr(), 0, 0, 0),
                  (0, 4, x.data_ptr() + 1, 0, 0, 0)):
         assert _lib.call_status("tm_check_finite", *args, f.data_ptr(), None) == _lib.TM_ERR_INVALID
+
+
+def test_checks_inside_a_check_keep_their_own_answers():
+    good, bad = torch.ones(5000, device=DEV), torch.ones(5000, device=DEV)
+    bad[7] = float("nan")
+    with pytest.raises(ValueError, match="outer"):
+        with finite_check(("outer", bad)):
+            torch.cuda.synchronize()
+            with finite_check(("inner", good)):
+                pass
+    with finite_check(("outer", good)):
+        with pytest.raises(ValueError, match="inner"):
+            with finite_check(("inner", bad)):
+                pass
+    with finite_check(("points", good), ("kappa", good)):
+        pass
+
+
+def test_an_assembler_called_from_a_saved_tensor_hook():
+    """A pack hook runs while the assembler's call is still being checked."""
+    mesh = tg.Mesh.gen_unit_square(3, device=DEV)
+
+    class KappaLaplace(tg.ElementAssembler):
+        def forward(self, gradu, gradv, kappa):
+            return kappa * (gradu @ gradv)
+
+    asm, load = KappaLaplace.from_mesh(mesh), tg.const_node_assembler(1.0).from_mesh(mesh)
+    kappa = torch.ones(mesh.n_elements, dtype=torch.float64, device=DEV)
+    kappa[2] = float("inf")
+
+    def pack(t):
+        torch.cuda.synchronize()
+        load(mesh.points)
+        return t
+
+    with pytest.raises(ValueError, match="the coefficient"):
+        with torch.autograd.graph.saved_tensors_hooks(pack, lambda t: t):
+            asm(mesh.points, element_data={"kappa": kappa.requires_grad_(True)})
