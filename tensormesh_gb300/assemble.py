@@ -255,6 +255,13 @@ class _AssemblerDevice:
     def dtype(self) -> torch.dtype:
         return self.points.dtype
 
+    def __setattr__(self, name, value):
+        super().__setattr__(name, value)
+        # native FP64 runs on the patch plan, which the topology of a large
+        # mesh does not build by itself: built here, not in the first call
+        if name == "precision" and value == "native" and "topology" in self.__dict__:
+            self.topology.plan_for(1)
+
     def type(self, dtype: torch.dtype):
         if dtype not in (torch.float32, torch.float64):
             raise TypeError(f"the dtype {dtype} is not supported (float32 or float64)")
@@ -477,6 +484,8 @@ class NodeAssembler(_AssemblerDevice, nn.Module):
     def __init__(self, topology: MeshTopology, points: torch.Tensor, quadrature_order: int, *args, **kwargs):
         super().__init__()
         self.topology = topology
+        if self.precision == "native":
+            topology.plan_for(1)
         self.quadrature_order = int(quadrature_order)
         self.register_buffer("points", points, persistent=False)
         self.element_types = [topology.element_type]

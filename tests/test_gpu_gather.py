@@ -683,3 +683,36 @@ def test_p1_stiffness_is_as_accurate_as_the_patch_kernels(etype, n, form, q, mon
 def test_p2_stiffness_is_as_accurate_as_the_patch_kernels(etype, n, form, q, monkeypatch):
     once, patch = both_routes(etype, n, form, q, monkeypatch)
     assert (once <= patch).all(), (once, patch)
+
+
+# -- native FP64 -------------------------------------------------------------------
+@pytest.mark.parametrize("how", ["instance", "class"])
+@pytest.mark.parametrize("kind", ["matrix", "load"])
+def test_the_first_native_call_can_be_captured(how, kind):
+    """Its plan is there when the precision is chosen, so that the first call
+    runs inside a CUDA graph (the tables come from an earlier call of any
+    assembler of this order)."""
+    pts, el = ragged("tetra", 5, 2)
+    base = KappaLaplace if kind == "matrix" else tg.const_node_assembler(2.0)
+    cls = type("Native", (base,), {"precision": "native"} if how == "class" else {})
+    x = torch.tensor(pts, device=DEV)
+    kw = {"element_data": {"kappa": torch.ones(el.shape[0], dtype=torch.float64, device=DEV)}} if kind == "matrix" else {}
+    cells = lambda: {"tetra": torch.tensor(el, device=DEV)}  # noqa: E731
+    values = lambda a: a(x, **kw).values if kind == "matrix" else a(x)  # noqa: E731
+    emulated = values(base.from_mesh(tg.Mesh(points=x, cells=cells()), 2))
+    asm = cls.from_mesh(tg.Mesh(points=x, cells=cells()), 2)
+    if how == "instance":
+        asm.precision = "native"
+    if kind == "matrix":   # recognising the form runs host code, not kernels
+        asm._resolve_form(None, kw["element_data"], {}, {})
+    tg.set_input_checks(False)
+    try:
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g):
+            out = values(asm)
+    finally:
+        tg.set_input_checks(True)
+    g.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(values(asm), out)
+    assert float((out - emulated).abs().max()) <= 1e-12 * float(emulated.abs().max())
