@@ -716,3 +716,38 @@ def test_the_first_native_call_can_be_captured(how, kind):
     torch.cuda.synchronize()
     assert torch.equal(values(asm), out)
     assert float((out - emulated).abs().max()) <= 1e-12 * float(emulated.abs().max())
+
+
+# -- units, position and coefficients of P1 stiffness ----------------------------------------
+@pytest.mark.parametrize("etype,n", [("triangle", 7), ("tetra", 4)])
+@pytest.mark.parametrize("form", ["laplace", "elasticity"])
+@pytest.mark.parametrize("scale", [1e-9, 1e-3, 1e3, 1e9])
+def test_units_of_p1_stiffness(etype, n, form, scale):
+    pts, el = ragged(etype, n, 11)
+    check(pts * scale, el, etype, form, np.exp(np.random.default_rng(n).normal(size=el.shape[0])))
+
+
+@pytest.mark.parametrize("etype,n", [("triangle", 7), ("tetra", 4)])
+@pytest.mark.parametrize("form", ["laplace", "elasticity"])
+def test_p1_stiffness_far_from_the_origin(etype, n, form):
+    """The oracle works on the same coordinates moved back, an exact
+    subtraction: its own Jacobian sums would cancel."""
+    pts, el = ragged(etype, n, 12)
+    shift = np.array([12345.0, -23456.0, 3456.0])[: pts.shape[1]]
+    away = pts + shift
+    kappa = np.exp(np.random.default_rng(n).normal(size=el.shape[0]))
+    mesh = tg.Mesh(points=torch.tensor(away, device=DEV), cells={etype: torch.tensor(el, device=DEV)})
+    asm = FORMS[form].from_mesh(mesh, quadrature_order=2)
+    got = asm(mesh.points, element_data={"kappa": torch.tensor(kappa, device=DEV)}).values.cpu().numpy()
+    ref = fem.assemble_csr(away - shift, el, etype, form, 2, coef=kappa)[2]
+    assert np.max(np.abs(got - ref)) <= 1e-12 * np.max(np.abs(ref))
+
+
+@pytest.mark.parametrize("etype,n", [("triangle", 7), ("tetra", 4)])
+@pytest.mark.parametrize("form", ["laplace", "elasticity"])
+@pytest.mark.parametrize("size", [1e150, 1e-150])
+def test_coefficients_of_p1_stiffness_beyond_float_range(etype, n, form, size):
+    pts, el = ragged(etype, n, 13)
+    kappa = np.exp(np.random.default_rng(n).normal(size=el.shape[0]))
+    check(pts, el, etype, form, size * kappa)
+    check(pts, el, etype, form, kappa * np.where(np.arange(el.shape[0]) % 97 == 0, 1e80, 1.0))
