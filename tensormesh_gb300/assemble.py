@@ -74,7 +74,7 @@ class MeshTopology:
         # gradients of patch forms) builds what it needs.
         if not self.element_once or self.gather.struct(0) is None or self.gather.struct(1) is None:
             self.plan_for(1)
-        self._block = {}
+        self._block = {1: (self.pattern.indptr, self.pattern.indices)}
         self._incidence = None
 
     # accumulator budget per patch in node slots (the scalar forms' kernels
@@ -124,7 +124,11 @@ class MeshTopology:
 
     def dof_pattern(self, H: int):
         if H not in self._block:
-            self._block[H] = block_pattern(self.pattern.indptr, self.pattern.indices, H)
+            with self._lock:
+                if H not in self._block:
+                    block = block_pattern(self.pattern.indptr, self.pattern.indices, H)
+                    _now(self.elements.device)   # complete on every stream, as the pattern is
+                    self._block[H] = block
         return self._block[H]
 
     @property

@@ -751,3 +751,21 @@ def test_coefficients_of_p1_stiffness_beyond_float_range(etype, n, form, size):
     kappa = np.exp(np.random.default_rng(n).normal(size=el.shape[0]))
     check(pts, el, etype, form, size * kappa)
     check(pts, el, etype, form, kappa * np.where(np.arange(el.shape[0]) % 97 == 0, 1e80, 1.0))
+
+
+def test_block_patterns_are_complete_when_they_become_visible(monkeypatch):
+    mesh = tg.Mesh.gen_unit_cube(4, device=DEV)
+    topo = KappaLaplace.from_mesh(mesh).topology
+    inner = tg.assemble.block_pattern
+
+    def slow(*args):
+        out = inner(*args)
+        torch.cuda._sleep(100_000_000)
+        return out
+
+    monkeypatch.setattr("tensormesh_gb300.assemble.block_pattern", slow)
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        topo.dof_pattern(3)
+        assert side.query()
