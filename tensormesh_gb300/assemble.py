@@ -186,12 +186,19 @@ def _mesh_single_type(mesh):
     return etype, elements
 
 
-# Fewest elements for the element-once kernels.  Below, the one-launch patch
-# kernel takes less host time than three launches and a scratch allocation
-# (us a call, patch / element-once): P1, 24576 tetrahedra 92 / 104 with the GPU
-# idle half of it, and element-once ahead from there in GPU time; P2 triangles
-# 2048 elasticity 113 / 104; P2 tetrahedra 48 elements 166 / 109 (Laplace),
-# 3072 elements 581 / 107.
+# Fewest elements for the element-once kernels.  They take less time on the GPU
+# at every size, but three launches and a scratch allocation, 10 to 15 us of host
+# time more than the one patch launch.  The line lies where the GPU time saved is
+# above that in every form, so that a call that is waited for gains; calls issued
+# one after another stay bound by the host to larger sizes still (float64 P1
+# Laplace, us a call, patch / element-once: 16,200 triangles 88 / 99, 24,576
+# tetrahedra 88 / 100).  us on the GPU, patch / element-once:
+#   P1  16,200 triangles   Laplace 32 / 8, mass 35 / 14, elasticity 67 / 10, load
+#       22 / 10; float32 Laplace 23 / 7, load 17 / 6
+#       16,464 tetrahedra  32 / 12, 103 / 17, 55 / 16, 65 / 15; float32 23 / 7, 31 / 8
+#       5,000 triangles 29 / 8 and 6,000 tetrahedra 28 / 12 (Laplace) lie below it
+#   P2  2,048 triangles    Laplace 35 / 16, mass 37 / 19, elasticity 106 / 42
+#       48 tetrahedra      Laplace 159 / 27, mass 60 / 25, elasticity 1887 / 68
 _GATHER_MIN_ELEMENTS = {"triangle": 16384, "tetra": 16384, "triangle6": 2048, "tetra10": 0}
 
 

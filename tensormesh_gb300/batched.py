@@ -59,13 +59,13 @@ def choose_cluster(rows: Sequence[int], dim: int, slots: dict) -> int:
     takes a number of iterations that grows with the nodes along one axis.
     Small clusters win where the batch has many times more instances than the
     chip has clusters, large ones where a few instances set the time: 64 square
-    meshes of 32^2 .. 160^2 cells ran 26.8 / 14.8 / 9.5 / 13.4 ms at C = 2 / 4 /
-    8 / 16, 256 of 32^2 .. 256^2 cells 123.8 / 80.2 / 85.5 / 114.2 ms, 20 of
-    20^2 .. 140^2 cells 16.8 / 10.3 / 6.4 / 4.4 ms, and 200 of 20^2 cells 0.61 /
-    0.95 / 1.43 ms at C = 1 / 2 / 4.  The estimate picks the fastest of each.
-    Within 5 % the smaller C is taken: the estimate is no closer than that, and
-    on tiny systems (8 of 16^2 cells: 0.34 / 0.39 / 0.40 ms at C = 1 / 4 / 16)
-    a larger cluster only costs its barrier."""
+    meshes of 32^2 .. 160^2 cells ran 26.0 / 14.6 / 9.3 / 14.9 ms at C = 2 / 4 /
+    8 / 16, 256 of 32^2 .. 256^2 cells 132.7 / 96.7 / 105.2 / 133.4 ms, 20 of
+    20^2 .. 140^2 cells 17.1 / 9.8 / 6.9 / 5.4 ms, and 200 of 20^2 cells 0.68 /
+    1.02 / 1.53 ms at C = 1 / 2 / 4.  The estimate picks the fastest of each.
+    Within 5 % the smaller C is taken: the estimate is no closer than that.
+    Batches of a few tiny systems take the same time at any size (8 of 16^2
+    cells: 0.42 .. 0.45 ms)."""
     rows = sorted(rows, reverse=True)
     span = {}
     for c, n_slots in slots.items():

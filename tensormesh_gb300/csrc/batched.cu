@@ -53,8 +53,9 @@ struct BatchArgs {
 };
 
 constexpr int kBatchThreads = 512;
-// 256 meshes of 32^2 to 256^2 cells, ms a launch: 2 rows x 4 entries 80.9,
-// 1 x 8 94.8, 2 x 8 90.3, 3 x 4 92.2 (2 x 4 with FP64 dot products: 99.8)
+// 256 meshes of 32^2 to 256^2 cells, ms a launch: 2 rows x 4 entries 84.9 (80.9
+// with dot products in pairs of floats, 99.8 in FP64); with pairs, 1 x 8 94.8,
+// 2 x 8 90.3, 3 x 4 92.2
 constexpr int kRowIlp = 4;  // CSR entries fetched together per row and round
 constexpr int kRows = 2;    // rows a thread advances together in the SpMV
 constexpr int kVec = 4;     // rows a thread advances together in the vector update

@@ -188,8 +188,7 @@ TM_D bool p1_element(const A (&d)[D][D], A cw, A (&out)[p1_values<D, kElast>()])
 // its 32 consecutive elements write one contiguous run.  Bound by instruction
 // issue: about 800 instructions an element in double-float, issued at 75 %,
 // with the FP64 pipe (the nine subtractions of the edges) at 52 %; 64
-// registers hold eight CTAs an SM (88 us for 3.07 M tetrahedra; 72 registers
-// and seven CTAs: 105 us).
+// registers hold eight CTAs an SM (95 us for 3.07 M tetrahedra).
 template <class T, int D, bool kElast>
 __global__ void __launch_bounds__(kElThreads, 8)
 p1_element_kernel(int64_t n_el, const int32_t* __restrict__ el, tm_assemble_args args, Head* __restrict__ head,
@@ -564,8 +563,8 @@ template <class T, int B> size_t group_rows_smem(const tm_gather_plan& p) {
 // K = lam M + mu M^T + mu tr(M) I; the diagonal block is minus the sum of the
 // row's (the cofactors of an element add to zero).  One thread per entry; the
 // blocks replace the cofactors in shared memory once every thread holds its
-// own, and the CTA writes the rows in order.  Issue-bound (63 % of the slots):
-// nine double-float multiply-adds per record; 380 us at 64^3, where the patch
+// own, and the CTA writes the rows in order.  Issue-bound (65 % of the slots):
+// nine double-float multiply-adds per record; 376 us at 64^3, where the patch
 // kernel, which forms all sixteen blocks of an element from staged values,
 // takes 1390 us.
 constexpr int kBlkGrpThreads = kBlockEntries;

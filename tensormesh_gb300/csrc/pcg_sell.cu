@@ -1,6 +1,7 @@
 // Jacobi-PCG over a SELL-32 copy of the matrix, in two forms: standard
-// (Hestenes-Stiefel) PCG with two grid barriers per iteration (the default,
-// pcg_sell_hs_kernel), and the pipelined form of Ghysels & Vanroose ("Hiding
+// (Hestenes-Stiefel) PCG with two barriers per iteration where the system stays
+// on chip and three where it streams (the default, pcg_sell_hs_kernel), and the
+// pipelined form of Ghysels & Vanroose ("Hiding
 // global synchronization latency in the preconditioned Conjugate Gradient
 // algorithm", Parallel Computing 40(7), 2014, Algorithm 4) with one barrier
 // per iteration (pcg_sell_kernel).  The pipelined recurrences lose accuracy
@@ -239,7 +240,7 @@ __global__ void sell_fill_kernel(int64_t n, const int64_t* __restrict__ indptr, 
 // acc[u] = sum_j sval[.] * g(scol[.]) over the rows of slices sl + u * kSellWarps
 // (u < kSellRows) of [sl, s_hi), for the calling lane's row.  g gathers the
 // operand's column value (one vector, or a combination of two).  Double-float
-// sums are normalised after every entry: left to the end (2 to 4 % of an
+// sums are normalised after every entry: left to the end (2 to 9 % of an
 // iteration less) a row's error is 1.7 times as large for 7 entries, 2.2 for 15
 // and 2.8 for 27 (rms, in units of the sum of |products|).
 template <class S, class CT, bool kGen = false, class G>
@@ -299,7 +300,8 @@ TM_D void sell_rows(const int64_t* __restrict__ sptr, const CT* scol, const S* s
 // and pt_old gathered and every vector in global memory / pt in a sweep of its
 // own / vectors in shared memory as well: 64^3 Poisson 21.3 / 20.4 / 19.0, 96^3
 // 53.5 / 53.5 / 46.3, 128^3 116 / 109 / 102, 1000^2 38.9 / - / 30.1, 40^3
-// elasticity 42.6 / 39.4 / 28.8.  kResident: a CTA's share of the matrix, x, q, M and its own rows of r and pt stay
+// elasticity 42.6 / 39.4 / 28.8 (with row sums normalised at the end; after every
+// entry, as now: 64^3 19.8, 96^3 47.0, 128^3 104, 1000^2 32.9).  kResident: a CTA's share of the matrix, x, q, M and its own rows of r and pt stay
 // in shared memory for the whole solve, and an iteration reads only the
 // gathered r and pt from L2.  kCluster: the same in one cluster, whose barriers
 // take a microsecond instead of three.  Chosen by launch_pcg_sell; a CTA whose
@@ -806,9 +808,9 @@ size_t resident_bytes(int64_t n_slices, int64_t n_pad, int nb, int optin, int& c
 // One cluster of 16 CTAs (8 where 16 do not fit a GPC) when the system fits
 // its shared memory (2D: to about 29,000 rows), a CTA per SM when it fits that
 // (2D to 270,000 rows, 3D to 130,000), streaming otherwise.  us per iteration,
-// a call's other work included: 64^2 6.5 in a cluster, 10.0 on the grid, 15.0
+// a call's other work included: 64^2 6.6 in a cluster, 10.0 on the grid, 15.0
 // before (atomic barriers, FP64 shuffle trees, divisions in every thread);
-// 256^2 9.3 resident, 16.2 before; 96^3 46 streaming, 65 before.
+// 256^2 9.8 resident, 16.2 before; 96^3 47 streaming, 65 before.
 template <class S, class CT>
 int sell_launch(int64_t n_slices, int64_t n_pad, SellLaunch& how) {
   int dev = 0, sms = 0, optin = 0;

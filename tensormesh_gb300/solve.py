@@ -2,8 +2,9 @@
 
 ``solve`` mirrors the reference's ``K.solve(b, **kw)`` (torch_sla signature;
 docs user_guide/linear_solvers.rst:80-110) for SPD systems: the solve runs
-as one cooperative CUDA launch (``tm_pcg_jacobi``), then the true residual
-||b - K x|| / ||b|| is recomputed with a plain SpMV; if it is above the
+as one CUDA launch over a SELL-32 copy of the matrix
+(``tm_pcg_jacobi_sell``; ``tm_pcg_jacobi`` with the CSR layout), then the true
+residual ||b - K x|| / ||b|| is recomputed with a plain SpMV; if it is above the
 target although the recurrence met it, the solve continues by iterative
 refinement (a bounded number of correction solves).  Non-convergence warns, as the reference does
 (sparse/solve/torch_solve.py:125-126, 245-246).  Gradients flow through the
