@@ -180,14 +180,15 @@ TM_D bool coef_in_range(double c) {
 
 constexpr int kTetChunk = kThreads;  // elements staged per chunk (one per thread)
 
-// A double in double-float for 2^-74 <= |x| < 2^128: hi = x truncated to 24
-// significant bits, lo = the low 29 bits rounded to float (2^-48 of x).  The
-// fast pass uses it for coefficients it has checked with coef_in_range (any
+// A double in double-float for x = 0 and 2^-74 <= |x| < 2^128: hi = x truncated
+// to 24 significant bits, lo = the low 29 bits rounded to float (2^-48 of x).
+// The fast pass uses it for coefficients it has checked with coef_in_range (any
 // other value sends the patch to the native pass, so its result is unused).
 TM_D L2 l2_from_double_in_range(double x) {
   const unsigned long long b = (unsigned long long)__double_as_longlong(x);
   const unsigned hw = (unsigned)(b >> 32);
   const unsigned e = (hw >> 20) & 0x7ffu;
+  if (e == 0u) return L2{0.f, 0.f};
   const float h = __uint_as_float((hw & 0x80000000u) | ((e - 896u) << 23) | ((unsigned)(b >> 29) & 0x7fffffu));
   const float l = __fmul_rn(__int2float_rn((int)(b & 0x1fffffffull)), __uint_as_float((e - 948u) << 23));
   return L2{h, (hw & 0x80000000u) ? -l : l};

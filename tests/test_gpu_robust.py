@@ -119,3 +119,15 @@ def test_sliver_fan(height):
     kappa = np.exp(np.random.default_rng(ring).normal(size=ring))
     for form in ("laplace", "elasticity"):
         check(pts, el, "tetra", form, kappa)
+
+
+@pytest.mark.parametrize("etype", ["triangle", "triangle6", "tetra", "tetra10"])
+@pytest.mark.parametrize("form", ["laplace", "mass", "elasticity"])
+def test_zero_coefficients(etype, form):
+    """Elements without a coefficient (holes) among others."""
+    mesh = jittered(etype, 4, 9)
+    el = mesh.cells[etype].numpy()
+    coef = np.exp(np.random.default_rng(3).normal(size=el.shape[0]))
+    coef[::3] = 0.0
+    coef[1::7] = -0.0
+    check(mesh.points.numpy(), el, etype, form, coef)
