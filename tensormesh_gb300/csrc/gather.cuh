@@ -15,7 +15,7 @@
 // coefficients scaled the same way, so neither units nor position matter.  Its
 // values are O(1) times 2^s, s = k p + k_coef (p the form's power of length).
 // The scratch holds them as float pairs relative to a call-wide exponent S,
-// that of element 0, as long as |s - S| <= kWindow; an element outside the
+// the median of 32 elements', as long as |s - S| <= kWindow; an element outside the
 // window stores plain doubles instead, sets its bit in `wide` and raises
 // `head->any`.  Where that is raised, every group of rows looks at its elements'
 // bits, and those that hold such an element add in native FP64 (loads: nodes).
@@ -120,6 +120,26 @@ TM_D double real_of(float2 v, bool wide, int S) {
 // Exponent of an element from its raw edge exponent and coefficient exponent.
 // ecoef = 0 means every coefficient is zero (or subnormal): the values are 0.
 TM_D int elem_exp(int eedge, int ecoef, int power) { return (eedge - 1023) * power + (ecoef ? ecoef - 1023 : 0); }
+
+// The element that a lane of the head kernels looks at: 32 of them, spread over
+// the mesh.
+TM_D int64_t head_element(int64_t n_el) { return (n_el - 1) * (int64_t)threadIdx.x / 31; }
+
+// Median of the exponents of the lanes that have one (0 if none has): one
+// outlying element must not leave all the others outside the window.  Whole
+// warps call it.
+TM_D int median_exp(int s, bool have) {
+  const int lane = threadIdx.x & 31;
+  const unsigned m = __ballot_sync(0xffffffffu, have);
+  if (m == 0u) return 0;
+  int rank = 0;
+  for (int j = 0; j < 32; ++j) {
+    const int o = __shfl_sync(0xffffffffu, s, j);
+    if (((m >> j) & 1u) != 0u && (o < s || (o == s && j < lane))) ++rank;
+  }
+  const unsigned hit = __ballot_sync(0xffffffffu, have && rank == __popc(m) / 2);
+  return __shfl_sync(0xffffffffu, s, __ffs(hit) - 1);
+}
 
 // ---- arithmetic traits of the stored value ---------------------------------
 // Sto<T>: what the scratch holds for value type T and the arithmetic of the sums

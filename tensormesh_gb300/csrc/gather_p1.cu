@@ -15,22 +15,24 @@ int64_t p1_value_bytes(int element, int form, int dtype, int64_t n_el) {
                             : (el ? p1_bytes<3, true>(dtype, n_el) : p1_bytes<3, false>(dtype, n_el));
 }
 
-// Clears the flag, sums the weights and sets the common exponent to that of
-// element 0.
+// Clears the flag, sums the weights and sets the common exponent (one warp).
 template <class T, int D>
-__global__ void p1_head_kernel(const int32_t* __restrict__ el, tm_assemble_args args, Head* head) {
+__global__ void p1_head_kernel(int64_t n_el, const int32_t* __restrict__ el, tm_assemble_args args, Head* head) {
   constexpr int NB = D + 1;
   double wsum = 0.0;
   for (int q = 0; q < args.n_quad; ++q) wsum += args.tables[q];
   int S = 0;
   if constexpr (sizeof(T) == 8) {
     int v[NB];
-    load_conn<NB>(el, 0, v);
+    const int64_t e = head_element(n_el);
+    load_conn<NB>(el, e, v);
     Edges<T, D, NB> ed;
     ed.load(static_cast<const T*>(args.points), v);
-    const int ec = dexp(p1_coef<NB>(args, 0, v, wsum));
-    S = elem_exp(ed.ok() ? ed.emax : 1023, ec > 0 && ec < 2047 ? ec : 1023, D - 2);
+    const int ec = dexp(p1_coef<NB>(args, e, v, wsum));
+    const bool have = ed.ok() && ec > 0 && ec < 2047;
+    S = median_exp(have ? elem_exp(ed.emax, ec, D - 2) : 0, have);
   }
+  if (threadIdx.x != 0) return;
   head->S = S;
   head->any = 0u;
   head->w = sizeof(T) == 8 ? pair_of(wsum) : make_float2((float)wsum, 0.f);
@@ -43,7 +45,7 @@ int launch_p1(const tm_gather_plan& plan, const tm_assemble_args& args, void* wo
   const int64_t n = plan.n_elements;
   const Scratch sc = scratch_of(work, n, n * p1_values<D, kElast>() * (int64_t)sizeof(S));
   S* vals = reinterpret_cast<S*>(sc.vals);
-  p1_head_kernel<T, D><<<1, 1, 0, s>>>(plan.elements, args, sc.head);
+  p1_head_kernel<T, D><<<1, 32, 0, s>>>(n, plan.elements, args, sc.head);
   p1_element_kernel<T, D, kElast><<<(unsigned)((n + kElThreads - 1) / kElThreads), kElThreads, 0, s>>>(
       n, plan.elements, args, sc.head, sc.wide, vals);
   const S* cv = vals;

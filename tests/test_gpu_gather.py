@@ -769,3 +769,44 @@ def test_block_patterns_are_complete_when_they_become_visible(monkeypatch):
     with torch.cuda.stream(side):
         topo.dof_pattern(3)
         assert side.query()
+
+
+@pytest.mark.parametrize("etype,n", [("tetra", 8), ("triangle", 24), ("tetra10", 4), ("triangle6", 9)])
+@pytest.mark.parametrize("first", [2.0 ** 70, 2.0 ** -70, 0.0])
+def test_an_outlying_first_element_leaves_the_others_in_the_window(etype, n, first):
+    """The first element's coefficient (load: its nodes') far from the others',
+    or zero: rows that share no group with it keep the bits they have without
+    it, that is, they still add in pairs."""
+    base = tg.Mesh.gen_unit_square(n) if etype.startswith("tri") else tg.Mesh.gen_unit_cube(n)
+    mesh = (base.to_p2() if etype in ("tetra10", "triangle6") else base).to(DEV)
+    cells = mesh.cells[etype].long()
+    g = torch.Generator(device=DEV).manual_seed(n)
+    x = mesh.points + 0.1 / n * torch.rand(mesh.points.shape, generator=g, device=DEV, dtype=torch.float64)
+    # coefficients of another scale than one, so that a window around one would miss them
+    k = 2.0 ** 100 * torch.exp(torch.randn(cells.shape[0], generator=g, device=DEV, dtype=torch.float64))
+    far = k.clone()
+    far[0] *= first
+    for form in ("laplace", "mass", "elasticity"):
+        asm = FORMS[form].from_mesh(mesh, 2)
+        a, b = (asm(x, element_data={"kappa": c}) for c in (k, far))
+        H = a.shape[0] // x.shape[0]
+        plan = asm.topology.gather
+        group = torch.arange(x.shape[0], device=DEV)
+        if plan.p1:
+            group[plan.order.long()] = group.clone()
+        group //= plan.struct(H).rows_per_cta
+        rows = ~torch.isin(group, group[cells[0]]).repeat_interleave(H)[a.row]
+        assert int(rows.sum()) > 500 and torch.equal(a.values[rows], b.values[rows])
+
+    class PointLoad(tg.NodeAssembler):
+        def forward(self, v, f):
+            return v * f
+
+    load = PointLoad.from_mesh(mesh, 2)
+    f = 2.0 ** 100 * (torch.rand(x.shape[0], generator=g, device=DEV, dtype=torch.float64) + 0.5)
+    f2 = f.clone()
+    f2[cells[0]] *= first
+    a, b = (load(x, point_data={"f": c}) for c in (f, f2))
+    away = torch.ones(x.shape[0], dtype=torch.bool, device=DEV)
+    away[cells[torch.isin(cells, cells[0]).any(1)]] = False
+    assert int(away.sum()) > 100 and torch.equal(a[away], b[away])
