@@ -52,11 +52,11 @@ class MeshTopology:
         assert elements.shape[1] == self.n_basis, \
             f"{element_type} elements have {self.n_basis} nodes, but the connectivity has {elements.shape[1]} columns"
         check_connectivity(elements, int(points.shape[0]))
-        self.elements = elements.to(torch.int32).contiguous()
-        if self.elements.data_ptr() % 16:   # a view into a larger array: the kernels read four nodes at once
-            self.elements = self.elements.clone()
+        # always a copy: the element-once kernels read it in every call, four
+        # nodes at once, and the caller's array may lie anywhere and be changed
+        # or used again after this
+        self.elements = elements.to(torch.int32, copy=True, memory_format=torch.contiguous_format)
         self._source = elements   # kept: topology_for knows a connectivity by its address
-        self._elements_long = elements.long()
         self.n_points = int(points.shape[0])
         self.n_elements = int(elements.shape[0])
         self.timings = {}  # seconds of the pattern build and of each patch plan (device work included)
@@ -89,7 +89,7 @@ class MeshTopology:
             budget = self._SLOT_BUDGET.get(H, max(64, 6144 // (H * H)))
         if budget not in self._plans:
             t0 = _now(self._coords.device)
-            plan = PatchPlan(self._elements_long, self._coords, self.pattern, slot_budget=budget)
+            plan = PatchPlan(self.elements.long(), self._coords, self.pattern, slot_budget=budget)
             self._plans[budget] = (plan, plan.to_struct())
             self.timings[f"plan_{budget}_s"] = _now(self._coords.device) - t0
         return self._plans[budget]

@@ -55,3 +55,21 @@ def test_connectivity_at_an_odd_address_is_copied(word):
     assert view.data_ptr() % 16 and view.is_contiguous()
     topo = tg.assemble.MeshTopology(view, mesh.points, "tetra")
     assert topo.elements.data_ptr() % 16 == 0 and torch.equal(topo.elements, el)
+
+
+@pytest.mark.parametrize("dtype", [torch.int32, torch.int64])
+@pytest.mark.parametrize("transposed", [False, True])
+def test_a_connectivity_changed_afterwards_does_not_reach_the_topology(dtype, transposed):
+    """The caller's array is written over once the assembler is made: the
+    connectivity and the plans built later are those of the mesh it was made for."""
+    mesh = tg.Mesh.gen_unit_cube(2)
+    el = mesh.cells["tetra"].to(dtype, copy=True)
+    if transposed:
+        el = el.t().contiguous().t()
+    expect = tg.assemble.MeshTopology(mesh.cells["tetra"], mesh.points, "tetra")
+    topo = tg.assemble.MeshTopology(el, mesh.points, "tetra")
+    el.fill_(10 ** 6)
+    assert torch.equal(topo.elements, mesh.cells["tetra"].to(torch.int32)) and topo.elements.is_contiguous()
+    for budget in (1, 3):
+        a, b = topo.plan_for(budget)[0], expect.plan_for(budget)[0]
+        assert torch.equal(a.vtx, b.vtx) and torch.equal(a.inc_pos, b.inc_pos) and torch.equal(a.elem, b.elem)
