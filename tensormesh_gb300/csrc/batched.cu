@@ -76,12 +76,15 @@ TM_D void dot_add(Dot3& acc, float a, float b) {
   acc = Dot3{s.hi, e.hi, __fadd_rn(acc.d, __fadd_rn(c.lo, e.lo))};
 }
 // The sum as a double, within a unit of its last place: s + c is rounded to
-// 53 bits, d is added in units of the last of them.
+// 53 bits, d is added in units of the last of them.  Where terms cancelled and
+// left d more than 2^-32 of s + c, d may exceed what an int counts: those few
+// add it in FP64.
 TM_D double dot_value(Dot3 a) {
   const df64 t = tm_two_sum(a.s, a.c);
   const double v = tm_to_double(t);
   const int e = (int)(((unsigned)__double2hiint(v) >> 20) & 0x7ffu);
-  if (e == 0 || e == 2047) return v;
+  if (e == 2047) return v;
+  if (e == 0 || fabsf(a.d) >= fabsf(t.hi) * 0x1p-32f) return v + (double)a.d;
   const int up = 1075 - e;   // d 2^up, in two factors within float's range
   const int k = __float2int_rn(__fmul_rn(__fmul_rn(a.d, tm_pow2f(up / 2)), tm_pow2f(up - up / 2)));
   return __longlong_as_double(__double_as_longlong(v) + (__double2hiint(v) < 0 ? -(long long)k : (long long)k));

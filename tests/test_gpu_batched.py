@@ -126,3 +126,27 @@ def test_dot_products_of_a_thread_are_as_good_as_fp64(length, kind):
         exact, size = math.fsum(terms), math.fsum(abs(v) for v in terms)
         bound = 2.0 ** -52 * abs(exact) + length ** 2 * 2.0 ** -71 * size
         assert abs(float(out[t]) - exact) <= bound, (t, float(out[t]) - exact, bound)
+
+
+@pytest.mark.parametrize("left", [2.0 ** -20, 2.0 ** -28, 2.0 ** -36, 0.0])
+def test_dot_products_that_cancel_keep_what_is_left(left):
+    """Every product is taken back in another order, then one small product is
+    added: the bound of the test above, where s + c is no larger than d or
+    vanishes."""
+    import math
+    from tensormesh_gb300 import _lib
+    rng = np.random.default_rng(4)
+    n, half = 300, 32
+    h, g = (rng.normal(size=(half, n)).astype(np.float32) for _ in range(2))
+    back = rng.permutation(half)
+    last = np.full((1, n), left, np.float32)
+    a, b = np.concatenate([h, -h[back], last]), np.concatenate([g, g[back], np.ones_like(last)])
+    out = torch.empty(n, dtype=torch.float64, device=DEV)
+    ta, tb = torch.tensor(a, device=DEV), torch.tensor(b, device=DEV)
+    _lib.call("tm_selftest_dot", n, a.shape[0], ta.data_ptr(), tb.data_ptr(), out.data_ptr(),
+              torch.cuda.current_stream().cuda_stream)
+    for t in range(n):
+        terms = [float(x) * float(y) for x, y in zip(a[:, t], b[:, t])]   # exact: 48 bits
+        exact, size = math.fsum(terms), math.fsum(abs(v) for v in terms)
+        bound = 2.0 ** -52 * abs(exact) + a.shape[0] ** 2 * 2.0 ** -71 * size
+        assert abs(float(out[t]) - exact) <= bound, (t, float(out[t]) - exact, bound)
