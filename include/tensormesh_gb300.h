@@ -467,8 +467,8 @@ int tm_pcg_result(const void* work, int32_t* iters, double* res, double* bnorm, 
 /*
  * The same Jacobi-PCG over a SELL-32 copy of the matrix (coalesced row
  * slices, the preconditioner folded into the stored values).  method
- * TM_PCG_STANDARD: the recurrence of tm_pcg_jacobi, two grid barriers per
- * iteration; TM_PCG_PIPELINED: pipelined CG (Ghysels & Vanroose 2014), one
+ * TM_PCG_STANDARD: the recurrence of tm_pcg_jacobi, two barriers per
+ * iteration where the system stays on chip, three where it streams; TM_PCG_PIPELINED: pipelined CG (Ghysels & Vanroose 2014), one
  * barrier per iteration, whose recurrences lose accuracy faster (it can stop
  * with TM_ERR_BREAKDOWN where the standard form converges).  Same stopping
  * rule, statuses and meaning of x as tm_pcg_jacobi; the result is read back
@@ -485,7 +485,8 @@ int tm_pcg_result(const void* work, int32_t* iters, double* res, double* bnorm, 
  *
  * tm_pcg_jacobi_sell: work is caller-owned device scratch of at least
  * tm_pcg_sell_workspace_bytes(dtype, n, n_pad) bytes (the SELL copy of the
- * values, the preconditioned vectors, per-CTA partial sums).  A slice_ptr
+ * values, the preconditioned vectors, per-CTA partial sums), 8-byte aligned.
+ * A slice_ptr
  * that does not cover every row, or a column index outside [0, n), returns
  * TM_ERR_INDEX through tm_pcg_result (nothing is iterated).  Asynchronous
  * on `stream`.
@@ -493,7 +494,7 @@ int tm_pcg_result(const void* work, int32_t* iters, double* res, double* bnorm, 
 int64_t tm_sell_plan(int64_t n, const int64_t* indptr, const int32_t* indices, int64_t* slice_ptr,
                      int32_t* out_narrow, void* stream);
 int64_t tm_pcg_sell_workspace_bytes(int32_t dtype, int64_t n, int64_t n_pad);
-#define TM_PCG_STANDARD 0   /* Hestenes-Stiefel PCG, two grid barriers per iteration */
+#define TM_PCG_STANDARD 0   /* Hestenes-Stiefel PCG, two or three barriers per iteration */
 #define TM_PCG_PIPELINED 1  /* Ghysels-Vanroose pipelined PCG, one barrier; less stable */
 #define TM_PCG_NARROW 2     /* or-ed in: 16-bit column offsets (the plan's out_narrow must be 1;
                                an offset that does not fit returns TM_ERR_INDEX) */

@@ -907,9 +907,10 @@ int launch_pcg_sell(int64_t n, const int64_t* indptr, const int32_t* indices, co
   CT* scol = reinterpret_cast<CT*>(q);
   S* dinv = vec[0];
   S* y = vec[5];  // M^-1 x0, read by the first sweep only
-  // the record, and the words of grid_sum (the first of the partial sums' array)
-  ulonglong2* slots = reinterpret_cast<ulonglong2*>(partials);
-  const size_t clear = pipe ? sizeof(PcgState) : 256 + grid_slot_bytes(nb);
+  // the record, and the words of grid_sum: the first of the partial sums'
+  // array, from a 16-byte boundary (the workspace itself may start on 8)
+  ulonglong2* slots = reinterpret_cast<ulonglong2*>((reinterpret_cast<uintptr_t>(partials) + 15) & ~uintptr_t(15));
+  const size_t clear = pipe ? sizeof(PcgState) : 256 + 16 + grid_slot_bytes(nb);
   if (cudaMemsetAsync(st, 0, clear, s) != cudaSuccess) return TM_ERR_CUDA;
   sell_dinv_kernel<S><<<(unsigned)((n + 255) / 256), 256, 0, s>>>(n, indptr, indices, values, dinv);
   const int64_t n_slices = (n + 31) >> 5;

@@ -238,3 +238,27 @@ def test_row_sums_have_the_error_of_normalised_pairs(n, per):
         K.solve(torch.tensor(b, device=DEV), x0=torch.tensor(x, device=DEV), rtol=1e-18, maxiter=0)
     got = K.last_solve_info.recurrence_residual
     assert abs(got - expect) <= 0.05 * expect, (got, expect)
+
+
+@pytest.mark.parametrize("dim,n", [(2, 20), (2, 250), (3, 70)])
+def test_workspace_on_eight_bytes(dim, n):
+    """A workspace that starts 8 bytes past a 16-byte boundary, in each launch
+    mode: the bits of an aligned one."""
+    K, f = poisson(dim, n, torch.float64)
+    sp, n_pad, narrow = S.sell_plan(K.indptr, K.indices)
+    rows = f.shape[0]
+    need = _lib.load().tm_pcg_sell_workspace_bytes(_lib.TM_F64, rows, n_pad)
+    out = []
+    for shift in (0, 8):
+        work = torch.empty(need + 16, dtype=torch.uint8, device=DEV)
+        at = work.data_ptr() + shift
+        assert work.data_ptr() % 16 == 0
+        x = torch.zeros_like(f)
+        stream = torch.cuda.current_stream().cuda_stream
+        _lib.call("tm_pcg_jacobi_sell", _lib.TM_F64, rows, K.indptr.data_ptr(), K.indices.data_ptr(),
+                  K.values.data_ptr(), sp.data_ptr(), n_pad, f.data_ptr(), x.data_ptr(), 1e-6, 0.0, 10000,
+                  _lib.TM_PCG_STANDARD | (_lib.TM_PCG_NARROW if narrow else 0), at, need, stream)
+        it, res, bn = ctypes.c_int32(0), ctypes.c_double(0.0), ctypes.c_double(0.0)
+        assert _lib.load().tm_pcg_result(at, ctypes.byref(it), ctypes.byref(res), ctypes.byref(bn), stream) == 0
+        out.append((x, it.value))
+    assert torch.equal(out[0][0], out[1][0]) and out[0][1] == out[1][1] > 10
