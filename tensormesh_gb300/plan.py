@@ -436,9 +436,15 @@ class GatherPlan:
     # elements, 21 KB of staged values, so eight 128-thread CTAs share an SM:
     # 124 us at 80^3 against 136 us for 64 rows and 256 threads); as many rows
     # of blocks as have at most 512 entries, one for each thread of the CTA
-    # (tm_group_count refuses more)
-    ROWS = {1: (32, 16, 8, 4, 2, 1), 2: (64, 56, 48, 40, 32, 24, 16, 8, 4, 2, 1),
-            3: (34, 32, 30, 28, 26, 24, 22, 20, 16, 12, 8, 4, 2, 1)}
+    # (tm_group_count refuses more).  One group too full (nodes of very high
+    # valence beside each other) takes every group to the next size; below the
+    # last one the patch kernels are faster, and no lists are made.  us a call,
+    # patches / groups of so many rows, float64, 64^3 tetrahedra and 400^2
+    # square's triangles: Laplace 168 / 132 at 32, 145 at 16, 181 at 8 and
+    # 54 / 35, 42, 61; blocks of three 1289 / 432 at 34, 545 at 16, 759 at 8,
+    # 1323 at 4; blocks of two 325 / 71 at 64, 126 at 16, 221 at 8 (float32 93 /
+    # 48, 98, 171)
+    ROWS = {1: (32, 16), 2: (64, 56, 48, 40, 32, 24, 16), 3: (34, 32, 30, 28, 26, 24, 22, 20, 16, 12, 8)}
     SMEM_BYTES = 200 * 1024
 
     def __init__(self, elements: torch.Tensor, points: torch.Tensor, pattern: NodePattern):

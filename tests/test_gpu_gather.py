@@ -810,3 +810,20 @@ def test_an_outlying_first_element_leaves_the_others_in_the_window(etype, n, fir
     away = torch.ones(x.shape[0], dtype=torch.bool, device=DEV)
     away[cells[torch.isin(cells, cells[0]).any(1)]] = False
     assert int(away.sum()) > 100 and torch.equal(a[away], b[away])
+
+
+@pytest.mark.parametrize("dtype", [torch.float64, torch.float32])
+def test_nodes_too_full_for_the_smallest_group_keep_the_patch_kernels(dtype):
+    """Two apexes of 242 neighbours side by side: no group of eight block rows
+    that holds both has at most 512 entries, so elasticity takes the patches."""
+    ring = 240
+    t = np.arange(ring) * 2 * np.pi / ring
+    rim = np.stack([np.cos(t), np.sin(t), 0.8 * np.sin(3 * t)], 1)
+    pts = np.concatenate([[[-0.3, -0.2, 0.1], [-0.3, -0.2, 0.12]], rim])
+    el = np.array([[0, 2 + k, 2 + (k + 1) % ring, 1] for k in range(ring)], dtype=np.int64)
+    coef = np.exp(np.random.default_rng(ring).normal(size=ring))
+    mesh = tg.Mesh(points=torch.tensor(pts, device=DEV), cells={"tetra": torch.tensor(el, device=DEV)})
+    plan = KappaLaplace.from_mesh(mesh).topology.gather
+    assert plan.struct(1) is not None and plan.struct(3) is None
+    check(pts, el, "tetra", "elasticity", coef, dtype)
+    check(pts, el, "tetra", "laplace", coef, dtype)
