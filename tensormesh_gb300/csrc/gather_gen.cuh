@@ -396,28 +396,41 @@ gen_element_kernel(int64_t n_el, const int32_t* __restrict__ el, tm_assemble_arg
   }
 }
 
-// The common exponent of a call, from its elements' largest edges and
-// coefficients (one warp).
-template <class T>
-__global__ void gen_head_kernel(int64_t n_el, int D, int B, int HC, int power, const int32_t* __restrict__ el_all,
-                                tm_assemble_args args, Head* head) {
-  const T* pts = static_cast<const T*>(args.points);
-  const T* coef = static_cast<const T*>(args.coef);
+// The common exponent of a call, from its elements' largest vertex edges and
+// coefficients (one warp; unrolled, so that the loads go out together).
+template <class T, int D, int B, int HC>
+__global__ void gen_head_kernel(int64_t n_el, int power, const int32_t* __restrict__ el, tm_assemble_args args,
+                                Head* head) {
+  const T* __restrict__ pts = static_cast<const T*>(args.points);
+  const T* __restrict__ coef = static_cast<const T*>(args.coef);
   const int Q = args.n_quad;
   const int64_t e = head_element(n_el);
-  const int32_t* __restrict__ el = el_all + e * B;
+  int v[B];
+#pragma unroll
+  for (int b = 0; b < B; ++b) v[b] = el[e * B + b];
   int em = 0, ec = 0;
-  for (int b = 1; b < B; ++b)
+#pragma unroll
+  for (int b = 1; b <= D; ++b)
+#pragma unroll
     for (int d = 0; d < D; ++d)
-      em = max(em, dexp((double)pts[(int64_t)el[b] * D + d] - (double)pts[(int64_t)el[0] * D + d]));
+      em = max(em, dexp((double)pts[(int64_t)v[b] * D + d] - (double)pts[(int64_t)v[0] * D + d]));
   auto see = [&](double c) {
     const int x = dexp(c);
     if (x != 2047) ec = max(ec, x);
   };
-  if (args.coef_kind == TM_COEF_SCALAR) for (int h = 0; h < HC; ++h) see(args.scal[h]);
-  else if (args.coef_kind == TM_COEF_ELEMENT) see((double)coef[e]);
-  else if (args.coef_kind == TM_COEF_QUAD) for (int i = 0; i < Q * HC; ++i) see((double)coef[e * Q * HC + i]);
-  else for (int b = 0; b < B; ++b) for (int h = 0; h < HC; ++h) see((double)coef[(int64_t)el[b] * HC + h]);
+  if (args.coef_kind == TM_COEF_SCALAR) {
+#pragma unroll
+    for (int h = 0; h < HC; ++h) see(args.scal[h]);
+  } else if (args.coef_kind == TM_COEF_ELEMENT) {
+    see((double)coef[e]);
+  } else if (args.coef_kind == TM_COEF_QUAD) {
+    for (int i = 0; i < Q * HC; ++i) see((double)coef[e * Q * HC + i]);
+  } else {
+#pragma unroll
+    for (int b = 0; b < B; ++b)
+#pragma unroll
+      for (int h = 0; h < HC; ++h) see((double)coef[(int64_t)v[b] * HC + h]);
+  }
   const bool have = em >= 200 && em <= 1846 && ec > 0;
   const int S = median_exp(have ? elem_exp(em, ec, power) : 0, have);
   if (threadIdx.x != 0) return;
@@ -716,7 +729,7 @@ int launch_gen(const tm_gather_plan& plan, const tm_assemble_args& args, void* w
   S* vals = reinterpret_cast<S*>(sc.vals);
   S* diag = reinterpret_cast<S*>(sc.diag);
   if constexpr (sizeof(T) == 8)
-    gen_head_kernel<T><<<1, 32, 0, s>>>(n, G::D, G::B, G::HC, G::power, plan.elements, args, sc.head);
+    gen_head_kernel<T, G::D, G::B, G::HC><<<1, 32, 0, s>>>(n, G::power, plan.elements, args, sc.head);
   int st = TM_OK;
   if constexpr (G::kLoad && G::kP1) {
     auto kern = args.coef_kind == TM_COEF_POINT ? p1_load_kernel<T, G::D, H, true> : p1_load_kernel<T, G::D, H, false>;
