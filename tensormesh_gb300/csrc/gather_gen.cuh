@@ -3,8 +3,8 @@
 // gather_load.cuh the loads of P1 elements).  A CTA integrates
 // 32 elements in three phases with one barrier each:
 //   0  edge vectors and coefficients with their exponents, to shared memory;
-//   1  one thread per (quadrature point, element): Jacobian, its adjugate, the
-//      scaled gradients G_a = det grad N_a and the point's factor
+//   1  one thread per (quadrature point, element): Jacobian (see edge_of_node),
+//      its adjugate, the scaled gradients G_a = det grad N_a and the point's factor
 //      (c w / |det| for stiffness, c w |det| for mass and loads); P1 elements
 //      have one geometry for all points;
 //   2  one warp per node pair, one lane per element: the pair's sum over the
@@ -43,7 +43,7 @@ struct Gen {
 template <int EL, int FORM, int H>
 constexpr size_t gen_words(int Q) {
   using G = Gen<EL, FORM, H>;
-  return kMaxQuad * (G::NT + G::B * G::D) + (size_t)(G::B - 1) * G::D * kGenEl +
+  return (size_t)Q * (G::NT + G::B * G::D + G::D * G::D) + (size_t)(G::B - 1) * G::D * kGenEl +
          (G::kStiff ? (size_t)Q * G::B * G::D * kGenEl : 0) + (size_t)Q * G::HC * kGenEl + (size_t)kGenEl * G::stage;
 }
 template <int EL, int FORM, int H, class T>
@@ -51,6 +51,26 @@ constexpr size_t gen_smem(int Q) {
   using G = Gen<EL, FORM, H>;
   return (size_t)Q * G::HC * kGenEl * 8 + gen_words<EL, FORM, H>(Q) * sizeof(typename Sto<T>::S) +
          (size_t)(G::B + 4) * kGenEl * 4;
+}
+
+// Vertices a < c between which node b > D of a P2 simplex lies.  The nodes on
+// the edges enter the Jacobian by their distance from the middle of their edge,
+// x_b = (x_a + x_c) / 2 + delta_b, the vertices with what that leaves them:
+//   J = sum_{k <= D} (dN_k + 1/2 sum_{b on k} dN_b) (x_k - x_0) + sum_b dN_b delta_b,
+// the tables' own J in another grouping.  The first factors are 0 and 1 but for
+// a rounding (tables with the nodes in another order have other factors and
+// take the general form), so straight elements have the Jacobian of their
+// edges: formed from the nodes as they are, its roundings were the same in every
+// element of a regular mesh.
+template <int D> TM_D void edge_of_node(int b, int& a, int& c) {
+  const int i = b - D - 1;
+  if constexpr (D == 2) {   // (1,2) (0,2) (0,1)
+    a = i == 0 ? 1 : 0;
+    c = i == 2 ? 1 : 2;
+  } else {                  // (2,3) (1,3) (1,2) (0,3) (0,2) (0,1)
+    a = i == 0 ? 2 : i < 3 ? 1 : 0;
+    c = i == 2 || i == 4 ? 2 : i == 5 ? 1 : 3;
+  }
 }
 
 // Storage word of arithmetic A in shared memory.
@@ -86,8 +106,9 @@ TM_D bool gen_pass(const tm_assemble_args& args, int64_t e0, int ne, double* s_c
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int Q = args.n_quad;
   W* s_N = reinterpret_cast<W*>(words);
-  W* s_dN = s_N + kMaxQuad * G::NT;
-  W* s_X = s_dN + kMaxQuad * B * D;               // [(B - 1) D][32]
+  W* s_dN = s_N + Q * G::NT;
+  W* s_T = s_dN + Q * B * D;                      // [Q][D vertices][D] factors of the vertices
+  W* s_X = s_T + Q * D * D;                       // [(B - 1) D][32] edges x_k - x_0, then deltas
   W* s_G = s_X + (B - 1) * D * kGenEl;            // [Q][B D][32]
   W* s_s = s_G + (G::kStiff ? Q * B * D * kGenEl : 0);  // [Q][HC][32]
   St* s_out = reinterpret_cast<St*>(s_s + Q * HC * kGenEl);   // [32][off + diag]
@@ -103,21 +124,40 @@ TM_D bool gen_pass(const tm_assemble_args& args, int64_t e0, int ne, double* s_c
   } else {
     for (int i = tid; i < Q * B; i += kGenThreads) s_N[i] = Pa::st(Pa::in(args.tables[Q + i]));
   }
-  for (int i = tid; i < Q * B * D; i += kGenThreads) s_dN[i] = Pa::st(Pa::in(args.tables[Q + Q * B + i]));
+  const double* __restrict__ dN = args.tables + Q + Q * B;
+  for (int i = tid; i < Q * B * D; i += kGenThreads) s_dN[i] = Pa::st(Pa::in(dN[i]));
+  bool general = false;
+  for (int i = tid; i < Q * D * D; i += kGenThreads) {
+    const int q = i / (D * D), k = (i - q * D * D) / D + 1, d = i % D;
+    double t = dN[(q * B + k) * D + d];
+    for (int b = D + 1; b < B; ++b) {
+      int a, c;
+      edge_of_node<D>(b, a, c);
+      if (a == k || c == k) t += 0.5 * dN[(q * B + b) * D + d];
+    }
+    s_T[i] = Pa::st(Pa::in(t));
+    general = general || fabs(t - (k - 1 == d ? 1.0 : 0.0)) > 0x1p-48;
+  }
   const T* __restrict__ pts = static_cast<const T*>(args.points);
   for (int i = tid; i < (B - 1) * kGenEl; i += kGenThreads) {
     const int b = i / kGenEl + 1;   // lane = element
-    const int em = s_emax[lane];
+    int a = 0, c = 0;
+    if (b > D) edge_of_node<D>(b, a, c);
+    const int em = s_emax[lane] + (b > D ? 1 : 0);   // (halves the deltas)
+    const T* __restrict__ pb = pts + (int64_t)s_v[b * kGenEl + lane] * D;
+    const T* __restrict__ pa = pts + (int64_t)s_v[a * kGenEl + lane] * D;
+    const T* __restrict__ pc = pts + (int64_t)s_v[c * kGenEl + lane] * D;
 #pragma unroll
     for (int d = 0; d < D; ++d) {
-      const T x = pts[(int64_t)s_v[b * kGenEl + lane] * D + d] - pts[(int64_t)s_v[lane] * D + d];
+      T x = pb[d] - pa[d];
+      if (b > D) x -= pc[d] - pb[d];
       A y;
       if constexpr (kPairsT) y = scaled<A>((double)x, em);
       else y = tm_scale_pow2(x, 1023 - em);
       s_X[((b - 1) * D + d) * kGenEl + lane] = Pa::st(y);
     }
   }
-  __syncthreads();
+  general = __syncthreads_or(general);
   // ---- phase 1
   bool flag = false;
   auto X = [&](int b, int d) -> A { return Pa::ld(s_X[((b - 1) * D + d) * kGenEl + lane]); };
@@ -127,19 +167,25 @@ TM_D bool gen_pass(const tm_assemble_args& args, int64_t e0, int ne, double* s_c
 #pragma unroll
     for (int i = 0; i < D; ++i)
 #pragma unroll
-      for (int j = 0; j < D; ++j) J[i][j] = Pa::zero();
-#pragma unroll
-    for (int b = 1; b < B; ++b) {
+      for (int j = 0; j < D; ++j) J[i][j] = X(i + 1, j);
+    auto add_node = [&](int b, const W* dn) {
       A x[D];
 #pragma unroll
       for (int j = 0; j < D; ++j) x[j] = X(b, j);
 #pragma unroll
-      for (int i = 0; i < D; ++i) {
-        const A dn = Pa::ld(s_dN[(q * B + b) * D + i]);
+      for (int i = 0; i < D; ++i)
 #pragma unroll
-        for (int j = 0; j < D; ++j) J[i][j] = norm(Pa::add(J[i][j], norm(Pa::mul(dn, x[j]))));
-      }
+        for (int j = 0; j < D; ++j) J[i][j] = norm(Pa::add(J[i][j], norm(Pa::mul(Pa::ld(dn[i]), x[j]))));
+    };
+    if (general) {   // nodes in another order than edge_of_node's
+#pragma unroll
+      for (int i = 0; i < D; ++i)
+#pragma unroll
+        for (int j = 0; j < D; ++j) J[i][j] = Pa::zero();
+      for (int k = 1; k <= D; ++k) add_node(k, s_T + (q * D + k - 1) * D);
     }
+#pragma unroll
+    for (int b = D + 1; b < B; ++b) add_node(b, s_dN + (q * B + b) * D);
 #pragma unroll
     for (int i = 0; i < D; ++i)
 #pragma unroll
@@ -172,7 +218,6 @@ TM_D bool gen_pass(const tm_assemble_args& args, int64_t e0, int ne, double* s_c
         if (!simplex_well_conditioned<D>(dv) || s_r[lane] == INT_MIN) flag = true;
       }
     }
-    const A geo = G::kStiff ? Pa::rcp(adet) : adet;
     const int q1 = G::kP1 ? Q : q + 1;
     for (int qq = q; qq < q1; ++qq) {
 #pragma unroll
@@ -186,7 +231,7 @@ TM_D bool gen_pass(const tm_assemble_args& args, int64_t e0, int ne, double* s_c
         } else {
           cs = (float)c;
         }
-        s_s[(qq * HC + h) * kGenEl + lane] = Pa::st(norm(Pa::mul(cs, geo)));
+        s_s[(qq * HC + h) * kGenEl + lane] = Pa::st(norm(G::kStiff ? Pa::div(cs, adet) : Pa::mul(cs, adet)));
       }
     }
     if constexpr (G::kStiff) {
@@ -663,7 +708,7 @@ TM_D void sum_blocks(const tm_gather_plan& plan, const typename Sto<T>::S* __res
     if (pos >= 0) s_val[pos * HH + c] = M::st(norm(acc));
   }
   __syncthreads();
-  const A lam = Pa::in(lam_d), mu = Pa::in(mu_d);
+  const A lam = Pa::in(lam_d), mu = Pa::in(mu_d), both = Pa::in(lam_d + 2.0 * mu_d);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   for (int w = warp; w < D * nr; w += kBlkThreads / 32) {
     const int lr = w / D, a = w - lr * D;
@@ -673,13 +718,15 @@ TM_D void sum_blocks(const tm_gather_plan& plan, const typename Sto<T>::S* __res
     for (int k = lane; k < deg * D; k += 32) {
       const int kk = k / D, b = k - kk * D;
       const auto* m = s_val + (l0 + kk) * HH;
-      A x = Pa::add(Pa::mul(lam, M::get(m[a * D + b])), Pa::mul(mu, M::get(m[b * D + a])));
+      A other = M::get(m[b * D + a]);   // what mu multiplies; on the diagonal the other diagonal components
       if (a == b) {
-        A tr = M::get(m[0]);
+        other = M::get(m[a ? 0 : D + 1]);
 #pragma unroll
-        for (int d = 1; d < D; ++d) tr = Pa::add(tr, M::get(m[d * D + d]));
-        x = Pa::add(x, Pa::mul(mu, norm(tr)));
+        for (int d = 1; d < D; ++d)
+          if (d != a && (a || d > 1)) other = Pa::add(other, M::get(m[d * D + d]));
+        other = norm(other);
       }
+      const A x = Pa::add(Pa::mul(a == b ? both : lam, M::get(m[a * D + b])), Pa::mul(mu, other));
       o[k] = (T)M::out(x, S);
     }
   }

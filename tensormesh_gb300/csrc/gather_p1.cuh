@@ -138,7 +138,7 @@ TM_D bool p1_element(const A (&d)[D][D], A cw, A (&out)[p1_values<D, kElast>()])
   const float dh = P::hi(det);
   // tr G tr adj G / det G (2D: tr G^2 / det G, adj G having G's trace)
   const bool good = dh * dh >= 1e-30f && trg * tra <= kCondMax * (dh * dh);
-  const A s = P::mul(cw, P::rcp(P::abs(det)));
+  const A s = P::div(cw, P::abs(det));
   if constexpr (kElast) {
 #pragma unroll
     for (int k = 0; k < D; ++k)
@@ -654,19 +654,31 @@ TM_D void group_blocks(const tm_gather_plan& plan, const typename Sto<T>::S* __r
       const A s = M::ld(v[B * D], we, S);
 #pragma unroll
       for (int i = 0; i < D; ++i) {
-        const A si = norm2d(Pa::mul(s, cof(v[a * D + i], we)));
+        const A ca = cof(v[a * D + i], we);
+        // triangles multiply the cofactors first: where their edges are those
+        // that make up the determinant, its rounding in s cancels
+        const A si = D == 2 ? ca : Pa::mul(s, ca);
 #pragma unroll
-        for (int j = 0; j < D; ++j) acc[i][j] = Pa::add(acc[i][j], Pa::mul(si, cb[j]));
+        for (int j = 0; j < D; ++j) {
+          const A x = Pa::mul(si, cb[j]);
+          acc[i][j] = Pa::add(acc[i][j], D == 2 ? Pa::mul(s, norm(x)) : x);
+        }
       }
       if (last) break;
     }
-    const A lam = Pa::in(lam_d), mu = Pa::in(mu_d);
+    // diagonal components (lam + 2 mu) M_ii + mu sum_{d != i} M_dd: two products
+    const A lam = Pa::in(lam_d), mu = Pa::in(mu_d), both = Pa::in(lam_d + 2.0 * mu_d);
 #pragma unroll
     for (int i = 0; i < D * D; ++i) acc[i / D][i % D] = norm2d(acc[i / D][i % D]);
-    A tr = acc[0][0];
+    A diag[D];
 #pragma unroll
-    for (int d = 1; d < D; ++d) tr = Pa::add(tr, acc[d][d]);
-    tr = Pa::mul(mu, norm2d(tr));
+    for (int i = 0; i < D; ++i) {
+      A rest = acc[i ? 0 : 1][i ? 0 : 1];
+#pragma unroll
+      for (int d = i ? 1 : 2; d < D; ++d)
+        if (d != i) rest = Pa::add(rest, acc[d][d]);
+      diag[i] = Pa::add(Pa::mul(both, acc[i][i]), Pa::mul(mu, norm(rest)));
+    }
 #pragma unroll
     for (int i = 0; i < D; ++i) {
 #pragma unroll
@@ -675,8 +687,7 @@ TM_D void group_blocks(const tm_gather_plan& plan, const typename Sto<T>::S* __r
         acc[i][j] = Pa::add(Pa::mul(lam, x), Pa::mul(mu, y));
         acc[j][i] = Pa::add(Pa::mul(lam, y), Pa::mul(mu, x));
       }
-      const A x = acc[i][i];
-      acc[i][i] = Pa::add(Pa::add(Pa::mul(lam, x), Pa::mul(mu, x)), tr);
+      acc[i][i] = diag[i];
     }
   }
   __syncthreads();   // the cofactors are done with

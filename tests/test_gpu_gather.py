@@ -685,6 +685,36 @@ def test_p2_stiffness_is_as_accurate_as_the_patch_kernels(etype, n, form, q, mon
     assert (once <= patch).all(), (once, patch)
 
 
+def on_regular_meshes(etype, sizes, form, q, monkeypatch):
+    """Relative 2-norm errors of the float64 values, element-once and patch
+    kernels, summed over regular meshes: the geometry's roundings are the same
+    in all elements of one and average out over the sizes only."""
+    err = np.zeros(2)
+    for n in sizes:
+        base = (tg.Mesh.gen_unit_square if etype.startswith("tri") else tg.Mesh.gen_unit_cube)(n)
+        mesh = (base.to_p2() if etype in ("triangle6", "tetra10") else base).to(DEV)
+        cells = mesh.cells[etype].long()
+        g = torch.Generator(device=DEV).manual_seed(n)
+        k = torch.exp(torch.randn(cells.shape[0], generator=g, device=DEV, dtype=torch.float64))
+        asm = FORMS[form].from_mesh(mesh, q)
+        for route, least in enumerate((0, 1 << 40)):
+            monkeypatch.setattr("tensormesh_gb300.assemble._GATHER_MIN_ELEMENTS", {etype: least})
+            values = asm(mesh.points, element_data={"kappa": k}).values
+            ref = exact_values(mesh.points, cells, etype, form, q, k, asm)
+            err[route] += float((values - ref).norm() / ref.norm())
+    return err
+
+
+@pytest.mark.parametrize("etype,sizes,q", [("triangle", (20, 27, 33, 47, 60, 100, 150, 255), 1),
+                                           ("triangle", (20, 27, 33, 47, 60, 100, 150, 255), 2),
+                                           ("triangle6", (10, 27, 39, 50, 51, 57, 75, 79), 2),
+                                           ("tetra", (8, 10, 13, 17, 21, 28), 2), ("tetra10", (4, 5, 6, 7, 8, 10), 2)])
+@pytest.mark.parametrize("form", ["laplace", "elasticity"])
+def test_stiffness_of_regular_meshes_is_as_accurate_as_the_patch_kernels(etype, sizes, q, form, monkeypatch):
+    once, patch = on_regular_meshes(etype, sizes, form, q, monkeypatch)
+    assert once <= patch, (once, patch)
+
+
 # -- native FP64 -------------------------------------------------------------------
 @pytest.mark.parametrize("how", ["instance", "class"])
 @pytest.mark.parametrize("kind", ["matrix", "load"])
