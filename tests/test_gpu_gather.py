@@ -715,6 +715,35 @@ def test_stiffness_of_regular_meshes_is_as_accurate_as_the_patch_kernels(etype, 
     assert once <= patch, (once, patch)
 
 
+@pytest.mark.parametrize("etype,sizes", [("triangle", (20, 31, 57, 100, 150, 255)), ("tetra", (8, 10, 13, 17, 21, 28))])
+@pytest.mark.parametrize("form", ["laplace", "elasticity"])
+def test_gradients_of_p1_matrices_are_as_accurate_as_the_patch_form(etype, sizes, form, monkeypatch):
+    """float32 gradients of the coefficient and the points against float64
+    ones, summed over regular meshes."""
+    err = np.zeros((2, 2))
+    struct = tg.plan.GatherPlan.struct
+    for n in sizes:
+        mesh = (tg.Mesh.gen_unit_square if etype == "triangle" else tg.Mesh.gen_unit_cube)(n).to(DEV)
+        asm = FORMS[form].from_mesh(mesh, 2)
+        g = torch.Generator(device=DEV).manual_seed(n)
+        k32 = torch.exp(torch.randn(mesh.cells[etype].shape[0], generator=g, device=DEV))
+        x32, G = mesh.points.float(), None
+
+        def gradients(dtype, patch):
+            nonlocal G
+            monkeypatch.setattr(tg.plan.GatherPlan, "struct", lambda p, H: None if H == 0 and patch else struct(p, H))
+            x, k = x32.to(dtype).requires_grad_(), k32.to(dtype).requires_grad_()
+            K = asm(x, element_data={"kappa": k})
+            if G is None:
+                G = torch.randn(K.values.shape[0], generator=g, device=DEV)
+            return torch.autograd.grad(K.values, (k, x), G.to(dtype))
+        exact = gradients(torch.float64, True)
+        for route in range(2):
+            got = gradients(torch.float32, bool(route))
+            err[route] += [float((a.double() - b).norm() / b.norm()) for a, b in zip(got, exact)]
+    assert (err[0] <= err[1]).all(), err
+
+
 # -- native FP64 -------------------------------------------------------------------
 @pytest.mark.parametrize("how", ["instance", "class"])
 @pytest.mark.parametrize("kind", ["matrix", "load"])
