@@ -19,9 +19,9 @@
 // the matrix's slots.
 //
 // FP64 runs native arithmetic, as the patch form does; its pipe (0.53 T
-// operations a second) bounds the float64 Laplace kernel: about 180 operations
-// an element.  Forward and backward call at 48^3 cells, order 2: 3577 us with
-// the patch form, 431 us with this one.
+// operations a second) bounds the float64 Laplace kernel: about 210 operations
+// an element, 280 us of a forward and backward call at 48^3 cells, order 2,
+// that takes 449 us (3577 with the patch form).
 #include "gather.cuh"
 
 namespace tmg {

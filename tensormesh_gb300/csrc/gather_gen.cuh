@@ -14,7 +14,7 @@
 // tetrahedron take about 40 double-float instructions a point each.  Against
 // the patch kernel, which stages the full matrix of an element (800 bytes for
 // Laplace, 7200 for elasticity) and so runs with few threads: calls at 27^3
-// cells 2720 -> 248 us (Laplace), 3072 elements 6055 -> 98 us (elasticity).
+// cells 2720 -> 247 us (Laplace), 3072 elements 6055 -> 98 us (elasticity).
 #pragma once
 #include "gather_load.cuh"
 

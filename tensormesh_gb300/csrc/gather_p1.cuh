@@ -186,9 +186,9 @@ TM_D bool p1_element(const A (&d)[D][D], A cw, A (&out)[p1_values<D, kElast>()])
 
 // One thread per element.  A warp's values go through shared memory so that
 // its 32 consecutive elements write one contiguous run.  Bound by instruction
-// issue: about 800 instructions an element in double-float, issued at 75 %,
-// with the FP64 pipe (the nine subtractions of the edges) at 52 %; 64
-// registers hold eight CTAs an SM (95 us for 3.07 M tetrahedra).
+// issue: about 930 instructions a warp of 32 elements in double-float, issued at
+// 81 %, with the FP64 pipe (the nine subtractions of the edges) at 56 %; 64
+// registers hold eight CTAs an SM (364 us for 12.6 M tetrahedra).
 template <class T, int D, bool kElast>
 __global__ void __launch_bounds__(kElThreads, 8)
 p1_element_kernel(int64_t n_el, const int32_t* __restrict__ el, tm_assemble_args args, Head* __restrict__ head,
@@ -564,7 +564,7 @@ template <class T, int B> size_t group_rows_smem(const tm_gather_plan& p) {
 // row's (the cofactors of an element add to zero).  One thread per entry; the
 // blocks replace the cofactors in shared memory once every thread holds its
 // own, and the CTA writes the rows in order.  Issue-bound (65 % of the slots):
-// nine double-float multiply-adds per record; 376 us at 64^3, where the patch
+// nine double-float multiply-adds per record; 370 us at 64^3, where the patch
 // kernel, which forms all sixteen blocks of an element from staged values,
 // takes 1390 us.
 constexpr int kBlkGrpThreads = kBlockEntries;
