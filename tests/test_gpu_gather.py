@@ -744,6 +744,39 @@ def test_gradients_of_p1_matrices_are_as_accurate_as_the_patch_form(etype, sizes
     assert (err[0] <= err[1]).all(), err
 
 
+@pytest.mark.parametrize("etype,n", [("triangle6", 9), ("tetra10", 4)])
+@pytest.mark.parametrize("form", ["laplace", "mass", "elasticity"])
+@pytest.mark.parametrize("dtype", [torch.float64, torch.float32])
+def test_edge_nodes_in_another_order(etype, n, form, dtype, monkeypatch):
+    """Tables and connectivity with the nodes on the edges in another order
+    than the framework's (a caller of the C entry may have one): the same
+    matrix, whose Jacobians no longer start from the vertices alone."""
+    base = tg.Mesh.gen_unit_square(n) if etype == "triangle6" else tg.Mesh.gen_unit_cube(n)
+    mesh = base.to_p2().to(DEV)
+    B, D = mesh.cells[etype].shape[1], mesh.points.shape[1]
+    g = torch.Generator(device=DEV).manual_seed(n)
+    x = (mesh.points + 0.05 / n * torch.rand(mesh.points.shape, generator=g, device=DEV, dtype=torch.float64)).to(dtype)
+    k = torch.exp(torch.randn(mesh.cells[etype].shape[0], generator=g, device=DEV, dtype=torch.float64)).to(dtype)
+    Q = tg.element.n_quadrature(etype, 2)
+    order = torch.arange(B, device=DEV)
+    order[D + 1:] = order[D + 1:].flip(0).roll(1)
+    K = FORMS[form].from_mesh(mesh, 2)(x, element_data={"kappa": k})
+    plain = tg.element.kernel_tables
+    t = plain(etype, 2, torch.device(DEV))
+    N, dN = t[Q:Q + Q * B].view(Q, B)[:, order], t[Q + Q * B:Q + Q * B + Q * B * D].view(Q, B, D)[:, order]
+    other = torch.cat([t[:Q], N.reshape(-1), dN.reshape(-1)])
+    turned = tg.Mesh(points=mesh.points, cells={etype: mesh.cells[etype][:, order].contiguous()})
+    asm = FORMS[form].from_mesh(turned, 2)
+    asm(x, element_data={"kappa": k})   # the form is recognised with the framework's tables
+    monkeypatch.setattr(tg.element, "kernel_tables", lambda *a: other)
+    L = asm(x, element_data={"kappa": k})
+    assert asm.topology.element_once
+    assert torch.equal(L.indptr, K.indptr) and torch.equal(L.indices, K.indices)
+    # the same sums in another order and grouping: float64 within 1e-13 of the largest, float32 within 4e-6
+    bar = 1e-13 if dtype == torch.float64 else 4e-6
+    assert float((L.values - K.values).abs().max()) <= bar * float(K.values.abs().max())
+
+
 # -- native FP64 -------------------------------------------------------------------
 @pytest.mark.parametrize("how", ["instance", "class"])
 @pytest.mark.parametrize("kind", ["matrix", "load"])
